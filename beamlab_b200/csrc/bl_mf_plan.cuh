@@ -16,9 +16,18 @@
 // The solution equals the column-by-column one up to the order of the floating-point sums.
 #pragma once
 
+#include <vector_functions.h>
+#include <vector_types.h>
+
 #include <algorithm>
 #include <cstdint>
 #include <vector>
+
+#ifdef __CUDACC__
+#define MF_HD __host__ __device__ __forceinline__
+#else
+#define MF_HD inline
+#endif
 
 namespace blg {
 
@@ -189,6 +198,133 @@ static MfPlan mf_finish(int NF, const std::vector<int>& col_ptr, const std::vect
         P.child_ptr.push_back((int)P.child.size());
     }
     return P;
+}
+
+// ------------------------------------------------------------------------------------------ the device's tiles and tasks
+constexpr int kMfT = 48;               // tile side (8 frame nodes)
+constexpr int kMfTile = kMfT * kMfT;   // doubles a tile
+constexpr int kMfFuseRows = 2;         // a front of one pivot tile and up to this many row tiles is one task
+
+struct MfFrontDev {
+    int p, npiv, nrow;   // pivot degrees of freedom, pivot and row nodes
+    int P, nt;           // pivot tiles, tiles a side
+    int bt, br;          // b's row tile, its row in it
+    int tile0;           // its first tile (column by column of the lower triangle)
+    int idx0;            // its nodes (global columns: pivots, then rows) in idx
+    int cpos0, cptr0;    // its row nodes' places in its parent (8 tile + slot) in cpos; per parent tile its first row node
+    int child0, child1;
+    int parent, comp;
+    int need;            // what fdone reaches when its Schur complement is complete
+    int pan0;            // its panels' flags in xflag
+};
+
+enum : int { MF_TILE = 0, MF_FRONT = 1, MF_BACK = 2 };
+
+// tile (i, j), i >= j, of a front of nt tiles a side
+MF_HD int mf_tix(int nt, int i, int j) { return j * nt - j * (j - 1) / 2 + (i - j); }
+
+struct MfLayout {
+    std::vector<MfFrontDev> fr;
+    std::vector<int> cpos, cptr, eptr;  // (MfDev's arrays)
+    std::vector<int2> ent;
+    std::vector<int4> task;
+    int64_t tiles = -1;                 // over all fronts (-1: more than fit their indexes)
+    int pans = 0;                       // pivot tiles on the diagonals
+    int widest = 1;                     // the most factorization tasks of one level
+};
+
+// The plan's tiles, maps and task list for k_mf_solve; goff_ptr: the off-diagonal blocks' assembly entries (a block
+// without any is fill, zero before the factorization)
+static MfLayout mf_layout(const MfPlan& P, const std::vector<int>& col_ptr, const std::vector<int>& row, const std::vector<int>& goff_ptr) {
+    MfLayout Y;
+    const int nfr = (int)P.npiv.size(), nlev = (int)P.level_ptr.size() - 1;
+    std::vector<MfFrontDev>& fr = Y.fr;
+    fr.resize(nfr);
+    int64_t tiles = 0;
+    int pans = 0;
+    auto alone = [&](int f) { return fr[f].P == 1 && fr[f].nt - fr[f].P <= kMfFuseRows; };
+    for (int f = 0; f < nfr; f++) {
+        MfFrontDev& d = fr[f];
+        d.npiv = P.npiv[f], d.nrow = P.nrow[f], d.p = 6 * d.npiv;
+        d.P = (d.npiv + 7) / 8;
+        d.nt = d.P + d.nrow / 8 + 1; // (the rows and b's row after them)
+        d.bt = d.P + d.nrow / 8, d.br = 6 * (d.nrow % 8);
+        d.idx0 = P.idx_ptr[f], d.child0 = P.child_ptr[f], d.child1 = P.child_ptr[f + 1], d.parent = P.parent[f], d.comp = P.comp[f];
+        d.tile0 = (int)tiles, d.pan0 = pans;
+        tiles += (int64_t)d.nt * (d.nt + 1) / 2, pans += d.P;
+        const int R = d.nt - d.P;
+        d.need = alone(f) ? 1 : d.parent >= 0 ? R * (R + 1) / 2 : 1;
+    }
+    if (tiles > (int64_t)1 << 30) return Y; // (its tiles' indexes; such a pool is far past the GPU's memory)
+    Y.tiles = tiles, Y.pans = pans;
+    // each row node's place in its parent's tiles, and per parent tile a front's first row node
+    std::vector<int>&cpos = Y.cpos, &cptr = Y.cptr;
+    for (int f = 0; f < nfr; f++) {
+        MfFrontDev& d = fr[f];
+        d.cpos0 = (int)cpos.size(), d.cptr0 = (int)cptr.size();
+        if (d.parent < 0) continue;
+        const MfFrontDev& q = fr[d.parent];
+        const int* place = P.cmap.data() + d.idx0 + d.npiv;
+        int t = 0;
+        for (int x = 0; x < d.nrow; x++) {
+            const int l = place[x], pos = l < q.npiv ? l : 8 * q.P + (l - q.npiv);
+            for (; t <= pos / 8; t++) cptr.push_back(x);
+            cpos.push_back(pos);
+        }
+        for (; t <= q.nt; t++) cptr.push_back(d.nrow);
+    }
+    // each pivot tile's assembled blocks (those with entries: the fill's are zero)
+    std::vector<int>& eptr = Y.eptr;
+    std::vector<int2>& ent = Y.ent;
+    eptr.assign(tiles + 1, 0);
+    {
+        std::vector<std::pair<int, int2>> e; // (tile, entry)
+        for (int f = 0; f < nfr; f++) {
+            const MfFrontDev& d = fr[f];
+            const int* first = P.idx.data() + d.idx0;
+            const int* last = first + d.npiv + d.nrow;
+            for (int l = 0; l < d.npiv; l++) {
+                const int k = first[l];
+                e.push_back({d.tile0 + mf_tix(d.nt, l / 8, l / 8), make_int2(-k - 1, 9 * (l % 8))});
+                for (int pb = col_ptr[k]; pb < col_ptr[k + 1]; pb++) {
+                    if (goff_ptr[pb] == goff_ptr[pb + 1]) continue;
+                    const int m = (int)(std::lower_bound(first, last, row[pb]) - first), pos = m < d.npiv ? m : 8 * d.P + (m - d.npiv);
+                    e.push_back({d.tile0 + mf_tix(d.nt, pos / 8, l / 8), make_int2(pb, 8 * (pos % 8) + l % 8)});
+                }
+            }
+        }
+        for (const auto& x : e) eptr[x.first + 1]++;
+        for (int64_t t = 0; t < tiles; t++) eptr[t + 1] += eptr[t];
+        ent.resize(e.size());
+        std::vector<int> fill(eptr.begin(), eptr.end() - 1);
+        for (const auto& x : e) ent[fill[x.first]++] = x.second;
+    }
+    // the tasks: level by level from the leaves, a level's whole fronts first, then its tiles column by column over all
+    // its fronts; then the backward solves from the root down, last panels first
+    std::vector<int4>& task = Y.task;
+    for (int L = 0; L < nlev; L++) {
+        int cols = 0;
+        const size_t t0 = task.size();
+        for (int f = P.level_ptr[L]; f < P.level_ptr[L + 1]; f++) {
+            if (alone(f)) task.push_back(make_int4(f, 0, 0, MF_FRONT));
+            else cols = std::max(cols, fr[f].nt);
+        }
+        for (int j = 0; j < cols; j++)
+            for (int f = P.level_ptr[L]; f < P.level_ptr[L + 1]; f++) {
+                const int end = fr[f].parent >= 0 ? fr[f].nt : fr[f].P; // (a root's Schur complement is nobody's)
+                if (alone(f) || j >= end) continue;
+                for (int i = j; i < fr[f].nt; i++) task.push_back(make_int4(f, i, j, MF_TILE));
+            }
+        Y.widest = std::max(Y.widest, (int)(task.size() - t0));
+    }
+    for (int L = nlev - 1; L >= 0; L--) {
+        int cols = 0;
+        for (int f = P.level_ptr[L]; f < P.level_ptr[L + 1]; f++) cols = std::max(cols, fr[f].P);
+        for (int b = 0; b < cols; b++)
+            for (int f = P.level_ptr[L]; f < P.level_ptr[L + 1]; f++)
+                if (b < fr[f].P) task.push_back(make_int4(f, 0, fr[f].P - 1 - b, MF_BACK));
+    }
+    return Y;
 }
 
 } // namespace blg

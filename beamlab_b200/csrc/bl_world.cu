@@ -204,19 +204,15 @@ struct bl_gpu_ctx {
     DevBuf<int> fcol, fchain;
     DevBuf<int4> fblk;
     DevBuf<double> fD, fb;
-    // the multifrontal factorization (bl_multifrontal.cuh), fem_dense_front == 2: fronts, their maps, the pool, and per
-    // level its task ranges (assembly; per panel, panel and update tasks)
+    // the multifrontal factorization and solves (bl_multifrontal.cuh), fem_mode 2: fronts, their maps, tasks, pool, flags
     MfDev mf{};
     DevBuf<MfFrontDev> mf_fr;
-    DevBuf<int> mf_idx, mf_cmap, mf_child, mf_brow;
-    DevBuf<double> mf_pool, mf_dt;
-    DevBuf<int2> mf_tpan;
-    DevBuf<int4> mf_tasm, mf_tupd;
-    std::vector<int> mf_level_ptr;             // fronts of each level (execution order)
-    std::vector<int> mf_tasm_ptr;              // per level: its assembly tasks
-    std::vector<std::vector<int>> mf_tpan_ptr, mf_tupd_ptr; // per level, per panel: its tasks
-    size_t mf_smem = 0;                        // the solves' dynamic shared memory (the largest front)
-    int fem_mode = 0;                          // the factorization in use: fem_dense_front, 3 resolved to 1 or 2
+    DevBuf<int> mf_idx, mf_cpos, mf_cptr, mf_child, mf_eptr, mf_ctr;
+    DevBuf<int2> mf_ent;
+    DevBuf<int4> mf_task;
+    DevBuf<double> mf_pool;
+    int mf_grid = 1, mf_levels = 0;
+    int fem_mode = 0;                          // the factorization in use: fem_dense_front, 3 resolved to 2
     unsigned long long wait_ns = 1000000000ull; // the beams kernel's bound on a wait for its bulk copies (bulk_wait_s)
     double mf_flops = 0;
     DevBuf<float> finertia, tX, tk, ttan, tb, tX0, th0, tdmg;
@@ -289,8 +285,8 @@ static void free_fem(bl_gpu_ctx* c) {
     c->feat.free_(), c->prev_dv.free_(), c->adj_ptr.free_(), c->adj.free_();
     c->gdiag.free_(), c->gu.free_(), c->rb.free_(), c->goff.free_(), c->tn.free_();
     c->fcol.free_(), c->fchain.free_(), c->fblk.free_(), c->fD.free_(), c->fb.free_(), c->front = FrontDev{}, c->front_level = 0;
-    c->mf_fr.free_(), c->mf_idx.free_(), c->mf_cmap.free_(), c->mf_child.free_(), c->mf_brow.free_(), c->mf_pool.free_(), c->mf_dt.free_();
-    c->mf_tasm.free_(), c->mf_tpan.free_(), c->mf_tupd.free_(), c->mf = MfDev{}, c->mf_level_ptr.clear(), c->mf_flops = 0;
+    c->mf_fr.free_(), c->mf_idx.free_(), c->mf_cpos.free_(), c->mf_cptr.free_(), c->mf_child.free_(), c->mf_eptr.free_(), c->mf_ctr.free_();
+    c->mf_ent.free_(), c->mf_task.free_(), c->mf_pool.free_(), c->mf = MfDev{}, c->mf_levels = 0, c->mf_flops = 0;
     c->mn.free_(), c->mmeta.free_(), c->mL0.free_(), c->mq.free_(), c->mfa.free_(), c->mta.free_(), c->mtb.free_(), c->mtan.free_();
     c->msec.free_(), c->mon.free_(), c->mkw.free_(), c->mkv.free_(), c->NM = 0;
     c->mps.free_(), c->mtg.free_(), c->mflag.free_(), c->credit.free_(), c->elastic.free_(), c->comp_again.free_(), c->comp_size.free_();
@@ -544,89 +540,41 @@ static int pull_state(bl_gpu_ctx* c) {
 // column's diagonal block then its off-diagonal ones) with each target's updates in the order of their source columns,
 // each row's blocks in the order of their columns for the forward substitution.
 // The multifrontal plan over every frame's columns (global pattern col_ptr / row, components col_comp): the fronts,
-// their maps and the pool on the device, and each level's task lists (bl_multifrontal.cuh)
-static int commit_multifrontal(bl_gpu_ctx* c, const std::vector<int>& col_ptr, const std::vector<int>& row, const std::vector<int>& col_comp) {
+// their tiles' maps and the pool on the device, and k_mf_solve's task list (bl_multifrontal.cuh)
+static int commit_multifrontal(bl_gpu_ctx* c, const std::vector<int>& col_ptr, const std::vector<int>& row, const std::vector<int>& col_comp,
+                               const std::vector<int>& goff_ptr, int ncomp) {
     const int NF = (int)col_ptr.size() - 1;
     std::vector<std::vector<int>> fr_cols;
     std::vector<int> fr_top, fr_comp;
     mf_plan_columns(NF, col_ptr, row, col_comp, fr_cols, fr_top, fr_comp);
     const MfPlan P = mf_finish(NF, col_ptr, row, fr_cols, fr_top, fr_comp);
-    const int nfr = (int)P.npiv.size(), nlev = (int)P.level_ptr.size() - 1;
-    std::vector<MfFrontDev> fr(nfr);
-    long long pool = 0;
-    int dtn = 0, maxn = 0;
-    for (int f = 0; f < nfr; f++) {
-        MfFrontDev& d = fr[f];
-        d.n = 6 * (P.npiv[f] + P.nrow[f]), d.p = 6 * P.npiv[f];
-        d.off = pool, d.idx0 = P.idx_ptr[f], d.child0 = P.child_ptr[f], d.child1 = P.child_ptr[f + 1], d.comp = P.comp[f];
-        d.dt0 = dtn;
-        pool += (long long)d.n * (d.n + 1);
-        dtn += 2 * kMfT * kMfT * ((d.p + kMfT - 1) / kMfT);
-        maxn = std::max(maxn, d.n);
-    }
-    // each off-diagonal block's row: its node's place in the front of its column
-    std::vector<int> brow(std::max<size_t>(row.size(), 1), 0);
-    for (int f = 0; f < nfr; f++) {
-        const int* first = P.idx.data() + P.idx_ptr[f];
-        const int* last = P.idx.data() + P.idx_ptr[f + 1];
-        for (int l = 0; l < P.npiv[f]; l++) {
-            const int k = first[l];
-            for (int pb = col_ptr[k]; pb < col_ptr[k + 1]; pb++) brow[pb] = (int)(std::lower_bound(first, last, row[pb]) - first);
-        }
-    }
-    std::vector<int4> tasm, tupd;
-    std::vector<int2> tpan;
-    c->mf_tasm_ptr.assign(1, 0), c->mf_tpan_ptr.assign(nlev, {}), c->mf_tupd_ptr.assign(nlev, {});
-    int64_t launches = 0;
-    for (int L = 0; L < nlev; L++) {
-        int np = 0;
-        for (int f = P.level_ptr[L]; f < P.level_ptr[L + 1]; f++) {
-            const int nt = (fr[f].n + kMfT - 1) / kMfT;
-            for (int it = 0; it < nt; it++) {
-                for (int jt = 0; jt <= it; jt++) tasm.push_back(make_int4(f, it, jt, 0));
-                tasm.push_back(make_int4(f, it, -1, 0));
-            }
-            np = std::max(np, (fr[f].p + kMfT - 1) / kMfT);
-        }
-        c->mf_tasm_ptr.push_back((int)tasm.size());
-        c->mf_tpan_ptr[L].push_back((int)tpan.size()), c->mf_tupd_ptr[L].push_back((int)tupd.size());
-        for (int sp = 0; sp < np; sp++) {
-            for (int f = P.level_ptr[L]; f < P.level_ptr[L + 1]; f++) {
-                if (fr[f].p <= kMfT * sp) continue;
-                const int nt = (fr[f].n + kMfT - 1) / kMfT;
-                for (int r = sp; r < nt; r++) tpan.push_back(make_int2(f, r));
-                tupd.push_back(make_int4(f, 0, -1, 0));
-                for (int i = sp + 1; i < nt; i++) tupd.push_back(make_int4(f, i, -2, 0));
-                for (int j = sp + 1; j < nt; j++)
-                    for (int i = j; i < nt; i++) tupd.push_back(make_int4(f, i, j, 0));
-            }
-            c->mf_tpan_ptr[L].push_back((int)tpan.size()), c->mf_tupd_ptr[L].push_back((int)tupd.size());
-        }
-        launches += 1 + 2 * np + 1;
-    }
+    const MfLayout Y = mf_layout(P, col_ptr, row, goff_ptr);
+    if (Y.tiles < 0) return BL_GPU_ELIMIT;
+    const int nfr = (int)Y.fr.size();
     int rc;
-    if ((rc = upload_vec(c, c->mf_fr, fr)) || (rc = upload_vec(c, c->mf_idx, P.idx)) || (rc = upload_vec(c, c->mf_cmap, P.cmap)) ||
-        (rc = upload_vec(c, c->mf_child, P.child.empty() ? std::vector<int>(1, 0) : P.child)) || (rc = upload_vec(c, c->mf_brow, brow)) ||
-        (rc = upload_vec(c, c->mf_tasm, tasm)) || (rc = upload_vec(c, c->mf_tpan, tpan.empty() ? std::vector<int2>(1) : tpan)) ||
-        (rc = upload_vec(c, c->mf_tupd, tupd.empty() ? std::vector<int4>(1) : tupd)))
+    if ((rc = upload_vec(c, c->mf_fr, Y.fr)) || (rc = upload_vec(c, c->mf_idx, P.idx)) || (rc = upload_vec(c, c->mf_cpos, Y.cpos)) ||
+        (rc = upload_vec(c, c->mf_cptr, Y.cptr)) || (rc = upload_vec(c, c->mf_child, P.child)) || (rc = upload_vec(c, c->mf_eptr, Y.eptr)) ||
+        (rc = upload_vec(c, c->mf_ent, Y.ent)) || (rc = upload_vec(c, c->mf_task, Y.task)))
         return rc;
-    BL_CUDA(c, c->mf_pool.alloc((size_t)std::max(pool, 1LL)));
-    BL_CUDA(c, c->mf_dt.alloc((size_t)std::max(dtn, 1)));
-    c->mf_smem = sizeof(double) * (size_t)maxn;
-    if (c->mf_smem > 200 * 1024) return BL_GPU_ELIMIT; // (a front of more than ~4,200 nodes: its backward solve's vector)
-    if (c->mf_smem > 40 * 1024) BL_CUDA(c, cudaFuncSetAttribute(k_mf_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->mf_smem));
-    c->mf = MfDev{c->mf_fr.p, c->mf_idx.p, c->mf_cmap.p, c->mf_child.p, c->mf_brow.p, c->mf_pool.p, c->mf_dt.p, c->mf_tasm.p, c->mf_tpan.p, c->mf_tupd.p};
-    c->mf_level_ptr = P.level_ptr;
+    BL_CUDA(c, c->mf_pool.alloc((size_t)Y.tiles * kMfTile));
+    BL_CUDA(c, c->mf_ctr.alloc(4 + 2 * (size_t)nfr + (size_t)Y.tiles + Y.pans));
+    MfDev& M = c->mf;
+    M = MfDev{};
+    M.fr = c->mf_fr.p, M.idx = c->mf_idx.p, M.cpos = c->mf_cpos.p, M.cptr = c->mf_cptr.p, M.child = c->mf_child.p, M.eptr = c->mf_eptr.p, M.ent = c->mf_ent.p;
+    M.pool = c->mf_pool.p, M.task = c->mf_task.p, M.ntask = (int)Y.task.size(), M.ncomp = ncomp;
+    M.ctr = c->mf_ctr.p, M.fdone = M.ctr + 4, M.xdone = M.fdone + nfr, M.tflag = M.xdone + nfr, M.xflag = M.tflag + Y.tiles;
+    // a CTA a task of the widest level, at most what is resident at once (a cooperative launch)
+    int per_sm = 0, nsm = 0;
+    BL_CUDA(c, cudaFuncSetAttribute(k_mf_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMfSmem));
+    BL_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mf_solve, kMfThreads, kMfSmem));
+    BL_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->cfg.device));
+    if (per_sm < 1) return BL_GPU_ECUDA;
+    c->mf_grid = std::min(per_sm * nsm, Y.widest);
+    c->mf_levels = (int)P.level_ptr.size() - 1;
     c->mf_flops = P.flops;
-    c->chol_launches = launches;
+    c->chol_launches = 1;
     return BL_GPU_OK;
 }
-
-// fem_dense_front 3 (automatic): the block-column path with its dense top chain while the frames' factorization makes
-// at most this many block updates, the multifrontal one above (measured on B200: the 64 x 64 plate's 1.4 M updates
-// factor in 2.3 ms a substep by block columns against 3.9 ms multifrontal; the 10k-node shell body's 12.6 M in 7.8 ms
-// against 8.0 ms; beyond, the block columns' update lists and levels grow as fast as the fill)
-constexpr int64_t kAutoMultifrontal = 8000000;
 
 static int commit_fem(bl_gpu_ctx* c) {
     int NF = 0, NT = 0, NB = 0, NC = 0, NS = 0, nfem_nodes = 0;
@@ -762,14 +710,11 @@ static int commit_fem(bl_gpu_ctx* c) {
     for (int k = 0; k < NF; k++) bylev[level[k]].push_back(k);
     c->NU = 0; // (the pattern's block updates, whether or not their list was built: sum over columns of d (d + 1) / 2)
     for (int k = 0; k < NF; k++) c->NU += (int64_t)(col_ptr[k + 1] - col_ptr[k]) * (col_ptr[k + 1] - col_ptr[k] + 1) / 2;
-    if (c->cfg.fem_dense_front == 3) {
-        bool lists = c->NU <= kAutoMultifrontal;
-        for (const HostBody& hb : c->bodies)
-            if (hb.fem && fem_update_count(*hb.fem) > 0 && hb.fem->upd.empty()) lists = false;
-        c->fem_mode = lists ? 1 : 2;
-    } else {
-        c->fem_mode = c->cfg.fem_dense_front;
-    }
+    // fem_dense_front 3: the multifrontal one, the fastest at every size measured (B200, a substep's whole FEM step, one
+    // launch for the factorization and both solves against block columns with the dense top chain: a ladder of 82
+    // nodes 0.43 against 0.45 ms, the 21 x 21 plate 0.41 / 0.65, the 64 x 64 plate 1.17 / 2.5; and against the same fronts
+    // factored a launch a panel: the 10k-node shell body 2.25 / 8.0, the 50k-node one 9.6 / 38.6)
+    c->fem_mode = c->cfg.fem_dense_front == 3 ? 2 : c->cfg.fem_dense_front;
     std::vector<std::vector<int>> col_upds(NF);
     for (size_t u = 0; u < gupd.size(); u++) col_upds[upd_col[u]].push_back((int)u);
     c->lvl_grp_ptr.assign(1, 0), c->lvl_col_ptr.assign(1, 0);
@@ -927,7 +872,7 @@ static int commit_fem(bl_gpu_ctx* c) {
         }
         c->chol_launches = 3 * (int64_t)c->front_level;
         if (c->front_level < nlev) c->chol_launches += 1 + c->front.nt + 2 * (c->front.nt - 1) + 2;
-        if (c->fem_mode == 2 && (rc = commit_multifrontal(c, col_ptr, row, col_comp))) return rc;
+        if (c->fem_mode == 2 && (rc = commit_multifrontal(c, col_ptr, row, col_comp, goff_ptr, NC))) return rc;
         c->fem_launches = 4 + (c->NT > 0 ? 1 : 0) + (c->NM > 0 ? 1 : 0) + c->chol_launches; // (begin, triangles, members, assembly, velocity, integration)
     }
     // PCG: vectors, block-Jacobi factors, the grid's partial sums (one cooperative launch: as many blocks as fit)
@@ -1571,21 +1516,15 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
             if (learned) k_mlp_infer<<<(c->NF + kLanes - 1) / kLanes, kLanes, 0, s>>>(F, MD, c->guess.p, c->gscale.p);
             auto cholesky = [c, &F](cudaStream_t cs) {
                 if (c->fem_mode == 2) {
-                    // multifrontal: per level of the front tree its fronts assembled, then panel by panel factored and
-                    // updated with the right side carried along (the forward substitution); the backward from the root down
-                    const MfDev& M = c->mf;
-                    const int nlev = (int)c->mf_level_ptr.size() - 1;
-                    for (int L = 0; L < nlev; L++) {
-                        k_mf_assemble<<<c->mf_tasm_ptr[L + 1] - c->mf_tasm_ptr[L], 256, 0, cs>>>(F, M, c->mf_tasm_ptr[L]);
-                        const std::vector<int>& tp = c->mf_tpan_ptr[L];
-                        const std::vector<int>& tu = c->mf_tupd_ptr[L];
-                        for (size_t sp = 0; sp + 1 < tp.size(); sp++) {
-                            k_mf_panel<<<tp[sp + 1] - tp[sp], 256, 0, cs>>>(M, tp[sp], (int)sp, F.comp_fail);
-                            k_mf_update<<<tu[sp + 1] - tu[sp], 256, 0, cs>>>(M, tu[sp], (int)sp);
-                        }
-                    }
-                    for (int L = nlev - 1; L >= 0; L--)
-                        k_mf_backward<<<c->mf_level_ptr[L + 1] - c->mf_level_ptr[L], 256, c->mf_smem, cs>>>(F, M, c->mf_level_ptr[L]);
+                    // multifrontal: the whole factorization and its solves in one cooperative launch (its flags zeroed first)
+                    cudaMemsetAsync(c->mf_ctr.p, 0, sizeof(int) * c->mf_ctr.n, cs);
+                    cudaLaunchConfig_t lc{};
+                    lc.gridDim = dim3(c->mf_grid), lc.blockDim = dim3(kMfThreads), lc.dynamicSmemBytes = kMfSmem, lc.stream = cs;
+                    cudaLaunchAttribute at[1];
+                    at[0].id = cudaLaunchAttributeCooperative;
+                    at[0].val.cooperative = 1;
+                    lc.attrs = at, lc.numAttrs = 1;
+                    cudaLaunchKernelEx(&lc, k_mf_solve, F, c->mf, c->deverr.p);
                     return;
                 }
                 // the levels of the elimination tree two launches each (factor; updates with the forward substitution),
@@ -2038,7 +1977,6 @@ int bl_gpu_add_body(bl_gpu_ctx* c, const bl_body_desc* d, int32_t* body_id) {
         std::shared_ptr<FemModel> M;
         const int mode = c->cfg.fem_dense_front;
         const int rc = build_fem_model(d->nodes, d->info, d->n_nodes, *d->fem, hb.sections, hb.fsections, M, mode == 0 || mode == 1);
-        if (!rc && mode == 3 && fem_update_count(*M) <= kAutoMultifrontal) fem_update_list(*M); // (the block-column path may be chosen)
         if (rc) return rc;
         hb.fq.assign(4 * M->node.size(), 0.0f);
         for (size_t i = 0; i < M->node.size(); i++) hb.fq[4 * i + 3] = 1.0f;
@@ -2392,7 +2330,7 @@ int bl_gpu_fem_stats(bl_gpu_ctx* c, bl_fem_stats* out) {
     out->columns = c->NF, out->blocks = c->NB, out->updates = c->NU, out->levels = (int64_t)c->lvl_col_ptr.size() - 1;
     out->fronts = c->fem_mode == 2 ? (int64_t)c->mf_fr.n : 0;
     out->factor_flops = c->fem_mode == 2 ? c->mf_flops : 432.0 * (double)c->NU;
-    if (c->fem_mode == 2) out->levels = (int64_t)c->mf_level_ptr.size() - 1;
+    if (c->fem_mode == 2) out->levels = c->mf_levels;
     if (c->any_plastic_members) {
         long long rp = 0;
         BL_CUDA(c, cudaMemcpy(&rp, c->repc.p, sizeof(rp), cudaMemcpyDeviceToHost));
