@@ -21,12 +21,12 @@
 // A pivot that is not positive marks the front's component failed (the reference's chol6 failing, frame_fem.cpp:
 // 2900-2909: that component's step falls back to its explicit forces) and goes on as 1.
 //
-// What bounds it: small frames by the chain of dependent panels (a panel ~16 us: the diagonal tile's 48 dependent columns
-// and inverse 10, a product with its inverse 2.5, the update of the next diagonal tile 2.5, their flags 1 each), large
-// ones by the fp64 rate. 48: a multiple of a node's 6 degrees of freedom and of the instruction's 8, three CTAs an SM
-// with both operands' ring. Measured on B200 (factorization and solves alone; before: the same fronts with a launch a
-// panel and a launch an update, 32 x 32 tiles on the plain fp64 units): the 64 x 64 plate 1.07 ms (3.9), the 10k-node
-// shell body 2.0 (7.8), the 50k-node one 8.8 (38.0: 82.9 GFLOP at 9.4 TFLOP/s of the 35.5 a cuBLAS DGEMM reaches).
+// What bounds it: small frames by the chain of dependent panels (a panel ~11 us: the diagonal tile's inverse factor 5.3, a
+// product with it 2.5, the update of the next diagonal tile 2.5, their flags 1 each), large ones by the fp64 rate. 48:
+// a multiple of a node's 6 degrees of freedom and of the instruction's 8, three CTAs an SM with both operands' ring.
+// Measured on B200 (factorization and solves alone, minimum-degree fronts; before: a launch a panel and a launch an
+// update, 32 x 32 tiles on the plain fp64 units): the 64 x 64 plate 0.86 ms (3.9), the 10k-node shell body 1.68 (7.8),
+// the 50k-node one 7.7 (38.0: 82.9 GFLOP at 10.8 TFLOP/s of the 35.5 a cuBLAS DGEMM reaches).
 #pragma once
 
 #include "bl_fem_kernels.cuh"
@@ -121,124 +121,156 @@ __device__ __forceinline__ int mf_acc_at(int x, int y, int wr, int wc, int lane)
     return (c >> 4) * kMfChunk + (3 * wr + x) * 128 + ((c >> 2) & 3) * 32 + (lane >> 2) * 4 + (c & 3);
 }
 
-constexpr int kMfLd = kMfT + 1; // the plain layout of the diagonal tile's factorization
+// ---- the diagonal tile's factor and its inverse, in 8 x 8 blocks (64 contiguous doubles of a tile)
+__device__ __forceinline__ int mf_blk(int rb, int cb) { return (cb >> 1) * kMfChunk + rb * 128 + (cb & 1) * 64; }
+// acc += A B^T and acc += A B of two blocks, by a warp
+__device__ __forceinline__ void mf_abt8(double (&acc)[2], const double* A, const double* B, int lane) {
+    mf_mma(acc, A[lane], B[lane]);
+    mf_mma(acc, A[32 + lane], B[32 + lane]);
+}
+__device__ __forceinline__ void mf_ab8(double (&acc)[2], const double* A, const double* B, int lane) {
+    const int t = (lane >> 4) * 32 + (lane & 3) * 4 + ((lane >> 2) & 3); // (B's entry (lane & 3, lane >> 2))
+    mf_mma(acc, A[lane], B[t]);
+    mf_mma(acc, A[32 + lane], B[t + 16]);
+}
+// where this lane's pair of an 8 x 8 accumulator lies in a block
+__device__ __forceinline__ int mf_pair8(int lane) { return ((lane & 3) >> 1) * 32 + (lane >> 2) * 4 + 2 * (lane & 1); }
 
-// A panel of 16 columns (c0 ..) of the diagonal tile, rows c0 .. 47, by one warp: lane l holds row c0 + l and, where there
-// is one, row c0 + l + 32. A column's chain is its pivot's broadcast, the inverse square root, a multiply and the next
-// pivot's update, which its own lane makes from its own entry; the other columns' updates read the finished column
-// from shared memory meanwhile.
-__device__ __forceinline__ bool mf_panel16(double (*D)[kMfLd], int c0, int lane) {
-    double a0[16], a1[16];
-    const int r0 = c0 + lane, r1 = c0 + lane + 32;
-    const bool h0 = r0 < kMfT, h1 = r1 < kMfT;
+// 1 / sqrt(s) for a normal s > 0 without a branch (the panel's other work is scheduled into its latency): the
+// instruction's 20-bit approximation y, then one step of Householder's third-order iteration,
+// y (1 + e / 2 + 3 e^2 / 8) with e = 1 - s y^2 (e below 2^-18 leaves 5 e^3 / 16, under a tenth of an ulp)
+__device__ __forceinline__ double mf_rsqrt(double s) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+    const double e = fma(-(s * y), y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// The inverse of an 8 x 8 block's Cholesky factor, by one warp: every lane factors the block in its own registers, so
+// that a column's chain is the inverse square root, a multiply and a multiply-add with no exchange of lanes; lane i < 8
+// carries row i of an identity along, which comes out as column i of the inverse. (Lanes a row each and the columns
+// broadcast by shuffles: 190 cycles a column against 85.) False at a pivot that is not positive.
+__device__ __forceinline__ bool mf_inv8(const double* B, double* inv, int lane) {
+    double d[8][8], a[8];
 #pragma unroll
-    for (int j = 0; j < 16; j++) a0[j] = h0 ? D[r0][c0 + j] : 0.0, a1[j] = h1 ? D[r1][c0 + j] : 0.0;
+    for (int r = 0; r < 8; r++)
+#pragma unroll
+        for (int c = 0; c <= r; c += 2) {
+            const double2 u = *reinterpret_cast<const double2*>(B + (c >> 2) * 32 + r * 4 + (c & 3));
+            d[r][c] = u.x, d[r][c + 1] = u.y;
+        }
+#pragma unroll
+    for (int c = 0; c < 8; c++) a[c] = c == lane ? 1.0 : 0.0;
     bool ok = true;
-    double piv = a0[0];
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
-        double s = __shfl_sync(0xffffffffu, piv, j);
-        if (!(s > 0)) ok = false, s = 1.0;
-        const double id = rsqrt(s);
-        a0[j] = lane == j ? s * id : a0[j] * id;
-        a1[j] *= id;
-        if (j < 15) piv = fma(-a0[j], a0[j], a0[j + 1]); // (lane j + 1's next pivot)
-        if (h0) D[r0][c0 + j] = lane >= j ? a0[j] : 0.0;
-        if (h1) D[r1][c0 + j] = a1[j];
-        if (lane == j) D[r0][kMfT] = id; // (the pad column: the pivots' inverses)
-        __syncwarp();
+    for (int j = 0; j < 8; j++) {
+        const bool good = d[j][j] >= 2.2250738585072014e-308;
+        ok = ok && good;
+        double id = mf_rsqrt(d[j][j]);
+        id = good ? id : 1.0; // (after the root, as a select: the test is off the chain)
 #pragma unroll
-        for (int l = j + 1; l < 16; l++) {
-            const double t = D[c0 + l][c0 + j];
-            a0[l] = fma(-a0[j], t, a0[l]), a1[l] = fma(-a1[j], t, a1[l]);
+        for (int l = j + 1; l < 8; l++) d[l][j] *= id;
+        a[j] *= id;
+#pragma unroll
+        for (int l = j + 1; l < 8; l++) {
+#pragma unroll
+            for (int m = j + 1; m <= l; m++) d[l][m] = fma(-d[l][j], d[m][j], d[l][m]);
+            a[l] = fma(-a[j], d[l][j], a[l]);
         }
     }
+    if (lane < 8)
+#pragma unroll
+        for (int r = 0; r < 8; r++) inv[(lane >> 2) * 32 + r * 4 + (lane & 3)] = r >= lane ? a[r] : 0.0;
     return ok;
 }
 
-// The inverse of the 16 x 16 lower triangle at c0, by one warp (lane c < 16: column c), into Y
-__device__ __forceinline__ void mf_inv16(double (*D)[kMfLd], double (*Y)[kMfLd], int c0, int lane) {
-    if (lane >= 16) return;
-    double x[16];
-#pragma unroll
-    for (int r = 0; r < 16; r++) x[r] = r == lane ? 1.0 : 0.0;
-#pragma unroll
-    for (int r = 0; r < 16; r++) {
-        x[r] *= D[c0 + r][kMfT];
-#pragma unroll
-        for (int q = r + 1; q < 16; q++) x[q] = fma(-D[c0 + q][c0 + r], x[r], x[q]);
-    }
-#pragma unroll
-    for (int r = 0; r < 16; r++) Y[c0 + r][c0 + lane] = x[r];
-}
-
-// Z (16 x 16 at zr, zc) = s A (ar, ac) B (br, bc), by the whole block, two entries a thread
-__device__ __forceinline__ void mf_mul16(double (*Z)[kMfLd], int zr, int zc, double (*A)[kMfLd], int ar, int ac, double (*B)[kMfLd], int br, int bc,
-                                         double s, bool add) {
-    const int r = threadIdx.x >> 3, c = threadIdx.x & 7;
-    double t0 = 0, t1 = 0;
-#pragma unroll
-    for (int m = 0; m < 16; m++) {
-        const double a = A[ar + r][ac + m];
-        t0 = fma(a, B[br + m][bc + c], t0), t1 = fma(a, B[br + m][bc + c + 8], t1);
-    }
-    if (add) t0 = fma(s, t0, Z[zr + r][zc + c]), t1 = fma(s, t1, Z[zr + r][zc + c + 8]);
-    else t0 *= s, t1 *= s;
-    Z[zr + r][zc + c] = t0, Z[zr + r][zc + c + 8] = t1;
-}
-
-// The diagonal tile's Cholesky factor and the factor's inverse: D (plain, lower) in, Y out. Three panels of 16 columns by
-// the first warp, each followed by the block's update of the columns after it while the second warp inverts the
-// panel's triangle; then the inverse's blocks below the diagonal. False at a pivot that is not positive.
-__device__ __forceinline__ bool mf_factor_tile(double (*D)[kMfLd], double (*Y)[kMfLd], int* bad) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int kb = 0; kb < 3; kb++) {
-        const int c0 = 16 * kb;
+// The inverse Y of the diagonal tile's Cholesky factor (lower; zero before); D (lower) is overwritten by the factor's
+// blocks below the diagonal. By columns of 8: the first warp makes the chain - L_(k+1)k = D_(k+1)k inv_k^T, the next
+// diagonal block less L L^T, its factor's inverse inv_(k+1) - while the other three make the rest of the block column,
+// the later blocks' updates and the inverse's rows: Y_kk = inv_k, Y_kj = -inv_k S_j, then the next row's
+// S_j = sum_(j <= m <= k) L_(k+1)m Y_mj; a warp keeps its columns j (j mod 3). One barrier a column of blocks. The chain
+// bounds it: 48 columns of an inverse square root, a multiply and a multiply-add. scr: 5 blocks of S, 2 of inverses in
+// turn, the chain's L. False at a pivot that is not positive.
+// (9.6 us with panels of 16 columns, plain multiply-adds for the updates and the inverse after them.)
+constexpr int kMfScr = 8 * 64;
+__device__ __forceinline__ bool mf_factor_tile(double* D, double* Y, double* scr, int* bad) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w = warp - 1, pr = mf_pair8(lane);
+    double *S = scr, *inv = scr + 5 * 64;
+    auto at2 = [&](double* p) -> double2& { return *reinterpret_cast<double2*>(p + pr); };
+    if (warp == 0 && !mf_inv8(D, inv, lane) && lane == 0) *bad = 1;
+    __syncthreads();
+    for (int kb = 0; kb < 6; kb++) {
+        const double* ik = inv + 64 * (kb & 1);
         if (warp == 0) {
-            if (!mf_panel16(D, c0, lane) && lane == 0) *bad = 1;
-        } else if (kb > 0 && warp == 1) {
-            mf_inv16(D, Y, c0 - 16, lane);
-        }
-        __syncthreads();
-        // the columns after the panel, lower triangle: D_rc -= sum_m L_rm L_cm, 8 (2) entries a thread
-        if (kb == 0) {
-            const int r = 16 + (tid >> 2), q = tid & 3; // (row r; columns 16 + q + 4 x)
-            double t[8];
+            if (kb < 5) {
+                double* L = D + mf_blk(kb + 1, kb);
+                double* N = D + mf_blk(kb + 1, kb + 1);
+                double t[2] = {0.0, 0.0}, u[2] = {0.0, 0.0};
+                mf_abt8(t, L, ik, lane);
+                at2(S + 7 * 64) = make_double2(t[0], t[1]); // (the chain's own copy: another warp stores L for the rest)
+                asm volatile("bar.arrive 2, 128;" ::: "memory");
+                __syncwarp();
+                mf_abt8(u, S + 7 * 64, S + 7 * 64, lane);
+                at2(N) = make_double2(at2(N).x - u[0], at2(N).y - u[1]);
+                __syncwarp();
+                if (!mf_inv8(N, inv + 64 * ((kb + 1) & 1), lane) && lane == 0) *bad = 1;
+            }
+        } else {
+            // the block column: rows kb + 1 + w, kb + 4 + w
+            double t[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
 #pragma unroll
-            for (int x = 0; x < 8; x++) t[x] = 0;
+            for (int x = 0; x < 2; x++)
+                if (kb + 1 + w + 3 * x < 6) mf_abt8(t[x], D + mf_blk(kb + 1 + w + 3 * x, kb), ik, lane);
+            // (the chain reads D_(k+1)k too, at the start of this step: its copy is made before this one is stored)
+            if (kb < 5) asm volatile("bar.sync 2, 128;" ::: "memory");
 #pragma unroll
-            for (int m = 0; m < 16; m++) {
-                const double l = D[r][m];
+            for (int x = 0; x < 2; x++)
+                if (kb + 1 + w + 3 * x < 6) at2(D + mf_blk(kb + 1 + w + 3 * x, kb)) = make_double2(t[x][0], t[x][1]);
+            // the inverse's row kb
 #pragma unroll
-                for (int x = 0; x < 8; x++) t[x] = fma(l, D[16 + q + 4 * x][m], t[x]);
+            for (int x = 0; x < 2; x++) {
+                const int j = w + 3 * x;
+                if (j < kb) {
+                    double u[2] = {0.0, 0.0};
+                    mf_ab8(u, ik, S + 64 * j, lane);
+                    at2(Y + mf_blk(kb, j)) = make_double2(-u[0], -u[1]);
+                } else if (j == kb) {
+                    at2(Y + mf_blk(kb, j)) = *reinterpret_cast<const double2*>(ik + pr);
+                }
+            }
+            asm volatile("bar.sync 1, 96;" ::: "memory"); // (the three warps: the block column is there)
+            // the later blocks (rb, cb), cb > kb, but the chain's; pairs by descending cb, at most five a warp
+            const int nb = (5 - kb) * (6 - kb) / 2;
+            double v[5][2];
+            int at[5];
+#pragma unroll
+            for (int x = 0; x < 5; x++) {
+                const int b = w + 3 * x;
+                v[x][0] = v[x][1] = 0.0, at[x] = -1;
+                if (b >= nb) continue;
+                const int cb = b < 1 ? 5 : b < 3 ? 4 : b < 6 ? 3 : b < 10 ? 2 : 1, rb = cb + b - (b < 1 ? 0 : b < 3 ? 1 : b < 6 ? 3 : b < 10 ? 6 : 10);
+                if (rb == kb + 1) continue;
+                mf_abt8(v[x], D + mf_blk(rb, kb), D + mf_blk(cb, kb), lane);
+                at[x] = mf_blk(rb, cb);
             }
 #pragma unroll
-            for (int x = 0; x < 8; x++)
-                if (16 + q + 4 * x <= r) D[r][16 + q + 4 * x] -= t[x];
-        } else if (kb == 1) {
-            const int r = 32 + (tid >> 3), q = tid & 7;
-            double t0 = 0, t1 = 0;
+            for (int x = 0; x < 5; x++)
+                if (at[x] >= 0) at2(D + at[x]) = make_double2(at2(D + at[x]).x - v[x][0], at2(D + at[x]).y - v[x][1]);
+            if (kb < 5)
 #pragma unroll
-            for (int m = 16; m < 32; m++) t0 = fma(D[r][m], D[32 + q][m], t0), t1 = fma(D[r][m], D[40 + q][m], t1);
-            if (32 + q <= r) D[r][32 + q] -= t0;
-            if (40 + q <= r) D[r][40 + q] -= t1;
+                for (int x = 0; x < 2; x++) {
+                    const int j = w + 3 * x;
+                    if (j > kb) continue;
+                    double u[2][2] = {{0.0, 0.0}, {0.0, 0.0}}; // (two sums: the instruction's latency)
+                    for (int m = j; m <= kb; m += 2) {
+                        mf_ab8(u[0], D + mf_blk(kb + 1, m), Y + mf_blk(m, j), lane);
+                        if (m + 1 <= kb) mf_ab8(u[1], D + mf_blk(kb + 1, m + 1), Y + mf_blk(m + 1, j), lane);
+                    }
+                    at2(S + 64 * j) = make_double2(u[0][0] + u[1][0], u[0][1] + u[1][1]);
+                }
         }
-        if (kb < 2) __syncthreads();
+        __syncthreads();
     }
-    // the inverse: Y00, Y11 there, Y22 now; T = L10 Y00, Y10 = -Y11 T; U = L20 Y00 + L21 Y10, W = L21 Y11;
-    // Y20 = -Y22 U, Y21 = -Y22 W (T, U, W in D's upper blocks (0, 1), (0, 2), (1, 2))
-    if (warp == 3) mf_inv16(D, Y, 32, lane);
-    mf_mul16(D, 0, 16, D, 16, 0, Y, 0, 0, 1.0, false);
-    mf_mul16(D, 0, 32, D, 32, 0, Y, 0, 0, 1.0, false);
-    mf_mul16(D, 16, 32, D, 32, 16, Y, 16, 16, 1.0, false);
-    __syncthreads();
-    mf_mul16(Y, 16, 0, Y, 16, 16, D, 0, 16, -1.0, false);
-    mf_mul16(Y, 32, 16, Y, 32, 32, D, 16, 32, -1.0, false);
-    __syncthreads();
-    mf_mul16(D, 0, 32, D, 32, 16, Y, 16, 0, 1.0, true);
-    __syncthreads();
-    mf_mul16(Y, 32, 0, Y, 32, 32, D, 0, 32, -1.0, false);
-    __syncthreads();
     return *bad == 0;
 }
 
@@ -364,25 +396,19 @@ __device__ bool mf_tile(const FemDev& F, const MfDev& M, const MfFrontDev& fr, i
         return true;
     }
     if (same) {
-        double(*D)[kMfLd] = reinterpret_cast<double(*)[kMfLd]>(ring);
-        double(*Y)[kMfLd] = D + kMfT;
+        double* Y = ring;
         if (tid == 0) s_bad = 0;
+        for (int e = tid; e < kMfTile / 2; e += kMfThreads) reinterpret_cast<double2*>(Y)[e] = make_double2(0.0, 0.0);
 #pragma unroll
         for (int x = 0; x < 3; x++)
 #pragma unroll
             for (int y = 0; y < 3; y++) {
-                const double2 c = *reinterpret_cast<const double2*>(C + mf_acc_at(x, y, wr, wc, lane));
-                const int r = 8 * (3 * wr + x) + (lane >> 2), cc = 8 * (3 * wc + y) + 2 * (lane & 3);
-                D[r][cc] = c.x - acc[x][y][0], D[r][cc + 1] = c.y - acc[x][y][1];
+                double2* c = reinterpret_cast<double2*>(C + mf_acc_at(x, y, wr, wc, lane));
+                *c = make_double2(c->x - acc[x][y][0], c->y - acc[x][y][1]);
             }
-        for (int e = tid; e < kMfT * kMfLd; e += kMfThreads) (&Y[0][0])[e] = 0.0;
         __syncthreads();
-        const bool ok = mf_factor_tile(D, Y, &s_bad);
-        for (int e = tid; e < kMfTile / 2; e += kMfThreads) { // (the pair e of the tile's order)
-            const int kc = e / (kMfChunk / 2), q = e % (kMfChunk / 2), rb = q / 64, cb = (q / 16) & 3, l = 2 * (q & 15);
-            const int r = 8 * rb + l / 4, c = 16 * kc + 4 * cb + l % 4;
-            reinterpret_cast<double2*>(out)[e] = make_double2(Y[r][c], Y[r][c + 1]);
-        }
+        const bool ok = mf_factor_tile(C, Y, ring + kMfTile, &s_bad);
+        for (int e = tid; e < kMfTile / 2; e += kMfThreads) reinterpret_cast<double2*>(out)[e] = reinterpret_cast<const double2*>(Y)[e];
         if (!ok && tid == 0) atomicExch(&F.comp_fail[fr.comp], 1);
     } else {
         // X = A L_jj^-T
