@@ -1,9 +1,8 @@
 // Host side of the multifrontal factorization of a frame's implicit step (the kernels: bl_multifrontal.cuh).
 //
 // The reference factors the step's block system column by column, right-looking, with the exact minimum-degree order
-// of its symbolic phase (frame_fem.cpp:2887-2920). The same order is kept here - the fill, and so the factor's
-// nonzeros, are the reference's - but the columns are grouped into fronts: dense blocks factored with dense kernels,
-// which is where a GPU is fast.
+// of its symbolic phase (frame_fem.cpp:2887-2920). Here the columns come in a nested-dissection order (FemDissection,
+// bl_fem_host.cuh) and are grouped into fronts: dense blocks factored with dense kernels, which is where a GPU is fast.
 //  * Elimination tree: column k's parent is its first off-diagonal row.
 //  * Fundamental supernodes: a column joins its parent's group when it is that parent's only child and its rows are the
 //    parent and the parent's rows (the columns then share one dense structure).
@@ -45,10 +44,10 @@ struct MfPlan {
 };
 
 struct MfParams { // relaxed amalgamation, in frame nodes (CHOLMOD's rule of thumb, scaled to 6 x 6 blocks)
-    int small = 4;        // merged groups up to this many columns merge whatever their zeros
-    int mid = 16;         // ... up to this many, while zeros stay under mid_frac of the entries
+    int small = 2;        // merged groups up to this many columns merge whatever their zeros
+    int mid = 8;          // ... up to this many, while zeros stay under mid_frac of the entries
     double mid_frac = 0.5;
-    int large = 48;
+    int large = 24;
     double large_frac = 0.1;
     double huge_frac = 0.05;
 };

@@ -24,9 +24,9 @@
 // What bounds it: small frames by the chain of dependent panels (a panel ~11 us: the diagonal tile's inverse factor 5.3, a
 // product with it 2.5, the update of the next diagonal tile 2.5, their flags 1 each), large ones by the fp64 rate. 48:
 // a multiple of a node's 6 degrees of freedom and of the instruction's 8, three CTAs an SM with both operands' ring.
-// Measured on B200 (factorization and solves alone, minimum-degree fronts; before: a launch a panel and a launch an
-// update, 32 x 32 tiles on the plain fp64 units): the 64 x 64 plate 0.86 ms (3.9), the 10k-node shell body 1.68 (7.8),
-// the 50k-node one 7.7 (38.0: 82.9 GFLOP at 10.8 TFLOP/s of the 35.5 a cuBLAS DGEMM reaches).
+// Measured on B200 (factorization and solves alone; before: minimum-degree fronts, a launch a panel and a launch an
+// update, 32 x 32 tiles on the plain fp64 units): the 64 x 64 plate 0.63 ms (3.9), the 10k-node shell body 1.52 (7.8),
+// the 50k-node one 6.7 (38.0): 63.3 GFLOP at 9.4 TFLOP/s of the 35.5 a cuBLAS DGEMM reaches.
 #pragma once
 
 #include "bl_fem_kernels.cuh"

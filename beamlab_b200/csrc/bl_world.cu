@@ -710,10 +710,9 @@ static int commit_fem(bl_gpu_ctx* c) {
     for (int k = 0; k < NF; k++) bylev[level[k]].push_back(k);
     c->NU = 0; // (the pattern's block updates, whether or not their list was built: sum over columns of d (d + 1) / 2)
     for (int k = 0; k < NF; k++) c->NU += (int64_t)(col_ptr[k + 1] - col_ptr[k]) * (col_ptr[k + 1] - col_ptr[k] + 1) / 2;
-    // fem_dense_front 3: the multifrontal one, the fastest at every size measured (B200, a substep's whole FEM step, one
-    // launch for the factorization and both solves against block columns with the dense top chain: a ladder of 82
-    // nodes 0.43 against 0.45 ms, the 21 x 21 plate 0.41 / 0.65, the 64 x 64 plate 1.17 / 2.5; and against the same fronts
-    // factored a launch a panel: the 10k-node shell body 2.25 / 8.0, the 50k-node one 9.6 / 38.6)
+    // fem_dense_front 3: the multifrontal one, the fastest at every size measured (B200, a substep, against block columns
+    // with the dense top chain: a ladder of 82 nodes 0.35 against 0.45 ms, the 21 x 21 plate 0.32 / 0.65, the 64 x 64
+    // plate 0.74 / 2.5, the 10k-node shell body 1.7 / 7.6)
     c->fem_mode = c->cfg.fem_dense_front == 3 ? 2 : c->cfg.fem_dense_front;
     std::vector<std::vector<int>> col_upds(NF);
     for (size_t u = 0; u < gupd.size(); u++) col_upds[upd_col[u]].push_back((int)u);
@@ -1618,7 +1617,7 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
 // A body's FEM frame of triangle elements made ready (bl_fem_host.cuh): frame nodes in the order FemFrame::add_tri
 // makes them, FemFrame::finalize's rest shapes and inertias, analyse's pattern, the elements' stiffnesses.
 static int build_fem_model(const bl_node* nodes, const bl_node_info* info, int32_t n_nodes, const bl_fem_desc& fd, std::vector<FemSection>& sections,
-                           std::vector<FrameSectionH>& fsections, std::shared_ptr<FemModel>& out, bool want_updates = true) {
+                           std::vector<FrameSectionH>& fsections, std::shared_ptr<FemModel>& out, bool want_updates = true, bool nested = false) {
     if (fd.n_tris < 0 || fd.n_members < 0 || (fd.n_tris > 0 && (!fd.tris || !fd.sections || fd.n_sections <= 0)) ||
         (fd.n_members > 0 && (!fd.members || !fd.frame_sections || fd.n_frame_sections <= 0)) || fd.n_tris + fd.n_members == 0 || !nodes || !info)
         return BL_GPU_EINVAL;
@@ -1680,7 +1679,7 @@ static int build_fem_model(const bl_node* nodes, const bl_node_info* info, int32
     for (size_t t = 0; t < M->tn.size(); t++) // (the caller's mass, else its section's over its area: tri_mass, frame_fem.h:373)
         if (!(M->tmass[t] > 0)) M->tmass[t] = sections[M->tsec[t]].rho * sections[M->tsec[t]].t * M->tarea0[t], again = true;
     if (again) fem_finalize(*M, px.data(), py.data(), pz.data(), ms.data(), mpm); // (the inertias from those masses)
-    fem_analyse(*M, want_updates);
+    fem_analyse(*M, want_updates, nested);
     M->tk.assign(162 * M->tn.size(), 0.0f), M->tb.assign(54 * M->tn.size(), 0.0f);
     for (size_t t = 0; t < M->tn.size(); t++) {
         if (M->tbroken[t]) continue;
@@ -1976,7 +1975,7 @@ int bl_gpu_add_body(bl_gpu_ctx* c, const bl_body_desc* d, int32_t* body_id) {
     if (d->fem && (d->fem->n_tris > 0 || d->fem->n_members > 0)) {
         std::shared_ptr<FemModel> M;
         const int mode = c->cfg.fem_dense_front;
-        const int rc = build_fem_model(d->nodes, d->info, d->n_nodes, *d->fem, hb.sections, hb.fsections, M, mode == 0 || mode == 1);
+        const int rc = build_fem_model(d->nodes, d->info, d->n_nodes, *d->fem, hb.sections, hb.fsections, M, mode == 0 || mode == 1, mode == 2 || mode == 3);
         if (rc) return rc;
         hb.fq.assign(4 * M->node.size(), 0.0f);
         for (size_t i = 0; i < M->node.size(); i++) hb.fq[4 * i + 3] = 1.0f;

@@ -88,11 +88,12 @@ typedef struct {
     int32_t beam_kernel;       /* 0 (default): the beams' kernel streams the beam arrays through shared memory by bulk
                                   (TMA) copies and the nodes' kernel reads 4-byte incidences where the rig allows; 1:
                                   plain loads and 8-byte incidences. Results are the same. */
-    int32_t fem_dense_front;   /* how the FEM step factors its system (the same pattern and fill as the reference's):
+    int32_t fem_dense_front;   /* how the FEM step factors its system:
                                   3 (default): 2;
-                                  2: multifrontal - the columns grouped into dense fronts (supernodes of the elimination
-                                  tree, small ones amalgamated) of 48 x 48 tiles, the whole factorization and both solves
-                                  one launch; 1: block column by block column, with the top chain of the elimination tree
+                                  2: multifrontal - the columns in a nested-dissection order, grouped into dense fronts
+                                  (supernodes of the elimination tree, small ones amalgamated) of 48 x 48 tiles, the whole
+                                  factorization and both solves one launch; with the reference's order, pattern and fill
+                                  1: block column by block column, with the top chain of the elimination tree
                                   (levels of one column each) as one dense front; 0: block column by block column in the
                                   reference's order of sums throughout. 2 and 1 differ from 0 in the order of the
                                   floating-point sums only. */
