@@ -12,9 +12,8 @@
 //                      tree: the level's columns factored (chol6, right_solve_lt), then their updates T -= P Q^T, one
 //                      warp per target block (frame_fem.cpp:2193-2220, 2887-2919), with the level's L y = r
 //   k_fem_backward_level: L^T x = y by levels, from the top down (frame_fem.cpp:2944-2954)
-//   k_fem_velocity     columns: the new velocities to forces m dv / step, spins advanced, safety clamps
-//                      (frame_fem.cpp:2998-3025)
-//   k_fem_integrate    the frame bodies' nodes: SoftBody::integrate_nodes, then FemFrame::sync_positions
+//   k_fem_integrate    the frame bodies' nodes: the new velocities as forces m dv / step, spins advanced, safety clamps
+//                      (frame_fem.cpp:2998-3025); SoftBody::integrate_nodes, then FemFrame::sync_positions
 //                      (softbody.cpp:769-795, frame_fem.cpp:3407-3422)
 // The factorization's sums per block are the reference's (same 6 x 6 loops, same order of updates); the element
 // kernels call the GPU's atan2 / sin / cos, which differ from libm's in the last bit, so the step matches the reference
@@ -532,59 +531,62 @@ __device__ __forceinline__ void condense(float c[3], bool pin_a, bool pin_b) {
 // [u_a, phi_a, u_b, phi_b] to the six deformations - elongation e1.(u_b - u_a), twist e1.(phi_b - phi_a), each end's
 // rotation about e2 against the chord e2.phi + e3.(u_b - u_a) / L and about e3 e3.phi - e2.(u_b - u_a) / L - and D is
 // ka, kt and the two planes' end pairs. Stored as its four 6 x 6 world blocks with K v at the ends' velocities.
-__device__ void member_world_k(const FemDev& F, const float4* __restrict__ nd, int ei, int2 ab, v3 e1, v3 e2, v3 e3, float L, float ka, float kt,
-                               const float cy_in[3], const float cz_in[3], uint32_t y) {
+//
+// By a warp, every lane with the same arguments: lane q < 12 (and q + 12) makes column q of B and of D B in registers and
+// shares B's; then rows 0-5 (6-11) of K's column q, and its part of K v from K's symmetry. Bs: the warp's 72 doubles.
+// (A thread a member, its B, D B and K in local memory: k_member_eval 34 us at 121 members; 9 so.)
+__device__ __forceinline__ void member_world_k(const FemDev& F, const float4* __restrict__ nd, int ei, int2 ab, v3 e1, v3 e2, v3 e3, float L, float ka,
+                                               float kt, const float cy_in[3], const float cz_in[3], uint32_t y, double* Bs) {
     float cy[3] = {cy_in[0], cy_in[1], cy_in[2]}, cz[3] = {cz_in[0], cz_in[1], cz_in[2]};
     if (y & 3) condense(cy, y & 1, y & 2), condense(cz, y & 1, y & 2);
     if (y & 4) ka *= 0.01f;
     if (y & 8) kt *= 0.01f;
+    const int lane = threadIdx.x & 31, q = lane % 12, half = lane < 12 ? 0 : 1, j = q % 3, dof = q / 3; // (dof: u_a, phi_a, u_b, phi_b)
     const double iL = 1.0 / L;
-    const double a1[3] = {e1.x, e1.y, e1.z}, a2[3] = {e2.x, e2.y, e2.z}, a3[3] = {e3.x, e3.y, e3.z};
-    double B[6][12];
-    for (int r = 0; r < 6; r++)
-        for (int q = 0; q < 12; q++) B[r][q] = 0;
-    for (int j = 0; j < 3; j++) {
-        const double g = a3[j] * iL, h = a2[j] * iL;
-        B[0][j] = -a1[j], B[0][6 + j] = a1[j];
-        B[1][3 + j] = -a1[j], B[1][9 + j] = a1[j];
-        B[2][j] = -g, B[2][6 + j] = g, B[2][3 + j] = a2[j];
-        B[3][j] = -g, B[3][6 + j] = g, B[3][9 + j] = a2[j];
-        B[4][j] = h, B[4][6 + j] = -h, B[4][3 + j] = a3[j];
-        B[5][j] = h, B[5][6 + j] = -h, B[5][9 + j] = a3[j];
+    const double a1 = j == 0 ? e1.x : j == 1 ? e1.y : e1.z, a2 = j == 0 ? e2.x : j == 1 ? e2.y : e2.z, a3 = j == 0 ? e3.x : j == 1 ? e3.y : e3.z;
+    const double g = a3 * iL, h = a2 * iL, sg = dof < 2 ? -1.0 : 1.0;
+    double b[6] = {0, 0, 0, 0, 0, 0};
+    if (dof == 0 || dof == 2) b[0] = sg * a1, b[2] = b[3] = sg * g, b[4] = b[5] = -sg * h;
+    else if (dof == 1) b[1] = -a1, b[2] = a2, b[4] = a3;
+    else b[1] = a1, b[3] = a2, b[5] = a3;
+    const double db[6] = {(double)ka * b[0], (double)kt * b[1], (double)cy[0] * b[2] + (double)cy[1] * b[3], (double)cy[1] * b[2] + (double)cy[2] * b[3],
+                          (double)cz[0] * b[4] + (double)cz[1] * b[5], (double)cz[1] * b[4] + (double)cz[2] * b[5]};
+    __syncwarp();
+    if (lane < 12)
+#pragma unroll
+        for (int k = 0; k < 6; k++) Bs[6 * q + k] = b[k];
+    __syncwarp();
+    double K[6];
+#pragma unroll
+    for (int r = 0; r < 6; r++) {
+        K[r] = 0;
+#pragma unroll
+        for (int k = 0; k < 6; k++) K[r] += Bs[6 * (6 * half + r) + k] * db[k];
     }
-    double DB[6][12];
-    for (int q = 0; q < 12; q++) {
-        DB[0][q] = (double)ka * B[0][q], DB[1][q] = (double)kt * B[1][q];
-        DB[2][q] = (double)cy[0] * B[2][q] + (double)cy[1] * B[3][q], DB[3][q] = (double)cy[1] * B[2][q] + (double)cy[2] * B[3][q];
-        DB[4][q] = (double)cz[0] * B[4][q] + (double)cz[1] * B[5][q], DB[5][q] = (double)cz[1] * B[4][q] + (double)cz[2] * B[5][q];
+    double* W = F.mkw + 144 * (size_t)ei; // (blocks aa, bb, ba, ab)
+    if (lane < 24) {
+        double* blk = W + (half == 0 ? (q < 6 ? 0 : 108) : (q < 6 ? 72 : 36)) + q % 6;
+#pragma unroll
+        for (int r = 0; r < 6; r++) blk[6 * r] = K[r];
     }
-    double K[12][12];
-    for (int r = 0; r < 12; r++)
-        for (int q = r; q < 12; q++) {
-            double v = 0;
-            for (int k = 0; k < 6; k++) v += B[k][r] * DB[k][q];
-            K[r][q] = K[q][r] = v;
-        }
-    double* W = F.mkw + 144 * (size_t)ei;
-    for (int r = 0; r < 6; r++)
-        for (int q = 0; q < 6; q++)
-            W[r * 6 + q] = K[r][q], W[36 + r * 6 + q] = K[6 + r][6 + q], W[72 + r * 6 + q] = K[6 + r][q], W[108 + r * 6 + q] = K[r][6 + q];
-    const float4 va = nd[2 * F.fnode[ab.x] + 1], vb = nd[2 * F.fnode[ab.y] + 1], wa = F.w[ab.x], wb = F.w[ab.y];
-    const double u[12] = {va.x, va.y, va.z, wa.x, wa.y, wa.z, vb.x, vb.y, vb.z, wb.x, wb.y, wb.z};
-    double* kv = F.mkv + 12 * (size_t)ei;
-    for (int r = 0; r < 12; r++) {
-        double s2 = 0;
-        for (int q = 0; q < 12; q++) s2 += K[r][q] * u[q];
-        kv[r] = s2;
-    }
+    const int end = half == 0 ? ab.x : ab.y;
+    const float4 v = nd[2 * F.fnode[end] + 1], w = F.w[end];
+    const double u[6] = {v.x, v.y, v.z, w.x, w.y, w.z};
+    double s2 = 0;
+#pragma unroll
+    for (int r = 0; r < 6; r++) s2 += K[r] * u[r];
+    const double other = __shfl_sync(0xffffffffu, s2, q + 12);
+    if (lane < 12) F.mkv[12 * (size_t)ei + q] = s2 + other;
 }
 
 template <bool kPlastic>
 __global__ void __launch_bounds__(128) k_member_eval(FemDev F, const float4* __restrict__ nd) {
-    const int ei = blockIdx.x * blockDim.x + threadIdx.x;
+    // (a warp a member: every lane the same kinematics and forces, lane 0's stored; the tangent by all lanes)
+    __shared__ double Bs[4][72];
+    const int ei = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (ei >= F.nmem) return;
-    F.mon[ei] = 0;
     const int meta = F.mmeta[ei];
+    if (lane == 0) F.mon[ei] = 0;
     if (meta < 0) return; // (broken: no length at rest)
     const int2 ab = F.mn[ei];
     const int endA = (meta >> 16) & 0xff, endB = (meta >> 24) & 0x7f;
@@ -683,37 +685,40 @@ __global__ void __launch_bounds__(128) k_member_eval(FemDev F, const float4* __r
     const v3 fav = e1 * N + e3 * (Sy / L) - e2 * (Sz / L);
     const v3 tav = e1 * T - e2 * Max - e3 * May;
     const v3 tbv = e1 * (-T) - e2 * Mbx - e3 * Mby;
-    F.mfa[ei] = make_float4(fav.x, fav.y, fav.z, 0.0f);
-    F.mta[ei] = make_float4(tav.x, tav.y, tav.z, 0.0f);
-    F.mtb[ei] = make_float4(tbv.x, tbv.y, tbv.z, 0.0f);
+    if (lane == 0) {
+        F.mfa[ei] = make_float4(fav.x, fav.y, fav.z, 0.0f);
+        F.mta[ei] = make_float4(tav.x, tav.y, tav.z, 0.0f);
+        F.mtb[ei] = make_float4(tbv.x, tbv.y, tbv.z, 0.0f);
+    }
     uint32_t y = 0;
     if (kPlastic) {
+        __syncwarp(); // (every lane has read the state that lane 0 writes below)
         // the plastic rotations into the rest frames past 0.02 rad, the twist half into each end (frame_fem.cpp:
         // 2045-2054)
         const float kBake = 0.02f;
         if (pax * pax + pay * pay > kBake * kBake) {
             const float4 q = F.mq[2 * ei];
             const q4 n = qnormalize(qmul(q4{q.x, q.y, q.z, q.w}, quat_exp(V(0, -pax, -pay))));
-            F.mq[2 * ei] = make_float4(n.x, n.y, n.z, n.w);
+            if (lane == 0) F.mq[2 * ei] = make_float4(n.x, n.y, n.z, n.w);
             bax = bax + pax, bay = bay + pay, pax = pay = 0;
         }
         if (pbx * pbx + pby * pby > kBake * kBake) {
             const float4 q = F.mq[2 * ei + 1];
             const q4 n = qnormalize(qmul(q4{q.x, q.y, q.z, q.w}, quat_exp(V(0, -pbx, -pby))));
-            F.mq[2 * ei + 1] = make_float4(n.x, n.y, n.z, n.w);
+            if (lane == 0) F.mq[2 * ei + 1] = make_float4(n.x, n.y, n.z, n.w);
             bbx = bbx + pbx, bby = bby + pby, pbx = pby = 0;
         }
         if (fabsf(tp) > kBake) {
             const float4 qa = F.mq[2 * ei], qb = F.mq[2 * ei + 1];
             const q4 na = qnormalize(qmul(q4{qa.x, qa.y, qa.z, qa.w}, quat_exp(V(0.5f * tp, 0, 0))));
             const q4 nb = qnormalize(qmul(q4{qb.x, qb.y, qb.z, qb.w}, quat_exp(V(-0.5f * tp, 0, 0))));
-            F.mq[2 * ei] = make_float4(na.x, na.y, na.z, na.w), F.mq[2 * ei + 1] = make_float4(nb.x, nb.y, nb.z, nb.w);
+            if (lane == 0) F.mq[2 * ei] = make_float4(na.x, na.y, na.z, na.w), F.mq[2 * ei + 1] = make_float4(nb.x, nb.y, nb.z, nb.w);
             bt += tp, tp = 0;
         }
-        F.mps[4 * ei] = make_float4(up, tp, bt, dmga);
-        F.mps[4 * ei + 1] = make_float4(pax, pay, pbx, pby);
-        F.mps[4 * ei + 2] = make_float4(bax, bay, bbx, bby);
-        F.mps[4 * ei + 3] = make_float4(dmgb, 0.0f, 0.0f, 0.0f);
+        if (lane == 0) F.mps[4 * ei] = make_float4(up, tp, bt, dmga);
+        if (lane == 0) F.mps[4 * ei + 1] = make_float4(pax, pay, pbx, pby);
+        if (lane == 0) F.mps[4 * ei + 2] = make_float4(bax, bay, bbx, bby);
+        if (lane == 0) F.mps[4 * ei + 3] = make_float4(dmgb, 0.0f, 0.0f, 0.0f);
         // the tangent: elastic, the parts flowing this step plastic unless the step unloads them (frame_fem.cpp:
         // 2056-2069): held elastic 16 steps after an unload, and while the re-passes' budget is spent
         const float kFlow = 1e-4f;
@@ -721,25 +726,25 @@ __global__ void __launch_bounds__(128) k_member_eval(FemDev F, const float4* __r
         uint32_t hold = (fl >> 16) & 0xff, unload = 0;
         if (hold > 0) hold--, unload = yl;
         if (F.elastic[F.fbody[ab.x]]) unload = yl;
-        F.mflag[ei] = yl | (unload << 8) | (hold << 16);
-        F.mtg[6 * ei] = make_float4(e1.x, e1.y, e1.z, L);
-        F.mtg[6 * ei + 1] = make_float4(e2.x, e2.y, e2.z, ka);
-        F.mtg[6 * ei + 2] = make_float4(e3.x, e3.y, e3.z, kt);
-        F.mtg[6 * ei + 3] = make_float4(cy[0], cy[1], cy[2], cz[0]);
-        F.mtg[6 * ei + 4] = make_float4(cz[1], cz[2], N, T);
-        F.mtg[6 * ei + 5] = make_float4(Max, May, Mbx, Mby);
+        if (lane == 0) F.mflag[ei] = yl | (unload << 8) | (hold << 16);
+        if (lane == 0) F.mtg[6 * ei] = make_float4(e1.x, e1.y, e1.z, L);
+        if (lane == 0) F.mtg[6 * ei + 1] = make_float4(e2.x, e2.y, e2.z, ka);
+        if (lane == 0) F.mtg[6 * ei + 2] = make_float4(e3.x, e3.y, e3.z, kt);
+        if (lane == 0) F.mtg[6 * ei + 3] = make_float4(cy[0], cy[1], cy[2], cz[0]);
+        if (lane == 0) F.mtg[6 * ei + 4] = make_float4(cz[1], cz[2], N, T);
+        if (lane == 0) F.mtg[6 * ei + 5] = make_float4(Max, May, Mbx, Mby);
         y = yl & ~unload;
     }
-    F.mon[ei] = 1;
-    F.mtan[ei] = make_float4(e1.x, e1.y, e1.z, N > 0 ? N / L : 0.0f);
-    member_world_k(F, nd, ei, ab, e1, e2, e3, L, ka, kt, cy, cz, y);
+    if (lane == 0) F.mon[ei] = 1, F.mtan[ei] = make_float4(e1.x, e1.y, e1.z, N > 0 ? N / L : 0.0f);
+    member_world_k(F, nd, ei, ab, e1, e2, e3, L, ka, kt, cy, cz, y, Bs[threadIdx.x >> 5]);
 }
 
 // The unload check after pass `pass`'s solve (frame_fem.cpp:2959-2989): a flowing part of a member whose end rates
 // from the solution run against its moment (force, torque) gets its elastic tangent (held 16 steps), its world blocks
 // again; its component is marked for another pass. Pass 1's check runs only where pass 1 ran.
 __global__ void k_member_unload(FemDev F, const float4* __restrict__ nd, int pass) {
-    const int ei = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double Bs[4][72];
+    const int ei = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31; // (a warp a member)
     if (ei >= F.nmem || (pass > 0 && F.rp[pass - 1] == 0) || !F.mon[ei]) return;
     const uint32_t fl = F.mflag[ei];
     const uint32_t yl = fl & 0xf, unload = (fl >> 8) & 0xf, y = yl & ~unload;
@@ -771,12 +776,12 @@ __global__ void k_member_unload(FemDev F, const float4* __restrict__ nd, int pas
     if ((y & 8) && dot(e1, wb - wa) * t4.w < 0) u |= 8;
     if (!u) return;
     const uint32_t un = unload | u;
-    F.mflag[ei] = yl | (un << 8) | (16u << 16);
+    __syncwarp(); // (every lane has read the flags)
+    if (lane == 0) F.mflag[ei] = yl | (un << 8) | (16u << 16);
     const float4 t3 = F.mtg[6 * ei + 3];
     const float cy[3] = {t3.x, t3.y, t3.z}, cz[3] = {t3.w, t4.x, t4.y};
-    member_world_k(F, nd, ei, ab, e1, e2, e3, t0.w, t1.w, t2.w, cy, cz, yl & ~un);
-    atomicOr(&F.comp_again[F.col_comp[F.iperm[ab.x]]], 1 << pass);
-    F.rp[pass] = 1;
+    member_world_k(F, nd, ei, ab, e1, e2, e3, t0.w, t1.w, t2.w, cy, cz, yl & ~un, Bs[threadIdx.x >> 5]);
+    if (lane == 0) atomicOr(&F.comp_again[F.col_comp[F.iperm[ab.x]]], 1 << pass), F.rp[pass] = 1;
 }
 
 // the condition of the IF node of pass + 1's re-pass: set where pass `pass`'s check found an unload
@@ -802,114 +807,101 @@ __global__ void k_repass_account(FemDev F) {
     F.elastic[b] = cr < 1.0f ? 1 : 0;
 }
 
-// gather_part's member block (frame_fem.cpp:927-941): block blk (0 aa, 1 bb, 2 ba, 3 ab) times c, with the geometric
-// stiffness of its tension (sign gs)
-__device__ __forceinline__ void member_block_add(const FemDev& F, int ei, int blk, double h2, double gs, double* D) {
+// gather_part's member block (frame_fem.cpp:927-941), its row r: block blk (0 aa, 1 bb, 2 ba, 3 ab) times c, with the
+// geometric stiffness of its tension (sign gs)
+__device__ __forceinline__ void member_row_add(const FemDev& F, int ei, int blk, int r, double h2, double gs, double* D) {
     const int meta = F.mmeta[ei];
     const double c = h2 + (double)F.msec[meta & 0xffff].damping * F.h;
-    const double* B = F.mkw + 144 * (size_t)ei + 36 * blk;
-    for (int x = 0; x < 36; x++) D[x] += c * B[x];
+    const double2* B = reinterpret_cast<const double2*>(F.mkw + 144 * (size_t)ei + 36 * blk + 6 * r);
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+        const double2 v = B[x];
+        D[2 * x] += c * v.x, D[2 * x + 1] += c * v.y;
+    }
     const float4 t = F.mtan[ei];
     const double gg = h2 * t.w;
-    if (gg != 0) {
-        double P[9];
+    if (gg != 0 && r < 3) {
         const double ee[3] = {t.x, t.y, t.z};
-        for (int r = 0; r < 3; r++)
-            for (int q = 0; q < 3; q++) P[r * 3 + q] = gg * ((r == q ? 1.0 : 0.0) - ee[r] * ee[q]);
-        for (int r = 0; r < 3; r++)
-            for (int q = 0; q < 3; q++) D[r * 6 + q] += gs * P[r * 3 + q];
+        const double er = r == 0 ? ee[0] : r == 1 ? ee[1] : ee[2];
+#pragma unroll
+        for (int q = 0; q < 3; q++) D[q] += gs * (gg * ((r == q ? 1.0 : 0.0) - er * ee[q]));
     }
 }
 
 // ------------------------------------------------------------------------------------------ assembly
 // A triangle's block of corners (i, j) in the world's axes times c, with its tension's geometric stiffness
-// (gather_part's tri_block, frame_fem.cpp:961-1003)
-__device__ void tri_block_add(const FemDev& F, int t, int i, int j, double h2, double* D) {
-    const FemSecDev s = F.sec[F.tn[t].w];
+// (gather_part's tri_block, frame_fem.cpp:961-1003): its row r
+__device__ __forceinline__ void tri_row_add(const FemDev& F, int t, int i, int j, int r, double h2, double* D) {
+    const FemSecDev& s = F.sec[F.tn[t].w];
     const double c = h2 + (double)s.damping * F.h;
     const float* tg = F.ttan + 18 * (size_t)t;
     const double E[3][3] = {{tg[0], tg[3], tg[6]}, {tg[1], tg[4], tg[7]}, {tg[2], tg[5], tg[8]}};
     const float* Km = F.tk + 162 * (size_t)t;
     const float* Kp = Km + 81;
+    const int ra = r / 3, pp = r % 3;
+    const double E0 = tg[pp], E1 = tg[3 + pp], E2 = tg[6 + pp];
 #define BL_M(s2, t2) ((double)Km[(3 * i + (s2)) * 9 + 3 * j + (t2)])
 #define BL_P(s2, t2) ((double)Kp[(3 * i + (s2)) * 9 + 3 * j + (t2)])
-    for (int ra = 0; ra < 2; ra++)
-        for (int cb = 0; cb < 2; cb++) {
-            double T[3][3];
-            for (int pp = 0; pp < 3; pp++) {
-                const double E0 = E[pp][0], E1 = E[pp][1], E2 = E[pp][2];
-                if (ra == 0 && cb == 0) {
-                    T[pp][0] = E0 * BL_M(0, 0) + E1 * BL_M(1, 0);
-                    T[pp][1] = E0 * BL_M(0, 1) + E1 * BL_M(1, 1);
-                    T[pp][2] = E2 * BL_P(0, 0);
-                } else if (ra == 0) {
-                    T[pp][0] = E2 * BL_P(0, 1);
-                    T[pp][1] = E2 * BL_P(0, 2);
-                    T[pp][2] = E0 * BL_M(0, 2) + E1 * BL_M(1, 2);
-                } else if (cb == 0) {
-                    T[pp][0] = E2 * BL_M(2, 0);
-                    T[pp][1] = E2 * BL_M(2, 1);
-                    T[pp][2] = E0 * BL_P(1, 0) + E1 * BL_P(2, 0);
-                } else {
-                    T[pp][0] = E0 * BL_P(1, 1) + E1 * BL_P(2, 1);
-                    T[pp][1] = E0 * BL_P(1, 2) + E1 * BL_P(2, 2);
-                    T[pp][2] = E2 * BL_M(2, 2);
-                }
-            }
-            for (int pp = 0; pp < 3; pp++)
-                for (int qq = 0; qq < 3; qq++) D[(3 * ra + pp) * 6 + 3 * cb + qq] += c * (T[pp][0] * E[qq][0] + T[pp][1] * E[qq][1] + T[pp][2] * E[qq][2]);
-        }
+    double T[2][3];
+    if (ra == 0) {
+        T[0][0] = E0 * BL_M(0, 0) + E1 * BL_M(1, 0), T[0][1] = E0 * BL_M(0, 1) + E1 * BL_M(1, 1), T[0][2] = E2 * BL_P(0, 0);
+        T[1][0] = E2 * BL_P(0, 1), T[1][1] = E2 * BL_P(0, 2), T[1][2] = E0 * BL_M(0, 2) + E1 * BL_M(1, 2);
+    } else {
+        T[0][0] = E2 * BL_M(2, 0), T[0][1] = E2 * BL_M(2, 1), T[0][2] = E0 * BL_P(1, 0) + E1 * BL_P(2, 0);
+        T[1][0] = E0 * BL_P(1, 1) + E1 * BL_P(2, 1), T[1][1] = E0 * BL_P(1, 2) + E1 * BL_P(2, 2), T[1][2] = E2 * BL_M(2, 2);
+    }
 #undef BL_M
 #undef BL_P
+#pragma unroll
+    for (int cb = 0; cb < 2; cb++)
+#pragma unroll
+        for (int qq = 0; qq < 3; qq++) D[3 * cb + qq] += c * (T[cb][0] * E[qq][0] + T[cb][1] * E[qq][1] + T[cb][2] * E[qq][2]);
     const double gg = h2 * tg[9 + 3 * i + j];
-    if (gg != 0)
-        for (int pp = 0; pp < 3; pp++) D[pp * 7] += gg;
+    if (gg != 0 && r < 3) {
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+            if (q == r) D[q] += gg;
+    }
 }
 
-// One column's diagonal block and right side; nforce: the nodes' forces of the substep
-__device__ __forceinline__ void assemble_column(const FemDev& F, const float4* __restrict__ nd, const float4* __restrict__ nforce, int k) {
+// Row r of one column's diagonal block and of its right side; nforce: the nodes' forces of the substep
+__device__ __forceinline__ void assemble_column(const FemDev& F, const float4* __restrict__ nd, const float4* __restrict__ nforce, int k, int r) {
     const int i = F.perm[k];
     const int bn = F.fnode[i];
     const float4 P = nd[2 * bn], Vv = nd[2 * bn + 1];
     const double h2 = F.ch2[k], hd = F.chd[k];
-    double D[36];
-    double* R = F.rhs + 6 * (size_t)k;
-    for (int x = 0; x < 36; x++) D[x] = 0.0;
-    if (k == 0 || F.col_comp[k] != F.col_comp[k - 1]) F.comp_fail[F.col_comp[k]] = 0;
+    double D[6] = {0, 0, 0, 0, 0, 0}, R = 0.0;
+    if (r == 0 && (k == 0 || F.col_comp[k] != F.col_comp[k - 1])) F.comp_fail[F.col_comp[k]] = 0;
     const bool fixed = P.w <= 0;
-    F.fixed[k] = fixed;
+    if (r == 0) F.fixed[k] = fixed;
+    auto diagonal = [&](double v) {
+#pragma unroll
+        for (int q = 0; q < 6; q++)
+            if (q == r) D[q] = v;
+    };
     if (fixed) {
-        for (int j = 0; j < 6; j++) D[j * 7] = 1.0, R[j] = 0.0;
+        diagonal(1.0);
     } else {
-        D[0] = D[7] = D[14] = Vv.w;
-        D[21] = D[28] = D[35] = F.inertia[i];
-        double rd[6] = {0, 0, 0, 0, 0, 0};
+        diagonal(r < 3 ? (double)Vv.w : (double)F.inertia[i]);
+        double rd = 0;
         for (int qq = F.gdiag_ptr[k]; qq < F.gdiag_ptr[k + 1]; qq++) {
             const int2 g = F.gdiag[qq];
             if (g.x < 0) { // (a member's end: -(member + 1), end)
                 const int ei = -g.x - 1;
                 if (!F.mon[ei]) continue;
-                member_block_add(F, ei, g.y, h2, 1.0, D);
+                member_row_add(F, ei, g.y, r, h2, 1.0, D);
                 const double cr = hd + (double)F.msec[F.mmeta[ei] & 0xffff].damping * F.h;
-                if (cr != 0) {
-                    const double* kv = F.mkv + 12 * (size_t)ei + 6 * g.y;
-                    for (int j = 0; j < 6; j++) rd[j] -= cr * kv[j];
-                }
+                if (cr != 0) rd -= cr * F.mkv[12 * (size_t)ei + 6 * g.y + r];
                 continue;
             }
             if (!F.ton[g.x]) continue;
-            tri_block_add(F, g.x, g.y, g.y, h2, D);
+            tri_row_add(F, g.x, g.y, g.y, r, h2, D);
             const double cr = hd + (double)F.sec[F.tn[g.x].w].damping * F.h;
-            if (cr != 0) {
-                const double* kv = F.tkv + 18 * (size_t)g.x + 6 * g.y;
-                for (int j = 0; j < 6; j++) rd[j] -= cr * kv[j];
-            }
+            if (cr != 0) rd -= cr * F.tkv[18 * (size_t)g.x + 6 * g.y + r];
         }
         const float4 f = nforce[bn], m = F.torque[i];
-        const double h = F.h;
-        R[0] = h * (double)f.x, R[1] = h * (double)f.y, R[2] = h * (double)f.z;
-        R[3] = h * (double)m.x, R[4] = h * (double)m.y, R[5] = h * (double)m.z;
-        if (F.contact_n) {
+        R = F.h * (double)(r == 0 ? f.x : r == 1 ? f.y : r == 2 ? f.z : r == 3 ? m.x : r == 4 ? m.y : m.z);
+        if (F.contact_n && r < 3) {
             // a ground contact: kappa n n^T towards the normal velocity change it asked for, kappa = 200 m; sticking,
             // along the ground too towards stopping its sliding (gather_part, frame_fem.cpp:1043-1064)
             const float4 c4 = F.contact_n[i];
@@ -919,55 +911,66 @@ __device__ __forceinline__ void assemble_column(const FemDev& F, const float4* _
                 const bool stick = l2 > 2.0f;
                 if (stick) cn = cn * 0.5f;
                 const double kap = 200.0 * Vv.w, want = F.step * (double)dot(V(f.x, f.y, f.z), cn) / Vv.w;
-                const double nn[3] = {cn.x, cn.y, cn.z};
-                for (int p = 0; p < 3; p++) {
-                    for (int q2 = 0; q2 < 3; q2++) D[p * 6 + q2] += kap * nn[p] * nn[q2];
-                    R[p] += kap * want * nn[p];
-                }
+                const double nn[3] = {cn.x, cn.y, cn.z}, nr = r == 0 ? nn[0] : r == 1 ? nn[1] : nn[2];
+#pragma unroll
+                for (int q2 = 0; q2 < 3; q2++) D[q2] += kap * nr * nn[q2];
+                R += kap * want * nr;
                 if (stick) {
                     const v3 vel = V(Vv.x, Vv.y, Vv.z);
                     const v3 vt = vel - cn * dot(vel, cn);
-                    const double wt[3] = {-vt.x, -vt.y, -vt.z};
-                    for (int p = 0; p < 3; p++) {
-                        for (int q2 = 0; q2 < 3; q2++) D[p * 6 + q2] += kap * ((p == q2 ? 1.0 : 0.0) - nn[p] * nn[q2]);
-                        R[p] += kap * wt[p];
-                    }
+                    const double wt = r == 0 ? -vt.x : r == 1 ? -vt.y : -vt.z;
+#pragma unroll
+                    for (int q2 = 0; q2 < 3; q2++) D[q2] += kap * ((r == q2 ? 1.0 : 0.0) - nr * nn[q2]);
+                    R += kap * wt;
                 }
             }
         }
-        for (int j = 0; j < 6; j++) R[j] += rd[j];
+        R += rd;
     }
-    double* Dg = F.diag + 36 * (size_t)k;
-    for (int x = 0; x < 36; x++) Dg[x] = D[x];
+    F.rhs[6 * (size_t)k + r] = R;
+    double2* Dg = reinterpret_cast<double2*>(F.diag + 36 * (size_t)k + 6 * r);
+#pragma unroll
+    for (int x = 0; x < 3; x++) Dg[x] = make_double2(D[2 * x], D[2 * x + 1]);
 }
 
-// The off-diagonal blocks, a thread each (pb: the block; its column from blk_col): zero where a corner is fixed, else
-// the sum of its triangles' blocks in their order
-__device__ __forceinline__ void assemble_off(const FemDev& F, const float4* __restrict__ nd, int pb) {
+// Row r of an off-diagonal block (pb; its column from blk_col): zero where a corner is fixed, else the sum of its
+// members' and triangles' rows in their order
+__device__ __forceinline__ void assemble_off(const FemDev& F, const float4* __restrict__ nd, int pb, int r) {
     const int k = F.blk_col[pb];
     const double h2 = F.ch2[k];
-    double O[36];
-    for (int x = 0; x < 36; x++) O[x] = 0.0;
+    double O[6] = {0, 0, 0, 0, 0, 0};
     const bool fixed = nd[2 * F.fnode[F.perm[k]]].w <= 0;
     const int rnode = F.fnode[F.perm[F.row[pb]]];
     if (!fixed && F.goff_ptr[pb] != F.goff_ptr[pb + 1] && !(nd[2 * rnode].w <= 0))
         for (int qq = F.goff_ptr[pb]; qq < F.goff_ptr[pb + 1]; qq++) {
             const int4 g = F.goff[qq];
             if (g.x < 0) { // (a member's block: -(member + 1), 2 ba / 3 ab)
-                if (F.mon[-g.x - 1]) member_block_add(F, -g.x - 1, g.y, h2, -1.0, O);
+                if (F.mon[-g.x - 1]) member_row_add(F, -g.x - 1, g.y, r, h2, -1.0, O);
             } else if (F.ton[g.x]) {
-                tri_block_add(F, g.x, g.y, g.z, h2, O);
+                tri_row_add(F, g.x, g.y, g.z, r, h2, O);
             }
         }
-    double* Og = F.off + 36 * (size_t)pb;
-    for (int x = 0; x < 36; x++) Og[x] = O[x];
+    double2* Og = reinterpret_cast<double2*>(F.off + 36 * (size_t)pb + 6 * r);
+#pragma unroll
+    for (int x = 0; x < 3; x++) Og[x] = make_double2(O[2 * x], O[2 * x + 1]);
 }
 
-// The columns' diagonal blocks and right sides (threads [0, nf)) and the off-diagonal blocks (threads [nf, nf + nblk))
-__global__ void __launch_bounds__(128) k_fem_assemble_all(FemDev F, const float4* __restrict__ nd, const float4* __restrict__ nforce) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < F.nf) assemble_column(F, nd, nforce, t);
-    else if (t < F.nf + F.nblk) assemble_off(F, nd, t - F.nf);
+// The columns' diagonal blocks and right sides, then the off-diagonal blocks: a thread a row of a block (the sums of each
+// entry as before, six times as many in flight and each block's rows stored side by side). Multifrontal: only the blocks
+// with entries (asm_blk, nasm of them) - the fill's are zero from the commit on; else every block of the pattern, since the
+// block columns are factored in place. reset: the bodies' bounds accumulators for this substep (where no beams kernel
+// does it).
+// (B200: a thread a block and every fill block written took 430 us on the 50k-node shell body, 19 on the 21 x 21 plate.)
+__global__ void __launch_bounds__(128) k_fem_assemble_all(FemDev F, const float4* __restrict__ nd, const float4* __restrict__ nforce,
+                                                          const int* __restrict__ asm_blk, int nasm, Body* __restrict__ reset, int nbodies) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x, t = g / 6, r = g - 6 * t;
+    if (reset && g < nbodies) {
+        Body& B = reset[g];
+        B.acc_mn[0] = B.acc_mn[1] = B.acc_mn[2] = 1e30f;
+        B.acc_mx[0] = B.acc_mx[1] = B.acc_mx[2] = -1e30f;
+    }
+    if (t < F.nf) assemble_column(F, nd, nforce, t, r);
+    else if (t < F.nf + nasm) assemble_off(F, nd, asm_blk ? asm_blk[t - F.nf] : t - F.nf, r);
 }
 
 // ------------------------------------------------------------------------------------------ factorization
@@ -1373,22 +1376,20 @@ __global__ void __launch_bounds__(1024) k_front_solve(FemDev F, FrontDev X) {
 }
 
 // ------------------------------------------------------------------------------------------ after the solve
-__global__ void k_fem_velocity(FemDev F, const float4* __restrict__ nd, float4* __restrict__ nforce) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= F.nf) return;
-    const int i = F.perm[k];
+// A frame node's new velocity from the solution, as a force m dv / step on its body's node (frame_fem.cpp:2998-3025): the
+// spin advanced (w), safety clamps; f: the node's force, in and out
+__device__ __forceinline__ void fem_velocity(const FemDev& F, int i, float mass, v3& f, float4& w4) {
+    const int k = F.iperm[i];
     F.torque[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f); // (used by this step: torques from outside add up until the next)
     if (F.comp_fail[F.col_comp[k]]) {
         if (k == 0 || F.col_comp[k] != F.col_comp[k - 1]) atomicAdd(&F.body_failures[F.fbody[i]], 1);
         return; // (a failed factorization: the elements' forces stay in the node forces, an explicit step this once)
     }
     if (F.fixed[k]) {
-        F.w[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        w4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         return;
     }
     const double* x = F.rhs + 6 * (size_t)k;
-    const int bn = F.fnode[i];
-    const float mass = nd[2 * bn + 1].w;
     v3 dv = V((float)x[0], (float)x[1], (float)x[2]);
     const v3 dw = V((float)x[3], (float)x[4], (float)x[5]);
     if (!isfinite(dv.x + dv.y + dv.z + dw.x + dw.y + dw.z)) {
@@ -1400,69 +1401,90 @@ __global__ void k_fem_velocity(FemDev F, const float4* __restrict__ nd, float4* 
         const float l = length(dv);
         if (l > kMaxDv) dv = dv * (kMaxDv / l), atomicAdd(&F.body_clamps[F.fbody[i]], 1);
     }
-    const v3 fv = dv * (mass / F.step);
-    nforce[bn] = make_float4(fv.x, fv.y, fv.z, 0.0f);
-    const float4 w0 = F.w[i];
-    v3 wn = V(w0.x, w0.y, w0.z) + dw;
+    f = dv * (mass / F.step);
+    v3 wn = V(w4.x, w4.y, w4.z) + dw;
     {
         const float l = length(wn);
         if (l > kMaxW) wn = wn * (kMaxW / l), atomicAdd(&F.body_clamps[F.fbody[i]], 1);
     }
-    F.w[i] = make_float4(wn.x, wn.y, wn.z, 0.0f);
+    w4 = make_float4(wn.x, wn.y, wn.z, 0.0f);
 }
 
-// The frame bodies' nodes: SoftBody::integrate_nodes with the forces the solve left (softbody.cpp:769-795), the body's
-// bounds and top speed; then a frame node's FemFrame::sync_positions (frame_fem.cpp:3407-3422): its double position
-// advanced by h v, its orientation turned by w h, its float position taken from the double one unless something moved
-// it. fem_nodes: the frame bodies' nodes (global node indices), fslot: a node's frame node (-1: none).
-__global__ void __launch_bounds__(256) k_fem_integrate(FemDev F, float4* __restrict__ nd, const float4* __restrict__ nforce,
+// the bounds, top speed and static contacts of a warp's nodes into their bodies' accumulators (bl_kernels.cuh)
+__device__ __forceinline__ void accumulate_bounds(Body* __restrict__ bodies, int body, bool live, v3 p, v3 pmx, float v2, int contact);
+
+// The frame bodies' nodes: a frame node's velocity from the solution (fem_velocity), SoftBody::integrate_nodes
+// (softbody.cpp:769-795), the body's bounds and top speed; then a frame node's FemFrame::sync_positions
+// (frame_fem.cpp:3407-3422): its double position advanced by h v, its orientation turned by w h, its float position taken
+// from the double one unless something moved it. fem_nodes: the frame bodies' nodes (global node indices), fslot: a
+// node's frame node (-1: none).
+// (B200, the 50k-node shell body: 236 us with seven atomics a node and 7 us for the velocities; 11 us with a warp's
+// bounds reduced first and both in one launch.)
+__global__ void __launch_bounds__(256) k_fem_integrate(FemDev F, float4* __restrict__ nd, float4* __restrict__ nforce,
                                                        const int* __restrict__ fem_nodes, int n_fem_nodes, const int* __restrict__ fslot,
                                                        const int4* __restrict__ info, Body* __restrict__ bodies, float dt) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_fem_nodes) return;
-    const int i = fem_nodes[t];
-    Body& B = bodies[info[i].w];
-    if (B.sleeping) return;
-    float4 P = nd[2 * i], Vv = nd[2 * i + 1];
-    v3 pos = V(P.x, P.y, P.z), vel = V(Vv.x, Vv.y, Vv.z);
+    int body = -1;
+    bool live = false;
+    v3 lo = V(1e30f, 1e30f, 1e30f), hi = V(-1e30f, -1e30f, -1e30f);
     float v2 = 0.0f;
-    if (P.w > 0) {
-        const float4 f4 = nforce[i];
-        vel = vel + V(f4.x, f4.y, f4.z) * (P.w * dt);
-        v2 = dot(vel, vel);
-        if (v2 > kMaxNodeSpeed * kMaxNodeSpeed) {
-            vel = vel * (kMaxNodeSpeed / sqrtf(v2));
-            v2 = kMaxNodeSpeed * kMaxNodeSpeed;
-        } else if (!(v2 >= 0.0f)) {
-            vel = V(0, 0, 0);
-            v2 = 0;
+    if (t < n_fem_nodes) {
+        const int i = fem_nodes[t], fs = fslot[i];
+        const float4 P = nd[2 * i], Vv = nd[2 * i + 1];
+        body = info[i].w;
+        const bool awake = !bodies[body].sleeping;
+        v3 f = V(0, 0, 0);
+        float4 w4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        {
+            const float4 f4 = nforce[i];
+            f = V(f4.x, f4.y, f4.z);
         }
-        pos = pos + vel * dt;
-    }
-    const int fs = fslot[i];
-    if (fs >= 0) {
-        double* x = F.xd + 3 * (size_t)fs;
-        const double h = F.h;
-        x[0] += h * vel.x, x[1] += h * vel.y, x[2] += h * vel.z;
-        const float4 w4 = F.w[fs];
-        const v3 w = V(w4.x, w4.y, w4.z);
-        if (dot(w, w) > 0) {
-            const float4 q0 = F.q[fs];
-            const q4 qn = qnormalize(qmul(quat_exp(w * F.h), q4{q0.x, q0.y, q0.z, q0.w}));
-            F.q[fs] = make_float4(qn.x, qn.y, qn.z, qn.w);
+        if (fs >= 0) {
+            w4 = F.w[fs];
+            fem_velocity(F, fs, Vv.w, f, w4);
+            F.w[fs] = w4;
+            nforce[i] = make_float4(f.x, f.y, f.z, 0.0f);
         }
-        const double tol = 1e-4 * (1.0 + fabs((double)pos.x) + fabs((double)pos.y) + fabs((double)pos.z));
-        if (P.w > 0 && fabs(x[0] - pos.x) <= tol && fabs(x[1] - pos.y) <= tol && fabs(x[2] - pos.z) <= tol)
-            pos = V((float)x[0], (float)x[1], (float)x[2]);
-        else
-            x[0] = pos.x, x[1] = pos.y, x[2] = pos.z;
+        if (awake) {
+            live = true;
+            v3 pos = V(P.x, P.y, P.z), vel = V(Vv.x, Vv.y, Vv.z);
+            if (P.w > 0) {
+                vel = vel + f * (P.w * dt);
+                v2 = dot(vel, vel);
+                if (v2 > kMaxNodeSpeed * kMaxNodeSpeed) {
+                    vel = vel * (kMaxNodeSpeed / sqrtf(v2));
+                    v2 = kMaxNodeSpeed * kMaxNodeSpeed;
+                } else if (!(v2 >= 0.0f)) {
+                    vel = V(0, 0, 0);
+                    v2 = 0;
+                }
+                pos = pos + vel * dt;
+            }
+            if (fs >= 0) {
+                double* x = F.xd + 3 * (size_t)fs;
+                const double h = F.h;
+                double x0 = x[0] + h * vel.x, x1 = x[1] + h * vel.y, x2 = x[2] + h * vel.z;
+                const v3 w = V(w4.x, w4.y, w4.z);
+                if (dot(w, w) > 0) {
+                    const float4 q0 = F.q[fs];
+                    const q4 qn = qnormalize(qmul(quat_exp(w * F.h), q4{q0.x, q0.y, q0.z, q0.w}));
+                    F.q[fs] = make_float4(qn.x, qn.y, qn.z, qn.w);
+                }
+                const double tol = 1e-4 * (1.0 + fabs((double)pos.x) + fabs((double)pos.y) + fabs((double)pos.z));
+                if (P.w > 0 && fabs(x0 - pos.x) <= tol && fabs(x1 - pos.y) <= tol && fabs(x2 - pos.z) <= tol)
+                    pos = V((float)x0, (float)x1, (float)x2);
+                else
+                    x0 = pos.x, x1 = pos.y, x2 = pos.z;
+                x[0] = x0, x[1] = x1, x[2] = x2;
+            }
+            nd[2 * i] = make_float4(pos.x, pos.y, pos.z, P.w);
+            nd[2 * i + 1] = make_float4(vel.x, vel.y, vel.z, Vv.w);
+            // (the bounds skip a non-finite coordinate)
+            lo = V(pos.x == pos.x ? pos.x : 1e30f, pos.y == pos.y ? pos.y : 1e30f, pos.z == pos.z ? pos.z : 1e30f);
+            hi = V(pos.x == pos.x ? pos.x : -1e30f, pos.y == pos.y ? pos.y : -1e30f, pos.z == pos.z ? pos.z : -1e30f);
+        }
     }
-    nd[2 * i] = make_float4(pos.x, pos.y, pos.z, P.w);
-    nd[2 * i + 1] = make_float4(vel.x, vel.y, vel.z, Vv.w);
-    if (pos.x == pos.x) atomic_min_f(&B.acc_mn[0], pos.x), atomic_max_f(&B.acc_mx[0], pos.x);
-    if (pos.y == pos.y) atomic_min_f(&B.acc_mn[1], pos.y), atomic_max_f(&B.acc_mx[1], pos.y);
-    if (pos.z == pos.z) atomic_min_f(&B.acc_mn[2], pos.z), atomic_max_f(&B.acc_mx[2], pos.z);
-    atomic_max_f(&B.acc_v2, v2);
+    accumulate_bounds(bodies, body, live, lo, hi, v2, 0);
 }
 
 } // namespace blg

@@ -786,21 +786,32 @@ __device__ __forceinline__ void fem_gather(const NodeFem& nf, int i, v3 f) {
     if (fs >= 0) {
         const int k = nf.iperm[fs];
         v3 tq = V(0, 0, 0);
-        for (int g = nf.gdiag_ptr[k]; g < nf.gdiag_ptr[k + 1]; g++) {
-            const int2 e = nf.gdiag[g];
-            if (e.x < 0) { // (a member's end a (+fa, ta) or b (-fa, tb): gather_forces, frame_fem.cpp:2092-2096)
-                const int ei = -e.x - 1;
-                if (!nf.mon[ei]) continue;
-                const float4 fa = nf.mfa[ei], tq4 = e.y == 0 ? nf.mta[ei] : nf.mtb[ei];
-                if (e.y == 0) f = V(f.x + fa.x, f.y + fa.y, f.z + fa.z);
-                else f = V(f.x - fa.x, f.y - fa.y, f.z - fa.z);
-                tq = V(tq.x + tq4.x, tq.y + tq4.y, tq.z + tq4.z);
-                continue;
+        // (four entries' loads issued together, then added in order)
+        const int g1 = nf.gdiag_ptr[k + 1];
+        for (int g = nf.gdiag_ptr[k]; g < g1; g += 4) {
+            int2 e[4];
+            bool on[4];
+            float4 ff[4], tt[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) e[u] = g + u < g1 ? nf.gdiag[g + u] : make_int2(0, -1);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                on[u] = false;
+                if (e[u].y < 0) continue;
+                if (e[u].x < 0) { // (a member's end a (+fa, ta) or b (-fa, tb): gather_forces, frame_fem.cpp:2092-2096)
+                    const int ei = -e[u].x - 1;
+                    on[u] = nf.mon[ei], ff[u] = nf.mfa[ei], tt[u] = e[u].y == 0 ? nf.mta[ei] : nf.mtb[ei];
+                } else {
+                    on[u] = nf.ton[e[u].x], ff[u] = nf.tf[3 * e[u].x + e[u].y], tt[u] = nf.tt[3 * e[u].x + e[u].y];
+                }
             }
-            if (!nf.ton[e.x]) continue;
-            const float4 tf = nf.tf[3 * e.x + e.y], tt = nf.tt[3 * e.x + e.y];
-            f = V(f.x + tf.x, f.y + tf.y, f.z + tf.z);
-            tq = V(tq.x + tt.x, tq.y + tt.y, tq.z + tt.z);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (!on[u]) continue;
+                if (e[u].x < 0 && e[u].y != 0) f = V(f.x - ff[u].x, f.y - ff[u].y, f.z - ff[u].z);
+                else f = V(f.x + ff[u].x, f.y + ff[u].y, f.z + ff[u].z);
+                tq = V(tq.x + tt[u].x, tq.y + tt[u].y, tq.z + tt[u].z);
+            }
         }
         nf.torque[fs] = make_float4(tq.x, tq.y, tq.z, 0.0f);
     }

@@ -184,6 +184,9 @@ struct bl_gpu_ctx {
     DevBuf<int2> gdiag, gu, rb;
     DevBuf<int4> goff, tn;
     DevBuf<double> xd, diag, ldiag, off, rhs, dinv, tkv, ch2, chd;
+    DevBuf<int> asm_blk;                       // the multifrontal path's blocks with entries (k_fem_assemble_all)
+    int n_asm = 0;                             // blocks assembled a substep
+    bool fem_only = false;                     // every body has a frame and none has beams: no beams or nodes kernels
     // the FEM members (k_member_eval)
     int NM = 0;
     DevBuf<int2> mn;
@@ -292,7 +295,7 @@ static void free_fem(bl_gpu_ctx* c) {
     c->mps.free_(), c->mtg.free_(), c->mflag.free_(), c->credit.free_(), c->elastic.free_(), c->comp_again.free_(), c->comp_size.free_();
     c->body_comp.free_(), c->rp.free_(), c->repc.free_();
     c->contact_n.free_(), c->fem_ground = false;
-    c->xd.free_(), c->diag.free_(), c->ldiag.free_(), c->off.free_(), c->rhs.free_(), c->dinv.free_(), c->tkv.free_(), c->ch2.free_(), c->chd.free_();
+    c->xd.free_(), c->diag.free_(), c->ldiag.free_(), c->off.free_(), c->rhs.free_(), c->dinv.free_(), c->asm_blk.free_(), c->fem_only = false, c->tkv.free_(), c->ch2.free_(), c->chd.free_();
     c->finertia.free_(), c->tX.free_(), c->tk.free_(), c->tb.free_(), c->tX0.free_(), c->th0.free_(), c->tdmg.free_(), c->ttan.free_(), c->tbroken.free_(), c->ton.free_(), c->ffixed.free_(), c->fsec.free_();
 }
 
@@ -785,6 +788,16 @@ static int commit_fem(bl_gpu_ctx* c) {
     BL_CUDA(c, c->dinv.alloc(6 * (size_t)NF));
     BL_CUDA(c, c->ffixed.alloc(NF));
     BL_CUDA(c, cudaMemsetAsync(c->ton.p, 0, NT, c->stream));
+    c->n_asm = NB;
+    if (c->fem_mode == 2) { // (the fill's blocks stay zero: the factor is in the fronts)
+        std::vector<int> blk;
+        for (int pb = 0; pb < NB; pb++)
+            if (goff_ptr[pb] != goff_ptr[pb + 1]) blk.push_back(pb);
+        c->n_asm = (int)blk.size();
+        if ((rc = upload_vec(c, c->asm_blk, blk))) return rc;
+        BL_CUDA(c, cudaMemsetAsync(c->off.p, 0, sizeof(double) * 36 * (size_t)std::max(NB, 1), c->stream));
+    }
+    c->fem_only = nfem_nodes == c->N && c->M == 0;
     FemDev& F = c->fd;
     F.nf = NF, F.ntri = NT, F.nblk = NB;
     F.fnode = c->fnode.p, F.fbody = c->fbody.p, F.perm = c->fperm.p, F.iperm = c->fiperm.p, F.xd = c->xd.p, F.q = c->fq.p, F.w = c->fw.p;
@@ -872,7 +885,7 @@ static int commit_fem(bl_gpu_ctx* c) {
         c->chol_launches = 3 * (int64_t)c->front_level;
         if (c->front_level < nlev) c->chol_launches += 1 + c->front.nt + 2 * (c->front.nt - 1) + 2;
         if (c->fem_mode == 2 && (rc = commit_multifrontal(c, col_ptr, row, col_comp, goff_ptr, NC))) return rc;
-        c->fem_launches = 4 + (c->NT > 0 ? 1 : 0) + (c->NM > 0 ? 1 : 0) + c->chol_launches; // (begin, triangles, members, assembly, velocity, integration)
+        c->fem_launches = 2 + (c->NT > 0 ? 1 : 0) + (c->NM > 0 ? 1 : 0) + c->chol_launches; // (triangles, members, assembly, integration)
     }
     // PCG: vectors, block-Jacobi factors, the grid's partial sums (one cooperative launch: as many blocks as fit)
     for (DevBuf<double>* d : {&c->px, &c->pr, &c->pz, &c->pp, &c->ppdi}) BL_CUDA(c, d->alloc(6 * (size_t)NF));
@@ -1332,6 +1345,7 @@ static bool rebuild_at(const bl_gpu_ctx* c, int k) { return k % c->interval == 0
 static int64_t frame_launches(const bl_gpu_ctx* c, int n) {
     int64_t per = 3 + (c->any_drag ? 1 : 0) + (c->NW > 0 ? 1 : 0) + (c->NWR > 0 && c->beam_grid == 0 ? 1 : 0) + (c->NSH > 0 ? 1 : 0);
     if (c->NF > 0) {
+        if (c->fem_only) per -= 2; // (no beams, no other nodes)
         per += c->fem_launches + (c->cfg.fem_check_residual ? 2 : 0) + (c->fem_ground ? 1 : 0);
         // (the unload re-pass: its checks, conditions and account; its passes' kernels, which run only where a check
         // finds an unload, are not counted - launched without a graph they always run)
@@ -1340,7 +1354,7 @@ static int64_t frame_launches(const bl_gpu_ctx* c, int n) {
         const bool learned = c->cfg.fem_solver == BL_GPU_FEM_PCG_LEARNED, rec = c->rec_on;
         per += (learned || rec ? 2 : 0) + (learned ? 1 : 0) + (rec ? 3 : 0);
     }
-    int64_t total = per * n + 3;
+    int64_t total = per * n + 3 + (c->NF > 0 ? 1 : 0); // (k_fem_begin a frame)
     if (c->contacts_on) {
         total += 1 + 3 * (int64_t)n; // k_islands; k_wake, k_detect, k_collide a substep
         for (int k = 0; k < n; k++) total += rebuild_at(c, k) ? 4 : 0; // (k_rebuild, k_pair_count, k_pair_place, k_pair_write)
@@ -1441,6 +1455,11 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
     NodeFem nfm{c->fslot.p, c->fiperm.p, c->gdiag_ptr.p, c->gdiag.p, c->ton.p, c->tf.p, c->tt.p, c->ftorque.p, c->nforce.p, c->ext.p,
                 c->mon.p, c->mfa.p, c->mta.p, c->mtb.p};
     const FemDev& F = c->fd;
+    auto assemble = [c, &F](cudaStream_t as) {
+        const int64_t rows = std::max<int64_t>(6 * ((int64_t)c->NF + c->n_asm), c->B);
+        k_fem_assemble_all<<<(unsigned)((rows + 127) / 128), 128, 0, as>>>(F, c->nd.p, c->nforce.p, c->fem_mode == 2 ? c->asm_blk.p : nullptr, c->n_asm,
+                                                                          c->fem_only ? c->dbodies.p : nullptr, c->B);
+    };
     for (int k = 0; k < n; k++) {
         if (c->contacts_on) {
             // wake requests, then the pair search on its substeps (on the positions and velocities the substep starts from)
@@ -1456,8 +1475,11 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
         }
         mark();
         if (c->any_drag) k_drag_parts<<<(c->B + 63) / 64, 64, 0, s>>>(c->dbodies.p, c->B, c->nd.p, c->ab.p, c->bmeta.p, dg);
-        if (c->NF > 0) k_fem_begin<<<(c->NF + tb - 1) / tb, tb, 0, s>>>(F, c->nd.p);
-        if (c->beam_grid > 0) {
+        if (c->NF > 0 && k == 0) // (nothing moves a frame node but its frame within a frame)
+            k_fem_begin<<<(c->NF + tb - 1) / tb, tb, 0, s>>>(F, c->nd.p);
+        if (c->fem_only) {
+            // (no beams; the bounds accumulators are reset by the assembly)
+        } else if (c->beam_grid > 0) {
             // (the wheels' step in the same launch, after each block's tiles)
             if (c->ends16)
                 k_beams_tma<true><<<c->beam_grid, kBeamThreads, beam_smem<true>(), s>>>(c->ab16.p, c->tbase.p, c->kd.p, c->bst.p, c->bmeta.p, c->bcold.p,
@@ -1476,8 +1498,8 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
             k_shocks<<<(c->NSH + 127) / 128, 128, 0, s>>>(sk, c->NSH, c->ab.p, c->bst.p, c->bmeta.p, c->stress.p, c->bbody.p, c->nd.p, c->dbodies.p);
         if (c->NT > 0 && c->any_plastic) k_tri_eval<true><<<(c->NT + 127) / 128, 128, 0, s>>>(F, c->nd.p);
         else if (c->NT > 0) k_tri_eval<false><<<(c->NT + 127) / 128, 128, 0, s>>>(F, c->nd.p);
-        if (c->NM > 0 && c->any_plastic_members) k_member_eval<true><<<(c->NM + 127) / 128, 128, 0, s>>>(F, c->nd.p);
-        else if (c->NM > 0) k_member_eval<false><<<(c->NM + 127) / 128, 128, 0, s>>>(F, c->nd.p);
+        if (c->NM > 0 && c->any_plastic_members) k_member_eval<true><<<(c->NM + 3) / 4, 128, 0, s>>>(F, c->nd.p);
+        else if (c->NM > 0) k_member_eval<false><<<(c->NM + 3) / 4, 128, 0, s>>>(F, c->nd.p);
         mark();
         if (c->packed_inc)
             k_force<true><<<std::max(gfn, 1), fb, 0, s>>>(c->nd.p, c->info.p, c->ell_ptr.p, c->inc4.p, c->ell_base.p, c->fsc.p, c->dbodies.p,
@@ -1492,7 +1514,7 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
             k_collide<<<c->B, kCollideThreads, kCollideSmem, s>>>(c->nd.p, c->info.p, c->dbodies.p, c->B, CT, c->nodef.p);
         }
         mark();
-        k_integrate<<<std::max(gin, 1), ib, 0, s>>>(c->nd.p, c->info.p, c->dbodies.p, c->st, dt, c->N, k == 0 ? 1 : 0, c->nodef.p, wh);
+        if (!c->fem_only) k_integrate<<<std::max(gin, 1), ib, 0, s>>>(c->nd.p, c->info.p, c->dbodies.p, c->st, dt, c->N, k == 0 ? 1 : 0, c->nodef.p, wh);
         if (c->NW > 0) k_tyres<<<(c->NW + 7) / 8, 256, 0, s>>>(c->nd.p, c->info.p, c->dbodies.p, dt, c->NW, k == 0 ? 1 : 0, c->nodef.p, wh);
         mark();
         if (c->NF > 0) {
@@ -1502,7 +1524,7 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
                 k_fem_static<<<(c->n_fem_nodes + 127) / 128, 128, 0, s>>>(c->nd.p, c->nforce.p, c->fem_nodes.p, c->n_fem_nodes, c->fslot.p, c->info.p,
                                                                         c->dbodies.p, c->st, dt, c->contact_n.p);
             }
-            k_fem_assemble_all<<<(c->NF + c->NB + 127) / 128, 128, 0, s>>>(F, c->nd.p, c->nforce.p);
+            assemble(s);
             if (c->cfg.fem_check_residual) {
                 cudaMemcpyAsync(c->a0d.p, c->diag.p, sizeof(double) * 36 * c->NF, cudaMemcpyDeviceToDevice, s);
                 cudaMemcpyAsync(c->a0o.p, c->off.p, sizeof(double) * 36 * std::max(c->NB, 1), cudaMemcpyDeviceToDevice, s);
@@ -1572,8 +1594,8 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
                 // the unload re-pass (frame_fem.cpp:2959-2995): where the step unloads a flowing hinge (bar, twist), its
                 // elastic tangent and the step again - assembled and factored again, at most twice; each pass under an
                 // IF node its check sets (launched without a graph, the passes run and solve the same system again)
-                auto repass = [c, &F, cholesky](cudaStream_t cs) {
-                    k_fem_assemble_all<<<(c->NF + c->NB + 127) / 128, 128, 0, cs>>>(F, c->nd.p, c->nforce.p);
+                auto repass = [c, cholesky, assemble](cudaStream_t cs) {
+                    assemble(cs);
                     if (c->cfg.fem_check_residual) {
                         cudaMemcpyAsync(c->a0d.p, c->diag.p, sizeof(double) * 36 * c->NF, cudaMemcpyDeviceToDevice, cs);
                         cudaMemcpyAsync(c->a0o.p, c->off.p, sizeof(double) * 36 * std::max(c->NB, 1), cudaMemcpyDeviceToDevice, cs);
@@ -1582,7 +1604,7 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
                     cholesky(cs);
                 };
                 for (int pass = 0; pass < 2; pass++) {
-                    k_member_unload<<<(c->NM + 127) / 128, 128, 0, s>>>(F, c->nd.p, pass);
+                    k_member_unload<<<(c->NM + 3) / 4, 128, 0, s>>>(F, c->nd.p, pass);
                     cudaGraphConditionalHandle h{};
                     const bool have = make_condition(c, s, &h);
                     if (have) k_repass_cond<<<1, 1, 0, s>>>(c->rp.p, pass, h);
@@ -1599,7 +1621,6 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
                 k_mlp_record_done<<<1, 1, 0, s>>>(MD, c->NF);
             }
             if (learned || rec) k_mlp_store_dv<<<(c->NF + 127) / 128, 128, 0, s>>>(F, MD);
-            k_fem_velocity<<<(c->NF + 127) / 128, 128, 0, s>>>(F, c->nd.p, c->nforce.p);
             k_fem_integrate<<<(c->n_fem_nodes + 255) / 256, 256, 0, s>>>(F, c->nd.p, c->nforce.p, c->fem_nodes.p, c->n_fem_nodes, c->fslot.p, c->info.p,
                                                                        c->dbodies.p, dt);
         }
