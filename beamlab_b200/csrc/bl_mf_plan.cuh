@@ -202,7 +202,11 @@ static MfPlan mf_finish(int NF, const std::vector<int>& col_ptr, const std::vect
 // ------------------------------------------------------------------------------------------ the device's tiles and tasks
 constexpr int kMfT = 48;               // tile side (8 frame nodes)
 constexpr int kMfTile = kMfT * kMfT;   // doubles a tile
-constexpr int kMfFuseRows = 2;         // a front of one pivot tile and up to this many row tiles is one task
+// In a level of many tasks (over kMfWide: several rounds of all resident CTAs) a front of one pivot tile and up to
+// kMfFuseRows row tiles is one task: no flags, its tiles still in the cache. In a narrower level its tiles are tasks of
+// their own, side by side. (B200: the 21 x 21 plate 231 us whole-front tasks off, 254 on; the 50k-node shell body 6.84
+// and 6.49 ms.)
+constexpr int kMfFuseRows = 3, kMfWide = 3000;
 
 struct MfFrontDev {
     int p, npiv, nrow;   // pivot degrees of freedom, pivot and row nodes
@@ -224,15 +228,16 @@ MF_HD int mf_tix(int nt, int i, int j) { return j * nt - j * (j - 1) / 2 + (i - 
 
 struct MfLayout {
     std::vector<MfFrontDev> fr;
-    std::vector<int> cpos, cptr, eptr;  // (MfDev's arrays)
+    std::vector<int> cpos, cptr, eptr, pan; // (MfDev's arrays)
     std::vector<int2> ent;
     std::vector<int4> task;
     int64_t tiles = -1;                 // over all fronts (-1: more than fit their indexes)
     int pans = 0;                       // pivot tiles on the diagonals
-    int widest = 1;                     // the most factorization tasks of one level
+    int nfactor = 0;                    // the factorization's tasks; the backward solves' come after
+    int widest = 1, widest_back = 1;    // the most of either in one level
 };
 
-// The plan's tiles, maps and task list for k_mf_solve; goff_ptr: the off-diagonal blocks' assembly entries (a block
+// The plan's tiles, maps and task list for k_mf_factor and k_mf_back; goff_ptr: the off-diagonal blocks' assembly entries (a block
 // without any is fill, zero before the factorization)
 static MfLayout mf_layout(const MfPlan& P, const std::vector<int>& col_ptr, const std::vector<int>& row, const std::vector<int>& goff_ptr) {
     MfLayout Y;
@@ -241,7 +246,13 @@ static MfLayout mf_layout(const MfPlan& P, const std::vector<int>& col_ptr, cons
     fr.resize(nfr);
     int64_t tiles = 0;
     int pans = 0;
-    auto alone = [&](int f) { return fr[f].P == 1 && fr[f].nt - fr[f].P <= kMfFuseRows; };
+    std::vector<int> level(nfr), tasks(nlev, 0);
+    auto alone = [&](int f) { return tasks[level[f]] > kMfWide && fr[f].P == 1 && fr[f].nt - fr[f].P <= kMfFuseRows; };
+    for (int L = 0; L < nlev; L++)
+        for (int f = P.level_ptr[L]; f < P.level_ptr[L + 1]; f++) {
+            const int nt = (P.npiv[f] + 7) / 8 + P.nrow[f] / 8 + 1;
+            level[f] = L, tasks[L] += nt * (nt + 1) / 2;
+        }
     for (int f = 0; f < nfr; f++) {
         MfFrontDev& d = fr[f];
         d.npiv = P.npiv[f], d.nrow = P.nrow[f], d.p = 6 * d.npiv;
@@ -256,6 +267,9 @@ static MfLayout mf_layout(const MfPlan& P, const std::vector<int>& col_ptr, cons
     }
     if (tiles > (int64_t)1 << 30) return Y; // (its tiles' indexes; such a pool is far past the GPU's memory)
     Y.tiles = tiles, Y.pans = pans;
+    Y.pan.assign(col_ptr.size() - 1, 0);
+    for (int f = 0; f < nfr; f++)
+        for (int l = 0; l < fr[f].npiv; l++) Y.pan[P.idx[fr[f].idx0 + l]] = fr[f].pan0 + l / 8;
     // each row node's place in its parent's tiles, and per parent tile a front's first row node
     std::vector<int>&cpos = Y.cpos, &cptr = Y.cptr;
     for (int f = 0; f < nfr; f++) {
@@ -316,12 +330,15 @@ static MfLayout mf_layout(const MfPlan& P, const std::vector<int>& col_ptr, cons
             }
         Y.widest = std::max(Y.widest, (int)(task.size() - t0));
     }
+    Y.nfactor = (int)task.size();
     for (int L = nlev - 1; L >= 0; L--) {
         int cols = 0;
+        const size_t t0 = task.size();
         for (int f = P.level_ptr[L]; f < P.level_ptr[L + 1]; f++) cols = std::max(cols, fr[f].P);
         for (int b = 0; b < cols; b++)
             for (int f = P.level_ptr[L]; f < P.level_ptr[L + 1]; f++)
                 if (b < fr[f].P) task.push_back(make_int4(f, 0, fr[f].P - 1 - b, MF_BACK));
+        Y.widest_back = std::max(Y.widest_back, (int)(task.size() - t0));
     }
     return Y;
 }

@@ -1,4 +1,4 @@
-// The multifrontal factorization and solves of the frames' implicit step in one launch (the plan: bl_mf_plan.cuh).
+// The multifrontal factorization and solves of the frames' implicit step in two launches (the plan: bl_mf_plan.cuh).
 //
 // Each front is a lower triangle of 48 x 48 tiles (8 frame nodes a side): its pivots in P tiles, then its rows, the right
 // side b one more row after them (so that eliminating the pivots leaves, in b's row, the forward substitution's y on the
@@ -6,7 +6,7 @@
 // instruction (mma.m8n8k4) takes either operand of L L^T: three chunks of 16 columns, each of 8 x 4 blocks whose 32
 // entries are a warp's lanes - operand loads from shared memory are conflict-free and a chunk is one contiguous copy.
 //
-// k_mf_solve runs persistent CTAs over one list of tasks in an order in which every task's inputs come from tasks before
+// k_mf_factor and k_mf_back run persistent CTAs over a list of tasks in an order in which every task's inputs come from tasks before
 // it: a CTA takes the next task, waits on the flags of what it reads, and sets its own. The earliest unfinished task is
 // always held by a running CTA with all its inputs done, so the waits end; each is bounded in time all the same
 // (kMfWaitNs, then DEVERR_TIMEOUT, every component marked failed, the CTAs leave).
@@ -21,12 +21,13 @@
 // A pivot that is not positive marks the front's component failed (the reference's chol6 failing, frame_fem.cpp:
 // 2900-2909: that component's step falls back to its explicit forces) and goes on as 1.
 //
-// What bounds it: small frames by the chain of dependent panels (a panel ~11 us: the diagonal tile's inverse factor 5.3, a
-// product with it 2.5, the update of the next diagonal tile 2.5, their flags 1 each), large ones by the fp64 rate. 48:
-// a multiple of a node's 6 degrees of freedom and of the instruction's 8, three CTAs an SM with both operands' ring.
-// Measured on B200 (factorization and solves alone; before: minimum-degree fronts, a launch a panel and a launch an
-// update, 32 x 32 tiles on the plain fp64 units): the 64 x 64 plate 0.63 ms (3.9), the 10k-node shell body 1.52 (7.8),
-// the 50k-node one 6.7 (38.0): 63.3 GFLOP at 9.4 TFLOP/s of the 35.5 a cuBLAS DGEMM reaches.
+// What bounds it: small frames by the chain of dependent panels (a panel ~11 us: the diagonal tile's inverse factor 4.0, a
+// product with it 2.5, the update of the next diagonal tile 2.5, their flags 1 each; backward 2.7), large ones by the
+// fp64 rate. 48: a multiple of a node's 6 degrees of freedom and of the instruction's 8, three CTAs an SM with both
+// operands' ring. Measured on B200 (factorization and solves alone; before: minimum-degree fronts, a launch a panel and
+// a launch an update, 32 x 32 tiles on the plain fp64 units): the 21 x 21 plate 0.21 ms, the 64 x 64 plate 0.56 (3.9),
+// the 10k-node shell body 1.43 (7.8), the 50k-node one 6.3 (38.0): 63.3 GFLOP at 10.1 TFLOP/s of the 35.5 a cuBLAS
+// DGEMM reaches, 24 to 28 in the large fronts.
 #pragma once
 
 #include "bl_fem_kernels.cuh"
@@ -46,16 +47,16 @@ struct MfDev {
     const int* cpos;
     const int* cptr;
     const int* child;
+    const int* pan;      // per global column: its panel
     const int* eptr;     // per tile + 1: its assembled blocks in ent
     const int2* ent;     // (off-diagonal block, or -(column + 1) for a diagonal one; 8 row slot + column slot)
     double* pool;        // kMfTile a tile
     const int4* task;    // (front, i, j, kind)
-    int ntask, ncomp;
-    int* ctr;            // zeroed before each launch: [0] the next task, [1] abort, then
+    int nfactor, ntask, ncomp; // the factorization's tasks, then the backward solves'
+    int* ctr;            // zeroed before each step: [0] the next task, [1] abort, [2] the next backward one, then
     int* fdone;          // per front
-    int* xdone;          // per front: panels solved backward
     int* tflag;          // per tile
-    int* xflag;          // per panel
+    int* xflag;          // per panel: the backward solve's warps that are done (4)
 };
 // entry (r, c) of a tile
 __host__ __device__ __forceinline__ int mf_at(int r, int c) {
@@ -184,18 +185,19 @@ __device__ __forceinline__ bool mf_inv8(const double* B, double* inv, int lane) 
     return ok;
 }
 
-// The inverse Y of the diagonal tile's Cholesky factor (lower; zero before); D (lower) is overwritten by the factor's
-// blocks below the diagonal. By columns of 8: the first warp makes the chain - L_(k+1)k = D_(k+1)k inv_k^T, the next
-// diagonal block less L L^T, its factor's inverse inv_(k+1) - while the other three make the rest of the block column,
-// the later blocks' updates and the inverse's rows: Y_kk = inv_k, Y_kj = -inv_k S_j, then the next row's
-// S_j = sum_(j <= m <= k) L_(k+1)m Y_mj; a warp keeps its columns j (j mod 3). One barrier a column of blocks. The chain
-// bounds it: 48 columns of an inverse square root, a multiply and a multiply-add. scr: 5 blocks of S, 2 of inverses in
-// turn, the chain's L. False at a pivot that is not positive.
-// (9.6 us with panels of 16 columns, plain multiply-adds for the updates and the inverse after them.)
-constexpr int kMfScr = 8 * 64;
-__device__ __forceinline__ bool mf_factor_tile(double* D, double* Y, double* scr, int* bad) {
+// The transposed inverse X of the diagonal tile's Cholesky factor (upper; zero before); D (lower) is overwritten by the
+// factor's blocks below the diagonal. The identity is carried as six more block rows below the tile: eliminating the
+// tile's columns turns it into the transposed inverse. By columns of 8: the first warp makes the chain -
+// L_(k+1)k = D_(k+1)k inv_k^T, the next diagonal block less L L^T, its factor's inverse inv_(k+1) - while the other
+// three make the rest of the block column (always six blocks) and its updates of the later blocks, evenly. One
+// barrier a column of blocks. The chain bounds it: 48 columns of an inverse square root, a multiply and a
+// multiply-add. scr: 2 blocks of inverses in turn, the chain's L. False at a pivot that is not positive.
+// (9.6 us with panels of 16 columns, plain multiply-adds for the updates and the inverse after them; 5.3 with the
+// inverse's rows made one after the other.)
+constexpr int kMfScr = 3 * 64;
+__device__ __forceinline__ bool mf_factor_tile(double* D, double* X, double* scr, int* bad) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w = warp - 1, pr = mf_pair8(lane);
-    double *S = scr, *inv = scr + 5 * 64;
+    double *inv = scr, *Lc = scr + 2 * 64;
     auto at2 = [&](double* p) -> double2& { return *reinterpret_cast<double2*>(p + pr); };
     if (warp == 0 && !mf_inv8(D, inv, lane) && lane == 0) *bad = 1;
     __syncthreads();
@@ -203,87 +205,73 @@ __device__ __forceinline__ bool mf_factor_tile(double* D, double* Y, double* scr
         const double* ik = inv + 64 * (kb & 1);
         if (warp == 0) {
             if (kb < 5) {
-                double* L = D + mf_blk(kb + 1, kb);
                 double* N = D + mf_blk(kb + 1, kb + 1);
                 double t[2] = {0.0, 0.0}, u[2] = {0.0, 0.0};
-                mf_abt8(t, L, ik, lane);
-                at2(S + 7 * 64) = make_double2(t[0], t[1]); // (the chain's own copy: another warp stores L for the rest)
+                mf_abt8(t, D + mf_blk(kb + 1, kb), ik, lane);
+                at2(Lc) = make_double2(t[0], t[1]); // (the chain's own copy: another warp stores L for the rest)
                 asm volatile("bar.arrive 2, 128;" ::: "memory");
                 __syncwarp();
-                mf_abt8(u, S + 7 * 64, S + 7 * 64, lane);
+                mf_abt8(u, Lc, Lc, lane);
                 at2(N) = make_double2(at2(N).x - u[0], at2(N).y - u[1]);
                 __syncwarp();
                 if (!mf_inv8(N, inv + 64 * ((kb + 1) & 1), lane) && lane == 0) *bad = 1;
             }
         } else {
-            // the block column: rows kb + 1 + w, kb + 4 + w
+            // the block column: the tile's rows kb + 1 .. 5, then the identity's 0 .. kb; two blocks a warp
             double t[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll
-            for (int x = 0; x < 2; x++)
-                if (kb + 1 + w + 3 * x < 6) mf_abt8(t[x], D + mf_blk(kb + 1 + w + 3 * x, kb), ik, lane);
-            // (the chain reads D_(k+1)k too, at the start of this step: its copy is made before this one is stored)
-            if (kb < 5) asm volatile("bar.sync 2, 128;" ::: "memory");
-#pragma unroll
-            for (int x = 0; x < 2; x++)
-                if (kb + 1 + w + 3 * x < 6) at2(D + mf_blk(kb + 1 + w + 3 * x, kb)) = make_double2(t[x][0], t[x][1]);
-            // the inverse's row kb
+            double* row[2]; // (the block row's first block; its others lie mf_blk(0, c) from it)
+            int last[2];    // its last block column to update
 #pragma unroll
             for (int x = 0; x < 2; x++) {
-                const int j = w + 3 * x;
-                if (j < kb) {
-                    double u[2] = {0.0, 0.0};
-                    mf_ab8(u, ik, S + 64 * j, lane);
-                    at2(Y + mf_blk(kb, j)) = make_double2(-u[0], -u[1]);
-                } else if (j == kb) {
-                    at2(Y + mf_blk(kb, j)) = *reinterpret_cast<const double2*>(ik + pr);
-                }
+                const int q = w + 3 * x, i = q - (5 - kb);
+                row[x] = (i < 0 ? D : X) + mf_blk(i < 0 ? kb + 1 + q : i, 0);
+                last[x] = i >= 0 ? 5 : q == 0 ? kb : kb + 1 + q; // (row kb + 1's one block is the chain's)
+                double a0 = (lane >> 2) == (lane & 3) ? 1.0 : 0.0, a1 = (lane >> 2) == (lane & 3) + 4 ? 1.0 : 0.0; // (the identity's own block)
+                if (i != kb) a0 = row[x][mf_blk(0, kb) + lane], a1 = row[x][mf_blk(0, kb) + 32 + lane];
+                mf_mma(t[x], a0, ik[lane]), mf_mma(t[x], a1, ik[32 + lane]);
             }
+            // (the chain reads D_(k+1)k too, at the start of this step: its copy is made before this one is stored)
+            if (kb < 5) asm volatile("bar.sync 2, 128;" ::: "memory");
+            else __syncwarp();
+#pragma unroll
+            for (int x = 0; x < 2; x++) at2(row[x] + mf_blk(0, kb)) = make_double2(t[x][0], t[x][1]);
             asm volatile("bar.sync 1, 96;" ::: "memory"); // (the three warps: the block column is there)
-            // the later blocks (rb, cb), cb > kb, but the chain's; pairs by descending cb, at most five a warp
-            const int nb = (5 - kb) * (6 - kb) / 2;
-            double v[5][2];
-            int at[5];
+            // the later blocks of these two rows less their product with the block column (a loop of few instructions:
+            // unrolled over its blocks it waited for its code)
+            double a[2][2];
 #pragma unroll
-            for (int x = 0; x < 5; x++) {
-                const int b = w + 3 * x;
-                v[x][0] = v[x][1] = 0.0, at[x] = -1;
-                if (b >= nb) continue;
-                const int cb = b < 1 ? 5 : b < 3 ? 4 : b < 6 ? 3 : b < 10 ? 2 : 1, rb = cb + b - (b < 1 ? 0 : b < 3 ? 1 : b < 6 ? 3 : b < 10 ? 6 : 10);
-                if (rb == kb + 1) continue;
-                mf_abt8(v[x], D + mf_blk(rb, kb), D + mf_blk(cb, kb), lane);
-                at[x] = mf_blk(rb, cb);
-            }
-#pragma unroll
-            for (int x = 0; x < 5; x++)
-                if (at[x] >= 0) at2(D + at[x]) = make_double2(at2(D + at[x]).x - v[x][0], at2(D + at[x]).y - v[x][1]);
-            if (kb < 5)
+            for (int x = 0; x < 2; x++) a[x][0] = -row[x][mf_blk(0, kb) + lane], a[x][1] = -row[x][mf_blk(0, kb) + 32 + lane];
+#pragma unroll 1
+            for (int cb = kb + 1; cb < 6; cb++) {
+                const double* L = D + mf_blk(cb, kb);
+                const double b0 = L[lane], b1 = L[32 + lane];
 #pragma unroll
                 for (int x = 0; x < 2; x++) {
-                    const int j = w + 3 * x;
-                    if (j > kb) continue;
-                    double u[2][2] = {{0.0, 0.0}, {0.0, 0.0}}; // (two sums: the instruction's latency)
-                    for (int m = j; m <= kb; m += 2) {
-                        mf_ab8(u[0], D + mf_blk(kb + 1, m), Y + mf_blk(m, j), lane);
-                        if (m + 1 <= kb) mf_ab8(u[1], D + mf_blk(kb + 1, m + 1), Y + mf_blk(m + 1, j), lane);
-                    }
-                    at2(S + 64 * j) = make_double2(u[0][0] + u[1][0], u[0][1] + u[1][1]);
+                    if (cb > last[x]) continue;
+                    double2 d = at2(row[x] + mf_blk(0, cb));
+                    double v[2] = {d.x, d.y};
+                    mf_mma(v, a[x][0], b0), mf_mma(v, a[x][1], b1);
+                    at2(row[x] + mf_blk(0, cb)) = make_double2(v[0], v[1]);
                 }
+            }
         }
         __syncthreads();
     }
     return *bad == 0;
 }
 
-// The tile's assembled blocks and its children's contributions into C (shared, zeroed). False when the launch aborts.
-__device__ __forceinline__ bool mf_assemble(const FemDev& F, const MfDev& M, const MfFrontDev& fr, int i, int j, double* C) {
+// The tile's assembled blocks and its children's Schur complements into C (shared). The children's maps - which of a
+// child's row nodes falls on each of the tile's 8 row and 8 column slots - are made before they are waited for; then a
+// thread gathers three rows of six entries each, over the children in their order. False when the launch aborts.
+constexpr int kMfKids = 16; // children at a time (8 threads each)
+struct MfKids {
+    int base[kMfKids], nt[kMfKids], P[kMfKids], bt[kMfKids], br[kMfKids]; // first tile, tiles a side, pivot tiles, b's tile and row
+    int row[kMfKids][8], col[kMfKids][8];                                 // its row node on each slot, -1: none
+};
+__device__ __forceinline__ bool mf_assemble(const FemDev& F, const MfDev& M, const MfFrontDev& fr, int i, int j, double* C, MfKids& K) {
     const int tid = threadIdx.x;
     for (int e = tid; e < kMfTile / 2; e += kMfThreads) reinterpret_cast<double2*>(C)[e] = make_double2(0.0, 0.0);
-    bool ok = true;
-    for (int q = fr.child0 + tid; q < fr.child1; q += kMfThreads) {
-        const int c = M.child[q];
-        ok = ok && mf_wait(M.fdone + c, M.fr[c].need, M.ctr + 1);
-    }
-    if (__syncthreads_or(!ok)) return false;
+    __syncthreads();
     if (j < fr.P) {
         const int t = fr.tile0 + mf_tix(fr.nt, i, j), e0 = M.eptr[t], e1 = M.eptr[t + 1];
         for (int e = tid; e < 18 * (e1 - e0); e += kMfThreads) { // (a thread a pair of a block's entries)
@@ -295,45 +283,84 @@ __device__ __forceinline__ bool mf_assemble(const FemDev& F, const MfDev& M, con
         if (i == fr.bt && tid < kMfT && 8 * j + tid / 6 < fr.npiv) C[mf_at(fr.br, tid)] = F.rhs[6 * (size_t)M.idx[fr.idx0 + 8 * j + tid / 6] + tid % 6];
         if (i == j && tid < kMfT && kMfT * j + tid >= fr.p) C[mf_at(tid, tid)] = 1.0; // (past the last pivot: an identity)
     }
-    for (int q = fr.child0; q < fr.child1; q++) {
-        const MfFrontDev cf = M.fr[M.child[q]];
-        const int* cp = M.cptr + cf.cptr0;
-        const int* pos = M.cpos + cf.cpos0;
-        const int ra = cp[i], rb = cp[i + 1], ca = cp[j], nc = cp[j + 1] - ca;
-        if (nc == 0 || (ra == rb && i != fr.bt)) continue;
-        __syncthreads();
-        const double* S = M.pool + (size_t)cf.tile0 * kMfTile;
-        for (int e = tid; e < 6 * (rb - ra) * nc; e += kMfThreads) {
-            const int qc = ca + e % nc, t = e / nc, a = t % 6, qr = ra + t / 6;
-            if (qr < qc) continue;
-            const double* T = S + (size_t)mf_tix(cf.nt, cf.P + (qr >> 3), cf.P + (qc >> 3)) * kMfTile;
-            const int sr = 6 * (qr & 7) + a, sc = 6 * (qc & 7), dr = 6 * (pos[qr] & 7) + a, dc = 6 * (pos[qc] & 7);
-            double2 v[3];
+    for (int q0 = fr.child0; q0 < fr.child1; q0 += kMfKids) {
+        const int nq = min(kMfKids, fr.child1 - q0), q = tid >> 3, k = tid & 7;
+        if (q0 > fr.child0) __syncthreads(); // (the maps' readers are done)
+        bool ok = true;
+        if (q < nq) {
+            const int c = M.child[q0 + q];
+            const MfFrontDev& cf = M.fr[c];
+            const int* cp = M.cptr + cf.cptr0;
+            const int* pos = M.cpos + cf.cpos0;
+            const int rx = cp[i] + k, re = cp[i + 1], cx = cp[j] + k, ce = cp[j + 1];
+            const int rp = rx < re ? pos[rx] : -1, cq = cx < ce ? pos[cx] : -1;
+            if (k == 0) K.base[q] = cf.tile0, K.nt[q] = cf.nt, K.P[q] = cf.P, K.bt[q] = cf.bt, K.br[q] = cf.br;
+            K.row[q][k] = -1, K.col[q][k] = -1;
+            __syncwarp(__activemask());
+            if (rp >= 0) K.row[q][rp & 7] = rx;
+            if (cq >= 0) K.col[q][cq & 7] = cx;
+            if (k == 0) ok = mf_wait(M.fdone + c, cf.need, M.ctr + 1);
+        }
+        if (__syncthreads_or(!ok)) return false;
+        double2 v[3][3];
+        bool any[3] = {false, false, false};
 #pragma unroll
-            for (int b = 0; b < 3; b++) v[b] = __ldcg(reinterpret_cast<const double2*>(T + mf_at(sr, sc + 2 * b)));
+        for (int m = 0; m < 3; m++)
+#pragma unroll
+            for (int b = 0; b < 3; b++) v[m][b] = make_double2(0.0, 0.0);
+#pragma unroll 1
+        for (int c = 0; c < nq; c++) {
+            const double* S = M.pool + (size_t)K.base[c] * kMfTile;
+            const int nt = K.nt[c], P = K.P[c];
+            double2 u[3][3];
+            bool on[3];
+#pragma unroll
+            for (int m = 0; m < 3; m++) { // (row a of the node pair (dr, dc))
+                const int g = tid + kMfThreads * m, pair = g / 6, a = g - 6 * pair, qr = K.row[c][pair >> 3], qc = K.col[c][pair & 7];
+                on[m] = qr >= qc && qc >= 0;
+                if (!on[m]) continue;
+                any[m] = true;
+                const double* T = S + (size_t)mf_tix(nt, P + (qr >> 3), P + (qc >> 3)) * kMfTile;
+#pragma unroll
+                for (int b = 0; b < 3; b++) u[m][b] = __ldcg(reinterpret_cast<const double2*>(T + mf_at(6 * (qr & 7) + a, 6 * (qc & 7) + 2 * b)));
+            }
+#pragma unroll
+            for (int m = 0; m < 3; m++)
+                if (on[m])
+#pragma unroll
+                    for (int b = 0; b < 3; b++) v[m][b].x += u[m][b].x, v[m][b].y += u[m][b].y;
+        }
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+            if (!any[m]) continue;
+            const int g = tid + kMfThreads * m, pair = g / 6, a = g - 6 * pair;
 #pragma unroll
             for (int b = 0; b < 3; b++) {
-                double2* d = reinterpret_cast<double2*>(C + mf_at(dr, dc + 2 * b));
+                double2* d = reinterpret_cast<double2*>(C + mf_at(6 * (pair >> 3) + a, 6 * (pair & 7) + 2 * b));
                 const double2 o = *d;
-                *d = make_double2(o.x + v[b].x, o.y + v[b].y);
+                *d = make_double2(o.x + v[m][b].x, o.y + v[m][b].y);
             }
         }
-        if (i == fr.bt)
-            for (int e = tid; e < 6 * nc; e += kMfThreads) {
-                const int qc = ca + e / 6;
-                const double* T = S + (size_t)mf_tix(cf.nt, cf.bt, cf.P + (qc >> 3)) * kMfTile;
-                C[mf_at(fr.br, 6 * (pos[qc] & 7) + e % 6)] += __ldcg(T + mf_at(cf.br, 6 * (qc & 7) + e % 6));
+        if (i == fr.bt && tid < kMfT) { // (b's row)
+            double t = 0;
+            for (int c = 0; c < nq; c++) {
+                const int qc = K.col[c][tid / 6];
+                if (qc >= 0)
+                    t += __ldcg(M.pool + (size_t)(K.base[c] + mf_tix(K.nt[c], K.bt[c], K.P[c] + (qc >> 3))) * kMfTile + mf_at(K.br[c], 6 * (qc & 7) + tid % 6));
             }
+            C[mf_at(fr.br, tid)] += t;
+        }
     }
     __syncthreads();
     return true;
 }
 
 // One tile of a front (alone: by this CTA alone, its inputs of the same front written by this CTA before)
-__device__ bool mf_tile(const FemDev& F, const MfDev& M, const MfFrontDev& fr, int f, int i, int j, bool alone, double* ring, double* C) {
+__device__ __forceinline__ bool mf_tile(const FemDev& F, const MfDev& M, const MfFrontDev& fr, int f, int i, int j, bool alone, double* ring, double* C) {
     __shared__ int s_ready, s_bad;
+    __shared__ MfKids s_kids;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wr = warp & 1, wc = warp >> 1;
-    if (!mf_assemble(F, M, fr, i, j, C)) return false;
+    if (!mf_assemble(F, M, fr, i, j, C, s_kids)) return false;
     const double* base = M.pool + (size_t)fr.tile0 * kMfTile;
     double acc[3][3][2];
 #pragma unroll
@@ -396,9 +423,9 @@ __device__ bool mf_tile(const FemDev& F, const MfDev& M, const MfFrontDev& fr, i
         return true;
     }
     if (same) {
-        double* Y = ring;
+        double* X = ring;
         if (tid == 0) s_bad = 0;
-        for (int e = tid; e < kMfTile / 2; e += kMfThreads) reinterpret_cast<double2*>(Y)[e] = make_double2(0.0, 0.0);
+        for (int e = tid; e < kMfTile / 2; e += kMfThreads) reinterpret_cast<double2*>(X)[e] = make_double2(0.0, 0.0);
 #pragma unroll
         for (int x = 0; x < 3; x++)
 #pragma unroll
@@ -407,8 +434,12 @@ __device__ bool mf_tile(const FemDev& F, const MfDev& M, const MfFrontDev& fr, i
                 *c = make_double2(c->x - acc[x][y][0], c->y - acc[x][y][1]);
             }
         __syncthreads();
-        const bool ok = mf_factor_tile(C, Y, ring + kMfTile, &s_bad);
-        for (int e = tid; e < kMfTile / 2; e += kMfThreads) reinterpret_cast<double2*>(out)[e] = reinterpret_cast<const double2*>(Y)[e];
+        const bool ok = mf_factor_tile(C, X, ring + kMfTile, &s_bad);
+        for (int e = tid; e < kMfTile / 2; e += kMfThreads) { // (the inverse: X transposed; the pair e of the tile's order)
+            const int kc = e / (kMfChunk / 2), q = e % (kMfChunk / 2), rb = q / 64, cb = (q / 16) & 3, l = 2 * (q & 15);
+            const int r = 8 * rb + l / 4, c = 16 * kc + 4 * cb + l % 4;
+            reinterpret_cast<double2*>(out)[e] = make_double2(X[mf_at(c, r)], X[mf_at(c + 1, r)]);
+        }
         if (!ok && tid == 0) atomicExch(&F.comp_fail[fr.comp], 1);
     } else {
         // X = A L_jj^-T
@@ -463,72 +494,85 @@ __device__ __forceinline__ double mf_sum_rows(double t) {
     return t + __shfl_xor_sync(0xffffffffu, t, 16);
 }
 
-// x of a front's panel s, from its rows' x (its ancestors') and its later panels'
-constexpr int kMfXTiles = 96; // row tiles' x held at a time
-__device__ bool mf_backward(const FemDev& F, const MfDev& M, const MfFrontDev& fr, int f, int s, double* ring) {
-    double* xs = ring;                       // kMfXTiles x 48
-    double* z = ring + kMfXTiles * kMfT;     // 48
+// x of a front's panel s: its rows' x (its ancestors') as they become known - the highest first, up to kMfXTiles tiles at a
+// time, each group when the panel of its lowest node is solved (then all above it are) - then its own later panels', then
+// x_s = L_ss^-T z. A warp that has stored its part of x_s adds one to the panel's flag.
+constexpr int kMfXTiles = 8;
+__device__ __forceinline__ bool mf_backward(const FemDev& F, const MfDev& M, const MfFrontDev& fr, int s, double* xs, double* z) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double* base = M.pool + (size_t)fr.tile0 * kMfTile;
     const int* idx = M.idx + fr.idx0;
-    double acc[3] = {0, 0, 0}, li[3][6], v[3][6];
-    // its tiles: a root's by their flags; below, the parent's solution comes after the whole factorization of both
+    double acc[3] = {0, 0, 0}, v[3][6];
+    double y[3]; // (this lane's of the panel's y)
+#pragma unroll
+    for (int m = 0; m < 3; m++) y[m] = __ldcg(base + (size_t)mf_tix(fr.nt, fr.bt, s) * kMfTile + mf_at(fr.br, 4 * (warp + 4 * m) + (lane & 3)));
     bool ok = true;
-    if (fr.parent < 0) {
-        for (int i = s + tid; i < fr.nt; i += kMfThreads) ok = ok && mf_wait(M.tflag + fr.tile0 + mf_tix(fr.nt, i, s), 1, M.ctr + 1);
-    } else if (tid == 0) {
-        ok = mf_wait(M.xdone + fr.parent, M.fr[fr.parent].P, M.ctr + 1);
-    }
-    if (__syncthreads_or(!ok)) return false;
-    mf_load_cols(li, base + (size_t)mf_tix(fr.nt, s, s) * kMfTile, warp, lane);
-    const double y = tid < kMfT ? __ldcg(base + (size_t)mf_tix(fr.nt, fr.bt, s) * kMfTile + mf_at(fr.br, tid)) : 0.0;
-    if (fr.nrow > 0) {
-        const int nrt = (fr.nrow + 7) / 8;
-        for (int t0 = 0; t0 < nrt; t0 += kMfXTiles) {
-            const int nt = min(kMfXTiles, nrt - t0);
-            if (t0 > 0) __syncthreads();
-            for (int e = tid; e < nt * kMfT; e += kMfThreads) {
-                const int q = 8 * t0 + e / 6;
-                xs[e] = q < fr.nrow ? __ldcg(F.rhs + 6 * (size_t)idx[fr.npiv + q] + e % 6) : 0.0;
-            }
-            __syncthreads();
-            for (int t = 0; t < nt; t++) {
-                mf_load_cols(v, base + (size_t)mf_tix(fr.nt, fr.P + t0 + t, s) * kMfTile, warp, lane);
-                mf_dot_cols(acc, v, xs + t * kMfT, lane);
-            }
+    for (int t1 = (fr.nrow + 7) / 8; t1 > 0; t1 -= kMfXTiles) {
+        const int t0 = max(0, t1 - kMfXTiles), nt = t1 - t0;
+        const double* L = base + (size_t)mf_tix(fr.nt, fr.P + t0, s) * kMfTile; // (a column's tiles lie one after the other)
+        mf_load_cols(v, L, warp, lane);                                      // (before the wait)
+        int at[kMfXTiles * kMfT / kMfThreads];
+#pragma unroll
+        for (int x = 0; x < kMfXTiles * kMfT / kMfThreads; x++) {
+            const int e = tid + kMfThreads * x, q = 8 * t0 + e / 6;
+            at[x] = e < nt * kMfT && q < fr.nrow ? 6 * idx[fr.npiv + q] + e % 6 : -1;
         }
+        if (ok) ok = mf_wait(M.xflag + M.pan[idx[fr.npiv + 8 * t0]], 4, M.ctr + 1);
+#pragma unroll
+        for (int x = 0; x < kMfXTiles * kMfT / kMfThreads; x++) xs[tid + kMfThreads * x] = at[x] >= 0 ? __ldcg(F.rhs + at[x]) : 0.0;
+        if (__syncthreads_or(!ok)) return false;
+        for (int t = 0; t < nt; t++) {
+            double w[3][6];
+            if (t + 1 < nt) mf_load_cols(w, L + (size_t)(t + 1) * kMfTile, warp, lane);
+            mf_dot_cols(acc, v, xs + t * kMfT, lane);
+#pragma unroll
+            for (int m = 0; m < 3; m++)
+#pragma unroll
+                for (int rb = 0; rb < 6; rb++) v[m][rb] = w[m][rb];
+        }
+        __syncthreads();
     }
     for (int i = fr.P - 1; i > s; i--) {
         mf_load_cols(v, base + (size_t)mf_tix(fr.nt, i, s) * kMfTile, warp, lane); // (before the wait)
-        if (tid == 0) ok = mf_wait(M.xflag + fr.pan0 + i, 1, M.ctr + 1);
+        if (tid < kMfT) {
+            const int at = kMfT * i + tid < fr.p ? 6 * idx[8 * i + tid / 6] + tid % 6 : -1;
+            ok = mf_wait(M.xflag + fr.pan0 + i, 4, M.ctr + 1);
+            xs[(i & 1) * kMfT + tid] = at >= 0 ? __ldcg(F.rhs + at) : 0.0;
+        }
         if (__syncthreads_or(!ok)) return false;
-        if (tid < kMfT) xs[tid] = kMfT * i + tid < fr.p ? __ldcg(F.rhs + 6 * (size_t)idx[8 * i + tid / 6] + tid % 6) : 0.0;
-        __syncthreads();
-        mf_dot_cols(acc, v, xs, lane);
+        mf_dot_cols(acc, v, xs + (i & 1) * kMfT, lane);
     }
+    mf_load_cols(v, base + (size_t)mf_tix(fr.nt, s, s) * kMfTile, warp, lane); // (L_ss^-1)
 #pragma unroll
     for (int m = 0; m < 3; m++) {
         const double t = mf_sum_rows(acc[m]);
-        if (lane < 4) z[4 * (warp + 4 * m) + lane] = t;
+        const int c = 4 * (warp + 4 * m) + lane;
+        if (lane < 4) z[c] = y[m] - t;
         acc[m] = 0.0;
     }
     __syncthreads();
-    if (tid < kMfT) z[tid] = y - z[tid];
-    __syncthreads();
-    mf_dot_cols(acc, li, z, lane);
+    mf_dot_cols(acc, v, z, lane);
 #pragma unroll
     for (int m = 0; m < 3; m++) {
         const double t = mf_sum_rows(acc[m]);
         const int c = kMfT * s + 4 * (warp + 4 * m) + lane;
         if (lane < 4 && c < fr.p) F.rhs[6 * (size_t)idx[c / 6] + c % 6] = t;
     }
-    __syncthreads();
-    if (tid == 0) mf_st_release(M.xflag + fr.pan0 + s, 1), mf_add_release(M.xdone + f, 1);
+    __syncwarp();
+    if (lane == 0) mf_add_release(M.xflag + fr.pan0 + s, 1);
+    __syncthreads(); // (xs, z: the next task's)
     return true;
 }
 
-// 128 threads, 66 KB of shared memory: three CTAs an SM
-__global__ void __launch_bounds__(kMfThreads, 3) k_mf_solve(FemDev F, MfDev M, uint32_t* deverr) {
+// the launch was aborted: flagged, every component failed
+__device__ __forceinline__ void mf_leave(const FemDev& F, const MfDev& M, uint32_t* deverr) {
+    if (!*(volatile int*)(M.ctr + 1)) return;
+    if (threadIdx.x == 0) atomicOr(deverr, DEVERR_TIMEOUT);
+    for (int c = threadIdx.x; c < M.ncomp; c += kMfThreads) F.comp_fail[c] = 1;
+}
+
+// The factorization: 128 threads, 66 KB of shared memory, three CTAs an SM
+__global__ void __launch_bounds__(kMfThreads, 3) k_mf_factor(FemDev F, MfDev M, uint32_t* deverr) {
     extern __shared__ __align__(16) double mf_smem[];
     __shared__ int s_task;
     double* ring = mf_smem;
@@ -538,32 +582,42 @@ __global__ void __launch_bounds__(kMfThreads, 3) k_mf_solve(FemDev F, MfDev M, u
         __syncthreads();
         const int t = s_task;
         __syncthreads();
-        if (t < 0 || t >= M.ntask) break;
+        if (t < 0 || t >= M.nfactor) break;
         const int4 task = M.task[t];
         const MfFrontDev fr = M.fr[task.x];
+        // one tile, or all of a front's (a root's Schur complement is nobody's)
+        const bool alone = task.w == MF_FRONT;
+        const int j1 = !alone ? task.z + 1 : fr.parent >= 0 ? fr.nt : fr.P;
         bool ok = true;
-        if (task.w == MF_TILE) {
-            ok = mf_tile(F, M, fr, task.x, task.y, task.z, false, ring, C);
-        } else if (task.w == MF_BACK) {
-            ok = mf_backward(F, M, fr, task.x, task.z, ring);
-        } else {
-            const int last = fr.parent >= 0 ? fr.nt : fr.P; // (a root's Schur complement is nobody's)
-            for (int j = 0; ok && j < last; j++)
-                for (int i = j; ok && i < fr.nt; i++) {
-                    ok = mf_tile(F, M, fr, task.x, i, j, true, ring, C);
-                    __syncthreads();
-                }
-            if (ok && threadIdx.x == 0) {
-                for (int k = 0; k < fr.nt; k++) mf_st_release(M.tflag + fr.tile0 + k, 1); // (its one pivot column's)
-                mf_add_release(M.fdone + task.x, 1);
+#pragma unroll 1
+        for (int j = task.z; ok && j < j1; j++) {
+            const int i1 = alone ? fr.nt : task.y + 1;
+#pragma unroll 1
+            for (int i = alone ? j : task.y; ok && i < i1; i++) {
+                ok = mf_tile(F, M, fr, task.x, i, j, alone, ring, C);
+                if (alone) __syncthreads();
             }
         }
+        if (alone && ok && threadIdx.x == 0) mf_add_release(M.fdone + task.x, 1);
         if (!ok) break;
     }
-    if (*(volatile int*)(M.ctr + 1)) {
-        if (threadIdx.x == 0) atomicOr(deverr, DEVERR_TIMEOUT);
-        for (int c = threadIdx.x; c < M.ncomp; c += kMfThreads) F.comp_fail[c] = 1;
+    mf_leave(F, M, deverr);
+}
+
+// The backward solves, after it
+__global__ void __launch_bounds__(kMfThreads, 3) k_mf_back(FemDev F, MfDev M, uint32_t* deverr) {
+    __shared__ double xs[kMfXTiles * kMfT], z[kMfT];
+    __shared__ int s_task;
+    for (;;) {
+        if (threadIdx.x == 0) s_task = *(volatile int*)(M.ctr + 1) ? -1 : M.nfactor + atomicAdd(M.ctr + 2, 1);
+        __syncthreads();
+        const int t = s_task;
+        __syncthreads();
+        if (t < 0 || t >= M.ntask) break;
+        const int4 task = M.task[t];
+        if (!mf_backward(F, M, M.fr[task.x], task.z, xs, z)) break;
     }
+    mf_leave(F, M, deverr);
 }
 
 } // namespace blg

@@ -210,11 +210,11 @@ struct bl_gpu_ctx {
     // the multifrontal factorization and solves (bl_multifrontal.cuh), fem_mode 2: fronts, their maps, tasks, pool, flags
     MfDev mf{};
     DevBuf<MfFrontDev> mf_fr;
-    DevBuf<int> mf_idx, mf_cpos, mf_cptr, mf_child, mf_eptr, mf_ctr;
+    DevBuf<int> mf_idx, mf_cpos, mf_cptr, mf_child, mf_eptr, mf_pan, mf_ctr;
     DevBuf<int2> mf_ent;
     DevBuf<int4> mf_task;
     DevBuf<double> mf_pool;
-    int mf_grid = 1, mf_levels = 0;
+    int mf_grid = 1, mf_back_grid = 1, mf_levels = 0;
     int fem_mode = 0;                          // the factorization in use: fem_dense_front, 3 resolved to 2
     unsigned long long wait_ns = 1000000000ull; // the beams kernel's bound on a wait for its bulk copies (bulk_wait_s)
     double mf_flops = 0;
@@ -288,7 +288,7 @@ static void free_fem(bl_gpu_ctx* c) {
     c->feat.free_(), c->prev_dv.free_(), c->adj_ptr.free_(), c->adj.free_();
     c->gdiag.free_(), c->gu.free_(), c->rb.free_(), c->goff.free_(), c->tn.free_();
     c->fcol.free_(), c->fchain.free_(), c->fblk.free_(), c->fD.free_(), c->fb.free_(), c->front = FrontDev{}, c->front_level = 0;
-    c->mf_fr.free_(), c->mf_idx.free_(), c->mf_cpos.free_(), c->mf_cptr.free_(), c->mf_child.free_(), c->mf_eptr.free_(), c->mf_ctr.free_();
+    c->mf_fr.free_(), c->mf_idx.free_(), c->mf_cpos.free_(), c->mf_cptr.free_(), c->mf_child.free_(), c->mf_eptr.free_(), c->mf_pan.free_(), c->mf_ctr.free_();
     c->mf_ent.free_(), c->mf_task.free_(), c->mf_pool.free_(), c->mf = MfDev{}, c->mf_levels = 0, c->mf_flops = 0;
     c->mn.free_(), c->mmeta.free_(), c->mL0.free_(), c->mq.free_(), c->mfa.free_(), c->mta.free_(), c->mtb.free_(), c->mtan.free_();
     c->msec.free_(), c->mon.free_(), c->mkw.free_(), c->mkv.free_(), c->NM = 0;
@@ -556,26 +556,28 @@ static int commit_multifrontal(bl_gpu_ctx* c, const std::vector<int>& col_ptr, c
     const int nfr = (int)Y.fr.size();
     int rc;
     if ((rc = upload_vec(c, c->mf_fr, Y.fr)) || (rc = upload_vec(c, c->mf_idx, P.idx)) || (rc = upload_vec(c, c->mf_cpos, Y.cpos)) ||
-        (rc = upload_vec(c, c->mf_cptr, Y.cptr)) || (rc = upload_vec(c, c->mf_child, P.child)) || (rc = upload_vec(c, c->mf_eptr, Y.eptr)) ||
+        (rc = upload_vec(c, c->mf_cptr, Y.cptr)) || (rc = upload_vec(c, c->mf_child, P.child)) || (rc = upload_vec(c, c->mf_eptr, Y.eptr)) || (rc = upload_vec(c, c->mf_pan, Y.pan)) ||
         (rc = upload_vec(c, c->mf_ent, Y.ent)) || (rc = upload_vec(c, c->mf_task, Y.task)))
         return rc;
     BL_CUDA(c, c->mf_pool.alloc((size_t)Y.tiles * kMfTile));
-    BL_CUDA(c, c->mf_ctr.alloc(4 + 2 * (size_t)nfr + (size_t)Y.tiles + Y.pans));
+    BL_CUDA(c, c->mf_ctr.alloc(4 + (size_t)nfr + (size_t)Y.tiles + Y.pans));
     MfDev& M = c->mf;
     M = MfDev{};
-    M.fr = c->mf_fr.p, M.idx = c->mf_idx.p, M.cpos = c->mf_cpos.p, M.cptr = c->mf_cptr.p, M.child = c->mf_child.p, M.eptr = c->mf_eptr.p, M.ent = c->mf_ent.p;
-    M.pool = c->mf_pool.p, M.task = c->mf_task.p, M.ntask = (int)Y.task.size(), M.ncomp = ncomp;
-    M.ctr = c->mf_ctr.p, M.fdone = M.ctr + 4, M.xdone = M.fdone + nfr, M.tflag = M.xdone + nfr, M.xflag = M.tflag + Y.tiles;
-    // a CTA a task of the widest level, at most what is resident at once (a cooperative launch)
-    int per_sm = 0, nsm = 0;
-    BL_CUDA(c, cudaFuncSetAttribute(k_mf_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMfSmem));
-    BL_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mf_solve, kMfThreads, kMfSmem));
+    M.fr = c->mf_fr.p, M.idx = c->mf_idx.p, M.cpos = c->mf_cpos.p, M.cptr = c->mf_cptr.p, M.child = c->mf_child.p, M.pan = c->mf_pan.p, M.eptr = c->mf_eptr.p, M.ent = c->mf_ent.p;
+    M.pool = c->mf_pool.p, M.task = c->mf_task.p, M.nfactor = Y.nfactor, M.ntask = (int)Y.task.size(), M.ncomp = ncomp;
+    M.ctr = c->mf_ctr.p, M.fdone = M.ctr + 4, M.tflag = M.fdone + nfr, M.xflag = M.tflag + Y.tiles;
+    // a CTA a task of the widest level, at most what is resident at once (cooperative launches)
+    int per_sm = 0, back_sm = 0, nsm = 0;
+    BL_CUDA(c, cudaFuncSetAttribute(k_mf_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMfSmem));
+    BL_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mf_factor, kMfThreads, kMfSmem));
+    BL_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&back_sm, k_mf_back, kMfThreads, 0));
     BL_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->cfg.device));
-    if (per_sm < 1) return BL_GPU_ECUDA;
+    if (per_sm < 1 || back_sm < 1) return BL_GPU_ECUDA;
     c->mf_grid = std::min(per_sm * nsm, Y.widest);
+    c->mf_back_grid = std::min(back_sm * nsm, Y.widest_back);
     c->mf_levels = (int)P.level_ptr.size() - 1;
     c->mf_flops = P.flops;
-    c->chol_launches = 1;
+    c->chol_launches = 2;
     return BL_GPU_OK;
 }
 
@@ -1537,7 +1539,7 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
             if (learned) k_mlp_infer<<<(c->NF + kLanes - 1) / kLanes, kLanes, 0, s>>>(F, MD, c->guess.p, c->gscale.p);
             auto cholesky = [c, &F](cudaStream_t cs) {
                 if (c->fem_mode == 2) {
-                    // multifrontal: the whole factorization and its solves in one cooperative launch (its flags zeroed first)
+                    // multifrontal: the factorization, then the backward solves, a cooperative launch each (their flags zeroed first)
                     cudaMemsetAsync(c->mf_ctr.p, 0, sizeof(int) * c->mf_ctr.n, cs);
                     cudaLaunchConfig_t lc{};
                     lc.gridDim = dim3(c->mf_grid), lc.blockDim = dim3(kMfThreads), lc.dynamicSmemBytes = kMfSmem, lc.stream = cs;
@@ -1545,7 +1547,9 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
                     at[0].id = cudaLaunchAttributeCooperative;
                     at[0].val.cooperative = 1;
                     lc.attrs = at, lc.numAttrs = 1;
-                    cudaLaunchKernelEx(&lc, k_mf_solve, F, c->mf, c->deverr.p);
+                    cudaLaunchKernelEx(&lc, k_mf_factor, F, c->mf, c->deverr.p);
+                    lc.gridDim = dim3(c->mf_back_grid), lc.dynamicSmemBytes = 0;
+                    cudaLaunchKernelEx(&lc, k_mf_back, F, c->mf, c->deverr.p);
                     return;
                 }
                 // the levels of the elimination tree two launches each (factor; updates with the forward substitution),
