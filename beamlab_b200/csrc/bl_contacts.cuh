@@ -372,6 +372,7 @@ __global__ void __launch_bounds__(256) k_detect(const float4* __restrict__ nd, c
         const unsigned bits = __ballot_sync(0xffffffffu, hit);
         if ((threadIdx.x & 31) == 0) C.hbits[i >> 5] = bits;
     }
+    pdl_wait(); // (it needs the positions, not the forces: it runs beside the forces' kernel)
 }
 
 // ------------------------------------------------------------------------------------------ response (each substep)
@@ -584,6 +585,7 @@ __global__ void __launch_bounds__(kCollideThreads, 1) k_collide(const float4* __
     unsigned short* slot_lvl = reinterpret_cast<unsigned short*>(rec + kRecChunk); // per slot: its latest contact's level
     __shared__ int used, overflow, ncontacts, s_depth;
     const int root = blockIdx.x, tid = threadIdx.x;
+    pdl_wait();
     if (root >= nbodies) return;
     const int cnt = C.isl_pcnt[root];
     if (cnt <= 0 || bodies[root].island != root || !bodies[root].pairs) return;

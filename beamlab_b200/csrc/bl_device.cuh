@@ -27,6 +27,16 @@ enum : uint32_t { BF_BROKEN = 1, BF_NO_DEFORM = 4, BF_NO_BREAK = 8, BF_SHOCK = 6
 enum : uint32_t { BB_DEFORM = 1u << 16, BB_BREAK = 1u << 17, BB_DUCTILE = 1u << 18 };
 enum : uint32_t { DEVERR_CANDIDATES = 1, DEVERR_NONFINITE = 2, DEVERR_TIMEOUT = 1u << 6 };
 
+// Programmatic dependent launches: a kernel launched so starts while the one before it (its predecessor) still runs, does
+// what does not depend on the predecessor's writes, and waits here until the predecessor is done. Every such kernel waits
+// (in every block, before it ends) before it lets its own successor start, so when a kernel runs, everything before its
+// predecessor is complete. Launched otherwise both are no-ops. What the predecessor writes is never read through a const
+// __restrict__ pointer: such loads may be moved above the wait.
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Ground model (GroundModel, static_world.h:18-31): the values of ground_models() (static_world.cpp:85-114)
 struct GroundModel {
     float va, ms, mc, t2, vs, alpha, strength, soft_depth, fluid_drag, fluid_density;

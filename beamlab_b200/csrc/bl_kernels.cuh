@@ -358,9 +358,10 @@ struct ShockDev {
     const int2* inc;         // (shock | bit 31 where the node is the beam's b end, the other end)
     float* ssc;              // per shock: its scalar (kNoPush: none this substep)
 };
-__global__ void k_shocks(ShockDev S, int nshocks, const int2* __restrict__ ab, const float4* __restrict__ bst, uint32_t* __restrict__ bmeta,
-                         float* __restrict__ stress, const int* __restrict__ bbody, const float4* __restrict__ nd, Body* __restrict__ bodies) {
+__global__ void k_shocks(ShockDev S, int nshocks, const int2* __restrict__ ab, const float4* bst, uint32_t* __restrict__ bmeta,
+                         float* __restrict__ stress, const int* __restrict__ bbody, const float4* nd, Body* __restrict__ bodies) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
     if (q >= nshocks) return;
     S.ssc[q] = kNoPush;
     const bl_shock s = S.sh[q];
@@ -458,31 +459,6 @@ __global__ void k_shocks(ShockDev S, int nshocks, const int2* __restrict__ ab, c
     S.ssc[q] = slen * inv_len;
 }
 
-// Two beams a thread (j and j + blockDim.x of the block's pair of tiles): both beams' loads are issued before either
-// computes. Thread t < nbodies of the grid also resets body t's bounds accumulator for this substep's k_integrate.
-__global__ void __launch_bounds__(256) k_beams(const int2* __restrict__ ab, const float2* __restrict__ kd, float4* __restrict__ bst,
-                                               uint32_t* __restrict__ bmeta, const float4* __restrict__ bcold, float* __restrict__ stress,
-                                               const int* __restrict__ bbody, float* __restrict__ fsc, const float4* __restrict__ nd,
-                                               Body* __restrict__ bodies, int nbeams, int nbodies) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < nbodies) {
-        Body& B = bodies[t];
-        B.acc_mn[0] = B.acc_mn[1] = B.acc_mn[2] = 1e30f;
-        B.acc_mx[0] = B.acc_mx[1] = B.acc_mx[2] = -1e30f;
-    }
-    const int j0 = 2 * blockIdx.x * blockDim.x + threadIdx.x, j1 = j0 + blockDim.x;
-    const bool h0 = j0 < nbeams, h1 = j1 < nbeams;
-    const uint32_t m0 = h0 ? bmeta[j0] : kBeamAsleep, m1 = h1 ? bmeta[j1] : kBeamAsleep;
-    const int2 e0 = h0 ? ab[j0] : make_int2(0, 0), e1 = h1 ? ab[j1] : make_int2(0, 0);
-    const float4 s0 = h0 ? bst[j0] : make_float4(0, 0, 0, 0), s1 = h1 ? bst[j1] : make_float4(0, 0, 0, 0);
-    const float2 c0 = h0 ? kd[j0] : make_float2(0, 0), c1 = h1 ? kd[j1] : make_float2(0, 0);
-    float4 pa0 = make_float4(0, 0, 0, 0), va0 = pa0, pb0 = pa0, vb0 = pa0, pa1 = pa0, va1 = pa0, pb1 = pa0, vb1 = pa0;
-    if (h0) pa0 = nd[2 * e0.x], va0 = nd[2 * e0.x + 1], pb0 = nd[2 * e0.y], vb0 = nd[2 * e0.y + 1];
-    if (h1) pa1 = nd[2 * e1.x], va1 = nd[2 * e1.x + 1], pb1 = nd[2 * e1.y], vb1 = nd[2 * e1.y + 1];
-    if (h0) beam_step(j0, m0, s0, c0, pa0, va0, pb0, vb0, bst, bmeta, bcold, stress, bbody, fsc, bodies);
-    if (h1) beam_step(j1, m1, s1, c1, pa1, va1, pb1, vb1, bst, bmeta, bcold, stress, bbody, fsc, bodies);
-}
-
 // ------------------------------------------------------------------------------------------ bulk copies (TMA)
 // cp.async.bulk global -> shared completing on an mbarrier: the beam arrays stream into shared memory tile after tile
 // while the block computes earlier tiles. Every wait is bounded in time (the context's bulk_wait_s, 1 s by default): a
@@ -551,7 +527,7 @@ struct WheelDev {
 // controller's torque (every substep: the first short step's), the brake's stop torque against the average speed and
 // the last reaction, the share a tyre node, the tread's speed (summed in the builder's order), the average speed and
 // the reaction of the inertia, and the drive's reaction on the arm; the nodes' terms are k_force's.
-__device__ void wheel_step(int w, int lane, const float4* __restrict__ nd, const int4* __restrict__ info, const Body* __restrict__ bodies,
+__device__ void wheel_step(int w, int lane, const float4* nd, const int4* __restrict__ info, const Body* __restrict__ bodies,
                            const WheelDev& wh, float dt) {
     const int4 W = wh.wheel[w];
     if (W.w == 0 || bodies[info[W.x].w].sleeping) return; // (an asleep body's forces are not made)
@@ -608,13 +584,43 @@ __device__ void wheel_step(int w, int lane, const float4* __restrict__ nd, const
     wh.wcf[w] = cf4;
     wh.wst[w] = make_float4(sp, avg, T, lrt);
 }
-__global__ void __launch_bounds__(256) k_wheels(const float4* __restrict__ nd, const int4* __restrict__ info, const Body* __restrict__ bodies,
-                                                WheelDev wh, float dt) {
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (w < wh.nreal) wheel_step(w, threadIdx.x & 31, nd, info, bodies, wh, dt); // (w is the warp's: its lanes go together)
+// The beams by plain loads: two beams a thread (j and j + blockDim.x of the block's pair of tiles), both beams' loads
+// issued before either computes, the beams' own arrays before the wait for the predecessor (which writes the nodes). The
+// blocks past bblocks take the wheels, a warp a wheel. Thread t < nbodies of the grid also resets body t's bounds
+// accumulator for this substep's k_integrate. The kernel of all but the largest worlds (kPlainBeams): no copy into shared
+// memory to wait for first, and the wheels beside the beams instead of after a block's tiles.
+__global__ void __launch_bounds__(256) k_beams(const int2* __restrict__ ab, const float2* __restrict__ kd, float4* __restrict__ bst,
+                                               uint32_t* __restrict__ bmeta, const float4* __restrict__ bcold, float* __restrict__ stress,
+                                               const int* __restrict__ bbody, float* __restrict__ fsc, const float4* nd,
+                                               Body* __restrict__ bodies, int nbeams, int nbodies, int bblocks, const int4* __restrict__ info, WheelDev wh,
+                                               float dt) {
+    if ((int)blockIdx.x >= bblocks) {
+        pdl_wait();
+        const int w = (int)((blockIdx.x - bblocks) * blockDim.x + threadIdx.x) >> 5;
+        if (w < wh.nreal) wheel_step(w, threadIdx.x & 31, nd, info, bodies, wh, dt); // (w is the warp's: its lanes go together)
+        return;
+    }
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j0 = 2 * blockIdx.x * blockDim.x + threadIdx.x, j1 = j0 + blockDim.x;
+    const bool h0 = j0 < nbeams, h1 = j1 < nbeams;
+    const uint32_t m0 = h0 ? bmeta[j0] : kBeamAsleep, m1 = h1 ? bmeta[j1] : kBeamAsleep;
+    const int2 e0 = h0 ? ab[j0] : make_int2(0, 0), e1 = h1 ? ab[j1] : make_int2(0, 0);
+    const float4 s0 = h0 ? bst[j0] : make_float4(0, 0, 0, 0), s1 = h1 ? bst[j1] : make_float4(0, 0, 0, 0);
+    const float2 c0 = h0 ? kd[j0] : make_float2(0, 0), c1 = h1 ? kd[j1] : make_float2(0, 0);
+    pdl_wait();
+    if (t < nbodies) {
+        Body& B = bodies[t];
+        B.acc_mn[0] = B.acc_mn[1] = B.acc_mn[2] = 1e30f;
+        B.acc_mx[0] = B.acc_mx[1] = B.acc_mx[2] = -1e30f;
+    }
+    float4 pa0 = make_float4(0, 0, 0, 0), va0 = pa0, pb0 = pa0, vb0 = pa0, pa1 = pa0, va1 = pa0, pb1 = pa0, vb1 = pa0;
+    if (h0) pa0 = nd[2 * e0.x], va0 = nd[2 * e0.x + 1], pb0 = nd[2 * e0.y], vb0 = nd[2 * e0.y + 1];
+    if (h1) pa1 = nd[2 * e1.x], va1 = nd[2 * e1.x + 1], pb1 = nd[2 * e1.y], vb1 = nd[2 * e1.y + 1];
+    if (h0) beam_step(j0, m0, s0, c0, pa0, va0, pb0, vb0, bst, bmeta, bcold, stress, bbody, fsc, bodies);
+    if (h1) beam_step(j1, m1, s1, c1, pa1, va1, pb1, vb1, bst, bmeta, bcold, stress, bbody, fsc, bodies);
 }
 
-// k_beams with the beam arrays staged by bulk copies: a persistent block takes every gridDim.x-th tile of kBeamTile
+// The beams with their arrays staged by bulk copies, for large worlds: a persistent block takes every gridDim.x-th tile of kBeamTile
 // beams; kBeamStages tiles are in flight while it computes (one thread issues the copies: each tile's a/b ends, k/d,
 // state and meta words, 18 KB). The beam arrays are padded to whole tiles (pads asleep). Per beam the same
 // beam_step as k_beams. kEnds16: each beam's ends as two 16-bit offsets from its tile's base node (tbase) in one
@@ -643,7 +649,7 @@ template <bool kEnds16>
 __global__ void __launch_bounds__(kBeamThreads) k_beams_tma(const void* __restrict__ ab_, const int* __restrict__ tbase, const float2* __restrict__ kd,
                                                             float4* __restrict__ bst, uint32_t* __restrict__ bmeta, const float4* __restrict__ bcold,
                                                             float* __restrict__ stress, const int* __restrict__ bbody, float* __restrict__ fsc,
-                                                            const float4* __restrict__ nd, Body* __restrict__ bodies, int nbeams, int nbodies, int ntiles,
+                                                            const float4* nd, Body* __restrict__ bodies, int nbeams, int nbodies, int ntiles,
                                                             uint32_t* __restrict__ deverr, const int4* __restrict__ info, WheelDev wh, float dt,
                                                             unsigned long long wait_ns) {
     using Stage = BeamStage<kEnds16>;
@@ -653,6 +659,7 @@ __global__ void __launch_bounds__(kBeamThreads) k_beams_tma(const void* __restri
     Stage* stg = reinterpret_cast<Stage*>(smem);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kBeamStages * sizeof(Stage));
     const int tid = threadIdx.x;
+    pdl_wait();
     for (int t = blockIdx.x * kBeamThreads + tid; t < nbodies; t += gridDim.x * kBeamThreads) {
         Body& B = bodies[t]; // (this substep's bounds accumulator, for k_integrate)
         B.acc_mn[0] = B.acc_mn[1] = B.acc_mn[2] = 1e30f;
@@ -717,7 +724,7 @@ __global__ void __launch_bounds__(kBeamThreads) k_beams_tma(const void* __restri
         }
         issued = min(issued + 1, mine);
     }
-    // then the wheels (k_wheels' work, a warp a wheel: it reads the substep's starting state as the beams do, and only
+    // then the wheels (a warp a wheel: it reads the substep's starting state as the beams do, and only
     // k_force reads what it writes)
     for (int w = blockIdx.x * (kBeamThreads / 32) + (tid >> 5); w < wh.nreal; w += gridDim.x * (kBeamThreads / 32))
         wheel_step(w, tid & 31, nd, info, bodies, wh, dt);
@@ -781,21 +788,22 @@ __device__ __forceinline__ void accumulate_bounds(Body* __restrict__ bodies, int
 
 // A frame node's force: its triangles' corner forces and torques added in the reference's order (gather_forces,
 // frame_fem.cpp:2080-2105) after gravity and its beams; kept in nforce for the frame's implicit step.
+template <int kAtOnce>
 __device__ __forceinline__ void fem_gather(const NodeFem& nf, int i, v3 f) {
     const int fs = nf.fslot[i];
     if (fs >= 0) {
         const int k = nf.iperm[fs];
         v3 tq = V(0, 0, 0);
-        // (four entries' loads issued together, then added in order)
+        // (kAtOnce entries' loads issued together, then added in order)
         const int g1 = nf.gdiag_ptr[k + 1];
-        for (int g = nf.gdiag_ptr[k]; g < g1; g += 4) {
-            int2 e[4];
-            bool on[4];
-            float4 ff[4], tt[4];
+        for (int g = nf.gdiag_ptr[k]; g < g1; g += kAtOnce) {
+            int2 e[kAtOnce];
+            bool on[kAtOnce];
+            float4 ff[kAtOnce], tt[kAtOnce];
 #pragma unroll
-            for (int u = 0; u < 4; u++) e[u] = g + u < g1 ? nf.gdiag[g + u] : make_int2(0, -1);
+            for (int u = 0; u < kAtOnce; u++) e[u] = g + u < g1 ? nf.gdiag[g + u] : make_int2(0, -1);
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < kAtOnce; u++) {
                 on[u] = false;
                 if (e[u].y < 0) continue;
                 if (e[u].x < 0) { // (a member's end a (+fa, ta) or b (-fa, tb): gather_forces, frame_fem.cpp:2092-2096)
@@ -806,7 +814,7 @@ __device__ __forceinline__ void fem_gather(const NodeFem& nf, int i, v3 f) {
                 }
             }
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < kAtOnce; u++) {
                 if (!on[u]) continue;
                 if (e[u].x < 0 && e[u].y != 0) f = V(f.x - ff[u].x, f.y - ff[u].y, f.z - ff[u].z);
                 else f = V(f.x + ff[u].x, f.y + ff[u].y, f.z + ff[u].z);
@@ -894,15 +902,20 @@ __global__ void k_drag_parts(Body* __restrict__ bodies, int nbodies, const float
 // padding), bit 15 set where this node is the beam's b end, the other end's index less this node's plus 32768 (bits
 // 16-31) - half the bytes of the (beam | b-end bit, other end) pairs, for rigs whose warps' beams and neighbours lie
 // close enough (bl_world.cu checks every warp)
-template <bool kPacked>
-__global__ void __launch_bounds__(256, 6) k_force(const float4* __restrict__ nd, const int4* __restrict__ info, const int* __restrict__ ell_ptr,
-                                               const void* __restrict__ ell_, const int* __restrict__ ell_base, const float* __restrict__ fsc,
+// kWide: a warp a node, a lane an incidence - the gathers of a node's beams all at once, their forces then added in their
+// order by broadcasts (the same sums) - for worlds whose nodes all fit on the GPU that way: a node of 26 beams waits for
+// one gather instead of seven (B200, a frame of 33 substeps of the 400-node truss car: 333 us a thread a node, 265 so).
+// The gathers of the nodes come before the wait for the beams' kernel, whose scalars are all that is new.
+template <bool kPacked, bool kWide>
+__global__ void __launch_bounds__(256, kWide ? 4 : 6) k_force(const float4* __restrict__ nd, const int4* __restrict__ info, const int* __restrict__ ell_ptr,
+                                               const void* __restrict__ ell_, const int* __restrict__ ell_base, const float* fsc,
                                                Body* __restrict__ bodies, float gx, float gy, float gz, int nnodes, int first, NodeFem nf,
                                                float4* __restrict__ fnode, DragDev dg, WheelDev wh, ShockDev sk) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g = blockIdx.x * blockDim.x + threadIdx.x, i = kWide ? g >> 5 : g;
     int body = -1;
     float v2 = 0.0f;
     bool live = false;
+    if (i >= nnodes) pdl_wait();
     if (i < nnodes) {
         // (the node's own loads and its warp's incidence range issued before its body's state arrives)
         const int4 inf = info[i];
@@ -912,6 +925,26 @@ __global__ void __launch_bounds__(256, 6) k_force(const float4* __restrict__ nd,
         const int base = kPacked ? ell_base[w] : 0;
         body = inf.w;
         const Body& B = bodies[body];
+        // entry q of the node in its warp's incidences
+        auto entry = [&](int q, int& beam, int& other, bool& pad, bool& bend) {
+            if (kPacked) {
+                const uint32_t x = static_cast<const uint32_t*>(ell_)[q0 + 32 * q + lane];
+                pad = (x & 0x7fffu) == 0x7fffu;
+                beam = base + (int)(x & 0x7fffu), bend = (x & 0x8000u) != 0, other = i + (int)(x >> 16) - 32768;
+            } else {
+                const int2 e = static_cast<const int2*>(ell_)[q0 + 32 * q + lane];
+                pad = e.y == i; // (padding: (0, the node itself))
+                beam = e.x & 0x7fffffff, bend = e.x < 0, other = e.y;
+            }
+        };
+        int beam1 = 0, other1 = i; // (kWide: this lane's first incidence and its other end)
+        bool pad1 = true, bend1 = false;
+        float4 Po1 = make_float4(0, 0, 0, 0);
+        if (kWide) {
+            if ((int)(g & 31) < width) entry(g & 31, beam1, other1, pad1, bend1);
+            if (!pad1) Po1 = nd[2 * other1];
+        }
+        pdl_wait();
         if (!B.sleeping) {
             const float m = Vv.w;
             v3 f;
@@ -944,23 +977,31 @@ __global__ void __launch_bounds__(256, 6) k_force(const float4* __restrict__ nd,
             };
             // the warp's incidences, interleaved: entry q of lane l at ell[ell_ptr[w] + 32 q + l] (a warp's load reads 32
             // neighbours), each node's in beam order, padded to the warp's widest node (a multiple of 4)
-            for (int q = 0; q < width; q += 4) {
+            if (kWide) {
+                for (int q = 0; q < width; q += 32) {
+                    if (q > 0) {
+                        pad1 = true;
+                        if (q + (int)(g & 31) < width) entry(q + (g & 31), beam1, other1, pad1, bend1);
+                        if (!pad1) Po1 = nd[2 * other1];
+                    }
+                    const float sc = pad1 ? kNoPush : fsc[beam1];
+                    const bool on = !pad1 && __float_as_uint(sc) != __float_as_uint(kNoPush);
+                    // (the force on the node: f + dis sc at the beam's a end, f - dis sc at its b end)
+                    v3 t = bend1 ? V(Po1.x - P.x, Po1.y - P.y, Po1.z - P.z) * sc : V(P.x - Po1.x, P.y - Po1.y, P.z - Po1.z) * sc;
+                    if (bend1) t = V(-t.x, -t.y, -t.z);
+                    for (unsigned m = __ballot_sync(0xffffffffu, on); m; m &= m - 1) {
+                        const int l = __ffs(m) - 1;
+                        f = V(f.x + __shfl_sync(0xffffffffu, t.x, l), f.y + __shfl_sync(0xffffffffu, t.y, l), f.z + __shfl_sync(0xffffffffu, t.z, l));
+                    }
+                }
+            }
+            for (int q = 0; !kWide && q < width; q += 4) {
                 int beam[4], other[4];
                 bool pad[4], bend[4];
                 float sc[4];
                 float4 Po[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    if (kPacked) {
-                        const uint32_t x = static_cast<const uint32_t*>(ell_)[q0 + 32 * (q + u) + lane];
-                        pad[u] = (x & 0x7fffu) == 0x7fffu;
-                        beam[u] = base + (int)(x & 0x7fffu), bend[u] = (x & 0x8000u) != 0, other[u] = i + (int)(x >> 16) - 32768;
-                    } else {
-                        const int2 e = static_cast<const int2*>(ell_)[q0 + 32 * (q + u) + lane];
-                        pad[u] = e.y == i; // (padding: (0, the node itself))
-                        beam[u] = e.x & 0x7fffffff, bend[u] = e.x < 0, other[u] = e.y;
-                    }
-                }
+                for (int u = 0; u < 4; u++) entry(q + u, beam[u], other[u], pad[u], bend[u]);
 #pragma unroll
                 for (int u = 0; u < 4; u++) sc[u] = pad[u] ? kNoPush : fsc[beam[u]], Po[u] = nd[2 * other[u]];
 #pragma unroll
@@ -995,9 +1036,9 @@ __global__ void __launch_bounds__(256, 6) k_force(const float4* __restrict__ nd,
             if (B.is_fem) {
                 live = true; // (its bounds and speeds after the frame's step: k_fem_integrate; the start's top speed here)
                 if (first) v2 = Vv.x * Vv.x + Vv.y * Vv.y + Vv.z * Vv.z;
-                fem_gather(nf, i, f);
+                fem_gather<kWide ? 4 : 1>(nf, i, f);
             } else {
-                fnode[i] = make_float4(f.x, f.y, f.z, 0.0f);
+                if (!kWide || (g & 31) == 0) fnode[i] = make_float4(f.x, f.y, f.z, 0.0f);
             }
         }
     }
@@ -1096,22 +1137,34 @@ __device__ __forceinline__ bool static_query(const Statics& st, const Body& B, v
 // starts from the velocities before it, world.cpp:3217-3222). Frame bodies' nodes are integrated after their solve.
 // A tyre node (NF_TYRE) in contact leaves its contact in wh.tcon / wh.tfric and its force in fnode to its wheel's
 // patch (k_tyres), which takes tyre_contact instead of primitive_collision and integrates it.
-__global__ void __launch_bounds__(256) k_integrate(float4* __restrict__ nd, const int4* __restrict__ info, Body* __restrict__ bodies, Statics st,
-                                                   float dt, int nnodes, int first, float4* __restrict__ fnode, WheelDev wh) {
+__global__ void __launch_bounds__(256) k_integrate(float4* nd, const int4* __restrict__ info, Body* __restrict__ bodies, Statics st,
+                                                   float dt, int nnodes, int first, const float4* fnode, WheelDev wh) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     int body = -1;
     v3 p = V(1e30f, 1e30f, 1e30f), pmx = V(-1e30f, -1e30f, -1e30f);
     float v2 = 0.0f, v2start = 0.0f;
     int contact = 0;
     bool live = false;
+    // (the static query needs no force: made before the wait for the forces' kernel)
+    int4 inf = make_int4(0, 0, 0, 0);
+    float4 P = make_float4(0, 0, 0, 0), Vv = P;
+    Contact c;
+    bool hit = false;
     if (i < nnodes) {
         // (the node's own loads issued before its body's state arrives)
-        const int4 inf = info[i];
-        const float4 P = nd[2 * i], Vv = nd[2 * i + 1], f4 = fnode[i];
+        inf = info[i];
+        P = nd[2 * i], Vv = nd[2 * i + 1];
         body = inf.w;
         const Body& B = bodies[body];
-        if (!B.sleeping && !B.is_fem) {
-            live = true;
+        live = !B.sleeping && !B.is_fem;
+        if (live && ((uint32_t)inf.x & NF_GROUND) && !(P.w <= 0) && !(P.y < st.kill_y))
+            hit = static_query(st, B, V(P.x, P.y, P.z), __int_as_float(inf.z), c);
+    }
+    pdl_wait();
+    if (i < nnodes) {
+        const float4 f4 = fnode[i];
+        const Body& B = bodies[body];
+        if (live) {
             const float m = Vv.w;
             v3 f = V(f4.x, f4.y, f4.z);
             if (first) v2start = Vv.x * Vv.x + Vv.y * Vv.y + Vv.z * Vv.z;
@@ -1125,8 +1178,7 @@ __global__ void __launch_bounds__(256) k_integrate(float4* __restrict__ nd, cons
                     inv_mass = 0;
                 } else {
                     {
-                        Contact c;
-                        if (static_query(st, B, pos, __int_as_float(inf.z), c)) {
+                        if (hit) {
                             contact = 1;
                             const GroundModel& gm = c_ground[c.surface < kSurfCount ? c.surface : 0];
                             const float fc = __int_as_float(inf.y) * B.fric;
@@ -1168,9 +1220,10 @@ __global__ void __launch_bounds__(256) k_integrate(float4* __restrict__ nd, cons
 // force; the touching ones' needs and caps summed in ascending node order (every lane adds the same broadcast values
 // in the same order); each touching node sticks (its need) if the patch as a whole can hold, else slides; then
 // SoftBody::integrate_nodes for them, the warp's bounds, top speed and contacts into the body's accumulators.
-__global__ void __launch_bounds__(256) k_tyres(float4* __restrict__ nd, const int4* __restrict__ info, Body* __restrict__ bodies, float dt,
-                                               int nwheels, int first, const float4* __restrict__ fnode, WheelDev wh) {
+__global__ void __launch_bounds__(256) k_tyres(float4* nd, const int4* __restrict__ info, Body* __restrict__ bodies, float dt,
+                                               int nwheels, int first, const float4* fnode, WheelDev wh) {
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    pdl_wait();
     if (w >= nwheels) return; // (w is the warp's: its lanes leave together)
     const int4 W = wh.wheel[w];
     if (W.w == 0) return;

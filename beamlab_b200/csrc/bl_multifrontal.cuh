@@ -103,23 +103,46 @@ __device__ __forceinline__ void mf_mma(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
 }
 
-// acc += A B^T over one chunk (16 of the summed columns): a warp's 24 x 24 quarter of the tile, 3 x 3 blocks of 8 x 8
+// A warp's 3 x 3 blocks of 8 x 8 of a tile: block rows 0, 3, 4 (wr = 0) or 1, 2, 5, block columns likewise by wc - so that the
+// four warps share the lower triangle of a diagonal tile (6, 4, 5, 6 blocks) and the columns of a triangular factor
+// evenly (a contiguous quarter each: 9 and 3 blocks, 36 and 6 of a column's 8-wide terms).
+__device__ __forceinline__ int mf_own(int w, int x) { return w == 0 ? (x == 0 ? 0 : x + 2) : (x == 2 ? 5 : x + 1); }
+// acc += A B^T over one chunk (16 of the summed columns). lower: only blocks on and below the diagonal.
+template <bool kLower>
 __device__ __forceinline__ void mf_mma_chunk(double (&acc)[3][3][2], const double* A, const double* B, int wr, int wc, int lane) {
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         double a[3], b[3];
 #pragma unroll
-        for (int x = 0; x < 3; x++) a[x] = A[(3 * wr + x) * 128 + k * 32 + lane], b[x] = B[(3 * wc + x) * 128 + k * 32 + lane];
+        for (int x = 0; x < 3; x++) a[x] = A[mf_own(wr, x) * 128 + k * 32 + lane], b[x] = B[mf_own(wc, x) * 128 + k * 32 + lane];
 #pragma unroll
         for (int x = 0; x < 3; x++)
 #pragma unroll
-            for (int y = 0; y < 3; y++) mf_mma(acc[x][y], a[x], b[y]);
+            for (int y = 0; y < 3; y++)
+                if (!kLower || mf_own(wr, x) >= mf_own(wc, y)) mf_mma(acc[x][y], a[x], b[y]);
+    }
+}
+// acc = A B^T of two tiles, B lower triangular
+__device__ __forceinline__ void mf_mma_lower(double (&acc)[3][3][2], const double* A, const double* B, int wr, int wc, int lane) {
+#pragma unroll 2
+    for (int k = 0; k < 12; k++) {
+        const int at = (k >> 2) * kMfChunk + (k & 3) * 32 + lane;
+        double a[3];
+#pragma unroll
+        for (int x = 0; x < 3; x++) a[x] = A[at + mf_own(wr, x) * 128];
+#pragma unroll
+        for (int y = 0; y < 3; y++) {
+            if (mf_own(wc, y) < k >> 1) continue;
+            const double b = B[at + mf_own(wc, y) * 128];
+#pragma unroll
+            for (int x = 0; x < 3; x++) mf_mma(acc[x][y], a[x], b);
+        }
     }
 }
 // where this lane's pair of accumulator (x, y) lies in a tile
 __device__ __forceinline__ int mf_acc_at(int x, int y, int wr, int wc, int lane) {
-    const int c = 8 * (3 * wc + y) + 2 * (lane & 3);
-    return (c >> 4) * kMfChunk + (3 * wr + x) * 128 + ((c >> 2) & 3) * 32 + (lane >> 2) * 4 + (c & 3);
+    const int c = 8 * mf_own(wc, y) + 2 * (lane & 3);
+    return (c >> 4) * kMfChunk + mf_own(wr, x) * 128 + ((c >> 2) & 3) * 32 + (lane >> 2) * 4 + (c & 3);
 }
 
 // ---- the diagonal tile's factor and its inverse, in 8 x 8 blocks (64 contiguous doubles of a tile)
@@ -402,7 +425,8 @@ __device__ __forceinline__ bool mf_tile(const FemDev& F, const MfDev& M, const M
             __syncthreads();
             issue(c + kMfStages - 1);
             const double* A = ring + 2 * (c % kMfStages) * kMfChunk;
-            mf_mma_chunk(acc, A, same ? A : A + kMfChunk, wr, wc, lane);
+            if (same) mf_mma_chunk<true>(acc, A, A, wr, wc, lane);
+            else mf_mma_chunk<false>(acc, A, A + kMfChunk, wr, wc, lane);
         }
         mf_cp_wait<0>();
         __syncthreads();
@@ -460,7 +484,7 @@ __device__ __forceinline__ bool mf_tile(const FemDev& F, const MfDev& M, const M
         mf_cp_commit();
         mf_cp_wait<0>();
         __syncthreads();
-        for (int kc = 0; kc < 3; kc++) mf_mma_chunk(acc, C + kc * kMfChunk, ring + kc * kMfChunk, wr, wc, lane);
+        mf_mma_lower(acc, C, ring, wr, wc, lane);
 #pragma unroll
         for (int x = 0; x < 3; x++)
 #pragma unroll

@@ -1345,7 +1345,7 @@ static int ensure_committed(bl_gpu_ctx* c) {
 static bool rebuild_at(const bl_gpu_ctx* c, int k) { return k % c->interval == 0; } // (s == 0 || s >= next_rebuild)
 
 static int64_t frame_launches(const bl_gpu_ctx* c, int n) {
-    int64_t per = 3 + (c->any_drag ? 1 : 0) + (c->NW > 0 ? 1 : 0) + (c->NWR > 0 && c->beam_grid == 0 ? 1 : 0) + (c->NSH > 0 ? 1 : 0);
+    int64_t per = 3 + (c->any_drag ? 1 : 0) + (c->NW > 0 ? 1 : 0) + (c->NSH > 0 ? 1 : 0);
     if (c->NF > 0) {
         if (c->fem_only) per -= 2; // (no beams, no other nodes)
         per += c->fem_launches + (c->cfg.fem_check_residual ? 2 : 0) + (c->fem_ground ? 1 : 0);
@@ -1433,6 +1433,27 @@ static void launch_pcg(bl_gpu_ctx* c, cudaStream_t s, cudaGraphConditionalHandle
     cudaLaunchKernelEx(&lc, k_fem_pcg, c->fd, P);
 }
 
+// Beams by plain loads up to this many, by bulk copies above; forces a warp a node up to this many nodes. Measured on B200, a
+// frame of 33 substeps in us, each rule alone against its alternative: the 400-node truss car 261 (bulk copies 368 with
+// programmatic launches, 458 without; a thread a node 333), one vehicle of 5,072 nodes 816 (976; 884), two of
+// 8,536 nodes 885 a thread a node, 935 a warp; 16 vehicles with 0.55 M beams 1150 by plain loads, 1207 by bulk copies, 64 with
+// 2.2 M 2498 and 2528, 256 with 8.9 M even. Programmatic launches beside the bulk copies' persistent blocks, which hold
+// the shared memory the running kernel's blocks need: 6 to 8 % slower from 32 vehicles on, so those go without.
+constexpr int kPlainBeams = 4000000, kWideNodes = 6000;
+
+// kernel<<<grid, block, smem, s>>>(args...); early: it may start while the kernel before it on the stream still runs
+// (pdl_wait, bl_device.cuh)
+template <class... Params, class... Args>
+static void launch_after(cudaStream_t s, bool early, void (*kernel)(Params...), int grid, int block, size_t smem, Args... args) {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(grid), lc.blockDim = dim3(block), lc.dynamicSmemBytes = smem, lc.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at, lc.numAttrs = early ? 1 : 0;
+    cudaLaunchKernelEx(&lc, kernel, Params(args)...);
+}
+
 static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev = nullptr) {
     int q = 0;
     auto mark = [&]() {
@@ -1441,8 +1462,12 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
     mark();
     const float dt = c->cfg.dt;
     const float frame_time = (float)n * dt;
-    const int tb = 256;
-    const int gb = std::max((c->M + 2 * tb - 1) / (2 * tb), (c->B + tb - 1) / tb), gbody = (c->B + tb - 1) / tb;
+    const int tb = 256, gbody = (c->B + tb - 1) / tb;
+    // (bulk_wait_s 0 keeps the copies whose waits it makes run out)
+    const bool bulk = c->beam_grid > 0 && (c->M > kPlainBeams || c->wait_ns == 0), wide = c->N <= kWideNodes;
+    const int bt = 64, gb = std::max(1, std::max((c->M + 2 * bt - 1) / (2 * bt), (c->B + bt - 1) / bt));
+    // the substep's kernels as programmatic dependent launches (not between timing events)
+    auto go = [&](auto kernel, int grid, int block, size_t smem, auto... args) { launch_after(s, ev == nullptr && !bulk, kernel, grid, block, smem, args...); };
     // (the node kernels' block sizes: bl_gpu_config.force_block / integrate_block, 256 unless tuned)
     const int fb = c->cfg.force_block > 0 ? c->cfg.force_block : 256, ib = c->cfg.integrate_block > 0 ? c->cfg.integrate_block : 256;
     const int gfn = (c->N + fb - 1) / fb, gin = (c->N + ib - 1) / ib;
@@ -1481,43 +1506,42 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
             k_fem_begin<<<(c->NF + tb - 1) / tb, tb, 0, s>>>(F, c->nd.p);
         if (c->fem_only) {
             // (no beams; the bounds accumulators are reset by the assembly)
-        } else if (c->beam_grid > 0) {
+        } else if (bulk) {
             // (the wheels' step in the same launch, after each block's tiles)
             if (c->ends16)
-                k_beams_tma<true><<<c->beam_grid, kBeamThreads, beam_smem<true>(), s>>>(c->ab16.p, c->tbase.p, c->kd.p, c->bst.p, c->bmeta.p, c->bcold.p,
-                                                                                       c->stress.p, c->bbody.p, c->fsc.p, c->nd.p, c->dbodies.p, c->M, c->B,
-                                                                                       c->beam_tiles, c->deverr.p, c->info.p, wh, dt, c->wait_ns);
+                go(k_beams_tma<true>, c->beam_grid, kBeamThreads, beam_smem<true>(), c->ab16.p, c->tbase.p, c->kd.p, c->bst.p, c->bmeta.p, c->bcold.p,
+                   c->stress.p, c->bbody.p, c->fsc.p, c->nd.p, c->dbodies.p, c->M, c->B, c->beam_tiles, c->deverr.p, c->info.p, wh, dt, c->wait_ns);
             else
-                k_beams_tma<false><<<c->beam_grid, kBeamThreads, beam_smem<false>(), s>>>(c->ab.p, nullptr, c->kd.p, c->bst.p, c->bmeta.p, c->bcold.p,
-                                                                                         c->stress.p, c->bbody.p, c->fsc.p, c->nd.p, c->dbodies.p, c->M, c->B,
-                                                                                         c->beam_tiles, c->deverr.p, c->info.p, wh, dt, c->wait_ns);
+                go(k_beams_tma<false>, c->beam_grid, kBeamThreads, beam_smem<false>(), c->ab.p, nullptr, c->kd.p, c->bst.p, c->bmeta.p, c->bcold.p,
+                   c->stress.p, c->bbody.p, c->fsc.p, c->nd.p, c->dbodies.p, c->M, c->B, c->beam_tiles, c->deverr.p, c->info.p, wh, dt, c->wait_ns);
         } else {
-            k_beams<<<std::max(gb, 1), tb, 0, s>>>(c->ab.p, c->kd.p, c->bst.p, c->bmeta.p, c->bcold.p, c->stress.p, c->bbody.p, c->fsc.p, c->nd.p,
-                                                   c->dbodies.p, c->M, c->B);
-            if (c->NWR > 0) k_wheels<<<(c->NWR + 7) / 8, 256, 0, s>>>(c->nd.p, c->info.p, c->dbodies.p, wh, dt);
+            go(k_beams, gb + (c->NWR * 32 + bt - 1) / bt, bt, 0, c->ab.p, c->kd.p, c->bst.p, c->bmeta.p, c->bcold.p, c->stress.p, c->bbody.p, c->fsc.p, c->nd.p,
+               c->dbodies.p, c->M, c->B, gb, c->info.p, wh, dt);
         }
         if (c->NSH > 0)
-            k_shocks<<<(c->NSH + 127) / 128, 128, 0, s>>>(sk, c->NSH, c->ab.p, c->bst.p, c->bmeta.p, c->stress.p, c->bbody.p, c->nd.p, c->dbodies.p);
+            go(k_shocks, (c->NSH + 127) / 128, 128, 0, sk, c->NSH, c->ab.p, c->bst.p, c->bmeta.p, c->stress.p, c->bbody.p, c->nd.p, c->dbodies.p);
         if (c->NT > 0 && c->any_plastic) k_tri_eval<true><<<(c->NT + 127) / 128, 128, 0, s>>>(F, c->nd.p);
         else if (c->NT > 0) k_tri_eval<false><<<(c->NT + 127) / 128, 128, 0, s>>>(F, c->nd.p);
         if (c->NM > 0 && c->any_plastic_members) k_member_eval<true><<<(c->NM + 3) / 4, 128, 0, s>>>(F, c->nd.p);
         else if (c->NM > 0) k_member_eval<false><<<(c->NM + 3) / 4, 128, 0, s>>>(F, c->nd.p);
         mark();
-        if (c->packed_inc)
-            k_force<true><<<std::max(gfn, 1), fb, 0, s>>>(c->nd.p, c->info.p, c->ell_ptr.p, c->inc4.p, c->ell_base.p, c->fsc.p, c->dbodies.p,
-                                                         c->cfg.gravity[0], c->cfg.gravity[1], c->cfg.gravity[2], c->N, k == 0 ? 1 : 0, nfm, c->nodef.p, dg, wh, sk);
-        else
-            k_force<false><<<std::max(gfn, 1), fb, 0, s>>>(c->nd.p, c->info.p, c->ell_ptr.p, c->inc2.p, nullptr, c->fsc.p, c->dbodies.p,
-                                                          c->cfg.gravity[0], c->cfg.gravity[1], c->cfg.gravity[2], c->N, k == 0 ? 1 : 0, nfm, c->nodef.p, dg, wh, sk);
+        auto force = [&](auto kernel, const void* ell, const int* base, int grid, int block) {
+            go(kernel, grid, block, 0, c->nd.p, c->info.p, c->ell_ptr.p, ell, base, c->fsc.p, c->dbodies.p, c->cfg.gravity[0], c->cfg.gravity[1],
+               c->cfg.gravity[2], c->N, k == 0 ? 1 : 0, nfm, c->nodef.p, dg, wh, sk);
+        };
+        if (wide && c->packed_inc) force(k_force<true, true>, c->inc4.p, c->ell_base.p, (c->N + 7) / 8, 256);
+        else if (wide) force(k_force<false, true>, c->inc2.p, nullptr, (c->N + 7) / 8, 256);
+        else if (c->packed_inc) force(k_force<true, false>, c->inc4.p, c->ell_base.p, std::max(gfn, 1), fb);
+        else force(k_force<false, false>, c->inc2.p, nullptr, std::max(gfn, 1), fb);
         mark();
         if (c->contacts_on) {
             // contacts between bodies on the forces so far (World::collide_pairs, before the static contacts)
-            k_detect<<<148 * 4, 256, 0, s>>>(c->nd.p, c->info.p, c->dbodies.p, CT);
-            k_collide<<<c->B, kCollideThreads, kCollideSmem, s>>>(c->nd.p, c->info.p, c->dbodies.p, c->B, CT, c->nodef.p);
+            go(k_detect, 148 * 4, 256, 0, c->nd.p, c->info.p, c->dbodies.p, CT);
+            go(k_collide, c->B, kCollideThreads, kCollideSmem, c->nd.p, c->info.p, c->dbodies.p, c->B, CT, c->nodef.p);
         }
         mark();
-        if (!c->fem_only) k_integrate<<<std::max(gin, 1), ib, 0, s>>>(c->nd.p, c->info.p, c->dbodies.p, c->st, dt, c->N, k == 0 ? 1 : 0, c->nodef.p, wh);
-        if (c->NW > 0) k_tyres<<<(c->NW + 7) / 8, 256, 0, s>>>(c->nd.p, c->info.p, c->dbodies.p, dt, c->NW, k == 0 ? 1 : 0, c->nodef.p, wh);
+        if (!c->fem_only) go(k_integrate, std::max(gin, 1), ib, 0, c->nd.p, c->info.p, c->dbodies.p, c->st, dt, c->N, k == 0 ? 1 : 0, c->nodef.p, wh);
+        if (c->NW > 0) go(k_tyres, (c->NW + 7) / 8, 256, 0, c->nd.p, c->info.p, c->dbodies.p, dt, c->NW, k == 0 ? 1 : 0, c->nodef.p, wh);
         mark();
         if (c->NF > 0) {
             // the frames' implicit step: assembly, factorization and substitutions level by level, velocities, integration
