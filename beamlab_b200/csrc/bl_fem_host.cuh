@@ -603,13 +603,6 @@ static void fem_symbolic(const std::vector<int>& order, const std::vector<int>& 
     }
 }
 
-// The pattern's block updates, whether or not their list is built: sum over the columns of d (d + 1) / 2
-static int64_t fem_update_count(const FemModel& M) {
-    int64_t u = 0;
-    for (size_t k = 0; k + 1 < M.col_ptr.size(); k++) u += (int64_t)(M.col_ptr[k + 1] - M.col_ptr[k]) * (M.col_ptr[k + 1] - M.col_ptr[k] + 1) / 2;
-    return u;
-}
-
 // The update list of the column-by-column factorization: each source column k: the rows of column c = row[i]
 // scattered into a position table once, then every later row j of column k looked up in it
 static void fem_update_list(FemModel& M) {

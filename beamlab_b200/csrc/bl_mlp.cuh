@@ -32,8 +32,6 @@ constexpr int kIn = 36, kHid = 64, kOut = 12;
 constexpr int kOffW1 = 0, kOffB1 = kOffW1 + kHid * kIn, kOffW2 = kOffB1 + kHid, kOffB2 = kOffW2 + kHid * kHid, kOffW3 = kOffB2 + kHid;
 constexpr int kOffB3 = kOffW3 + kHid * kHid, kOffW4 = kOffB3 + kHid, kOffB4 = kOffW4 + kOut * kHid, kParams = kOffB4 + kOut;
 constexpr float kS0 = 1e-3f;
-constexpr int kLanes = 32;   // samples a block (one warp)
-constexpr int kLd = 33;      // shared-memory row stride (a feature's 32 samples, padded against bank conflicts)
 
 struct MlpDev {
     const __nv_bfloat16* wb; // the parameters in BF16 (what the forward reads)
@@ -56,108 +54,102 @@ struct MlpDev {
 __device__ __forceinline__ float slog(float x) { return x < 0 ? -log1pf(-x / kS0) : log1pf(x / kS0); }
 __device__ __forceinline__ float islog(float y) { return y < 0 ? -kS0 * expm1f(-y) : kS0 * expm1f(y); }
 
-// ------------------------------------------------------------------------------------------ the network (one sample a lane)
-constexpr int kKIn = 48;         // the first layer's inputs padded to whole k-steps of 16 (36 features + 12 zeros)
-constexpr int kPadIn = 64 + 8;   // the staged activations' row stride in BF16 (144 B: rows fall in distinct banks)
-constexpr int kOutPad = 16;      // the last layer's outputs padded to two n-tiles of 8
+// ------------------------------------------------------------------------------------------ the network
+// A block of 8 warps takes tiles of 32 samples; a layer is 32 samples x 64 outputs as mma.sync m16n8k16 tiles (BF16
+// operands, FP32 accumulation), a warp one column of 8 outputs: A = the layer's input, 32 rows of BF16 in shared memory
+// (row stride kPadIn: rows fall in distinct banks), B = the weights, kept in the warp's registers over all its tiles. The
+// inputs are rounded to BF16 as they are staged (the activations the next layer reads are the BF16 values); the
+// accumulators, bias and ReLU stay FP32.
+constexpr int kTile = 32;        // samples a tile
+constexpr int kMlpThreads = 256;
+constexpr int kPadIn = 64 + 8;   // a BF16 row
+constexpr int kPadF = 64 + 4;    // an FP32 row
 
-struct MlpTc {
-    __nv_bfloat16 act[kLanes * kPadIn];   // the current layer's input
-    __nv_bfloat16 w[kHid * kPadIn];       // the current layer's weights, nout x nin
-};
-
-// activations in shared memory, [feature][kLd]: lane s holds its sample in column s; the backward's deltas share
-// their storage with the forward's tensor-core staging (live one after the other)
-struct MlpSmem {
-    float a0[kIn * kLd];
-    float a1[kHid * kLd];
-    float a2[kHid * kLd];
-    float a3[kHid * kLd];
-    float y[kOut * kLd];
-    union {
-        struct {
-            float d0[kHid * kLd];
-            float d1[kHid * kLd];
-        };
-        MlpTc tc;
-    };
-};
-
-// ------------------------------------------------------------------------------------------ the layers on the tensor cores
-// One warp runs a layer's 32 samples x nout outputs as mma.sync m16n8k16 tiles (BF16 operands, FP32 accumulation):
-// A = the layer's input, 32 samples x nin, BF16, row-major in shared memory (row stride kPadIn); B = the weights,
-// nout x nin row-major (the "col" operand as it is), BF16 in shared memory. The inputs are rounded to BF16 as they are
-// staged (the activations the next layer reads are the BF16 values); the accumulators, bias and ReLU stay FP32.
-__device__ __forceinline__ void mma_bf16(float c[4], const uint32_t a[4], const uint32_t b[2]) {
+__device__ __forceinline__ void mma_bf16(float c[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ uint32_t lds32(const __nv_bfloat16* p) { return *reinterpret_cast<const uint32_t*>(p); }
 
-// out[o * kLd + s] = (relu)(b_o + sum_i W[o][i] act[s][i]) for the 32 samples; the layer's weights (nout x nin from
-// global, zero rows past nout) staged first. nin: a multiple of 16; nout_t: n-tiles of 8.
-__device__ __forceinline__ void dense_tc(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ b, int nin, int nin_real, int nout,
-                                         int nout_t, MlpTc& T, float* out, bool relu) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    for (int e = lane; e < nout_t * 8 * nin; e += 32) {
-        const int o = e / nin, i = e % nin;
-        T.w[o * kPadIn + i] = (o < nout && i < nin_real) ? W[(size_t)o * nin_real + i] : __float2bfloat16(0.0f);
-    }
-    __syncwarp();
-    for (int mt = 0; mt < 2; mt++) {
-        for (int nt = 0; nt < nout_t; nt++) {
-            float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            for (int k0 = 0; k0 < nin; k0 += 16) {
-                const __nv_bfloat16* a_lo = T.act + (16 * mt + g) * kPadIn + k0 + 2 * t;
-                const __nv_bfloat16* a_hi = a_lo + 8 * kPadIn;
-                const uint32_t a[4] = {lds32(a_lo), lds32(a_hi), lds32(a_lo + 8), lds32(a_hi + 8)};
-                const __nv_bfloat16* wp = T.w + (8 * nt + g) * kPadIn + k0 + 2 * t;
-                const uint32_t bb[2] = {lds32(wp), lds32(wp + 8)};
-                mma_bf16(c, a, bb);
-            }
-            // c0, c1: sample 16 mt + g, outputs 8 nt + 2 t, + 1; c2, c3: sample + 8
-            for (int q = 0; q < 4; q++) {
-                const int smp = 16 * mt + g + (q >= 2 ? 8 : 0), o = 8 * nt + 2 * t + (q & 1);
-                if (o < nout) {
-                    const float v = c[q] + __bfloat162float(b[o]);
-                    out[o * kLd + smp] = relu ? fmaxf(v, 0.0f) : v;
-                }
-            }
-        }
-    }
-    __syncwarp();
-}
+// a tile's activations: act - the current layer's input and the next one's, BF16; a - each layer's input as FP32 of the
+// BF16 values (what the weight gradients multiply); y - the outputs
+struct MlpTile {
+    __nv_bfloat16 act[2][kTile * kPadIn];
+    float a[4][kTile * kPadF];
+    float y[kTile * 16];
+};
 
-// the next layer's input: `in` ([feature][kLd], FP32) as BF16 rows, padded with zeros to nin_pad
-__device__ __forceinline__ void stage_act(const float* in, int nin, int nin_pad, MlpTc& T) {
-    const int lane = threadIdx.x & 31;
-    __syncwarp();
-    for (int e = lane; e < kLanes * nin_pad; e += 32) {
-        const int smp = e / nin_pad, i = e % nin_pad;
-        T.act[smp * kPadIn + i] = __float2bfloat16(i < nin ? in[i * kLd + smp] : 0.0f);
-    }
-    __syncwarp();
-}
-
-// The forward of the warp's 32 samples (S.a0 holds their features): a1..a3 and y in S, the BF16-rounded inputs of
-// each layer written back into a0..a3 (what the backward's weight gradients multiply)
-__device__ void mlp_forward(const MlpDev& M, MlpSmem& S, MlpTc& T) {
-    const int lane = threadIdx.x & 31;
-    float* acts[4] = {S.a0, S.a1, S.a2, S.a3};
-    const int nins[4] = {kIn, kHid, kHid, kHid};
+// a warp's weights: its 8 outputs of each layer (k-steps of 16; zero past the layer's inputs and outputs) and biases
+struct MlpFrag {
+    uint32_t w[4][4][2];
+    float b[4][2];
+};
+__device__ __forceinline__ void mlp_load(const __nv_bfloat16* __restrict__ wb, MlpFrag& W) {
+    const int lane = threadIdx.x & 31, nt = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int offw[4] = {kOffW1, kOffW2, kOffW3, kOffW4}, offb[4] = {kOffB1, kOffB2, kOffB3, kOffB4};
+#pragma unroll
     for (int l = 0; l < 4; l++) {
-        const int nin = nins[l], nin_pad = l == 0 ? kKIn : kHid;
-        stage_act(acts[l], nin, nin_pad, T);
-        for (int e = lane; e < kLanes * nin; e += 32) { // (the layer's input as the tensor cores read it)
-            const int smp = e / nin, i = e % nin;
-            acts[l][i * kLd + smp] = __bfloat162float(T.act[smp * kPadIn + i]);
-        }
-        const int offw[4] = {kOffW1, kOffW2, kOffW3, kOffW4}, offb[4] = {kOffB1, kOffB2, kOffB3, kOffB4};
-        const int nout = l == 3 ? kOut : kHid;
-        dense_tc(M.wb + offw[l], M.wb + offb[l], nin_pad, nin, nout, l == 3 ? kOutPad / 8 : kHid / 8, T, l == 3 ? S.y : acts[l + 1], l < 3);
+        const int nin = l == 0 ? kIn : kHid, nout = l == 3 ? kOut : kHid, o = 8 * nt + g;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int i = 16 * k + 8 * h + 2 * t; // (even, as nin: a pair is inside or outside)
+                W.w[l][k][h] = o < nout && i < nin ? *reinterpret_cast<const uint32_t*>(wb + offw[l] + (size_t)o * nin + i) : 0u;
+            }
+#pragma unroll
+        for (int h = 0; h < 2; h++) W.b[l][h] = 8 * nt + 2 * t + h < nout ? __bfloat162float(wb[offb[l] + 8 * nt + 2 * t + h]) : 0.0f;
     }
-    __syncwarp();
+}
+
+// The forward of a tile: x(sample, feature) its features. Ends with y in place and the block synchronised.
+template <class X>
+__device__ __forceinline__ void mlp_forward(const MlpFrag& W, MlpTile& S, X x) {
+    const int lane = threadIdx.x & 31, nt = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    for (int e = threadIdx.x; e < kTile * 48; e += kMlpThreads) { // (36 features, zeros to three k-steps)
+        const int smp = e / 48, i = e % 48;
+        const __nv_bfloat16 v = __float2bfloat16(i < kIn ? x(smp, i) : 0.0f);
+        S.act[0][smp * kPadIn + i] = v;
+        if (i < kIn) S.a[0][smp * kPadF + i] = __bfloat162float(v);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int l = 0; l < 4; l++) {
+        const __nv_bfloat16* in = S.act[l & 1];
+        if (l < 3 || nt < 2) {
+            float c[2][4];
+#pragma unroll
+            for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) c[mt][q] = 0.0f;
+#pragma unroll
+            for (int k = 0; k < (l == 0 ? 3 : 4); k++)
+#pragma unroll
+                for (int mt = 0; mt < 2; mt++) {
+                    const __nv_bfloat16* lo = in + (16 * mt + g) * kPadIn + 16 * k + 2 * t;
+                    const __nv_bfloat16* hi = lo + 8 * kPadIn;
+                    const uint32_t a[4] = {lds32(lo), lds32(hi), lds32(lo + 8), lds32(hi + 8)};
+                    mma_bf16(c[mt], a, W.w[l][k][0], W.w[l][k][1]);
+                }
+            // c0, c1: sample 16 mt + g, outputs 8 nt + 2 t, + 1; c2, c3: sample + 8
+#pragma unroll
+            for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int smp = 16 * mt + g + (q >= 2 ? 8 : 0), o = 8 * nt + 2 * t + (q & 1);
+                    const float v = c[mt][q] + W.b[l][q & 1];
+                    if (l == 3) {
+                        S.y[smp * 16 + o] = v;
+                    } else {
+                        const __nv_bfloat16 r = __float2bfloat16(fmaxf(v, 0.0f));
+                        S.act[(l + 1) & 1][smp * kPadIn + o] = r;
+                        S.a[l + 1][smp * kPadF + o] = __bfloat162float(r);
+                    }
+                }
+        }
+        __syncthreads();
+    }
 }
 
 // ------------------------------------------------------------------------------------------ the step's side
@@ -210,17 +202,19 @@ __global__ void k_mlp_features(FemDev F, MlpDev M, const float4* __restrict__ nd
 }
 
 // The network on every frame node's features: the PCG's guess and scale
-__global__ void __launch_bounds__(kLanes) k_mlp_infer(FemDev F, MlpDev M, float* __restrict__ guess, float* __restrict__ gscale) {
-    __shared__ __align__(16) MlpSmem S;
-    MlpTc& T = S.tc;
-    const int s = threadIdx.x;
-    const int i = blockIdx.x * kLanes + s;
-    const bool on = i < F.nf;
-    for (int f = 0; f < kIn; f++) S.a0[f * kLd + s] = on ? M.feat[(size_t)kIn * i + f] : 0.0f;
-    mlp_forward(M, S, T);
-    if (!on) return;
-    for (int a = 0; a < 3; a++) guess[3 * i + a] = islog(S.y[a * kLd + s]);
-    for (int q = 0; q < 9; q++) gscale[9 * i + q] = ((q % 4) == 0 ? 1.0f : 0.0f) + 0.25f * tanhf(S.y[(3 + q) * kLd + s]);
+__global__ void __launch_bounds__(kMlpThreads) k_mlp_infer(FemDev F, MlpDev M, float* __restrict__ guess, float* __restrict__ gscale) {
+    __shared__ __align__(16) MlpTile S;
+    MlpFrag W;
+    mlp_load(M.wb, W);
+    const int i0 = blockIdx.x * kTile;
+    mlp_forward(W, S, [&](int smp, int f) { return i0 + smp < F.nf ? M.feat[(size_t)kIn * (i0 + smp) + f] : 0.0f; });
+    for (int e = threadIdx.x; e < kTile * kOut; e += kMlpThreads) {
+        const int i = i0 + e / kOut, q = e % kOut;
+        if (i >= F.nf) continue;
+        const float y = S.y[(e / kOut) * 16 + q];
+        if (q < 3) guess[3 * i + q] = islog(y);
+        else gscale[9 * i + q - 3] = (((q - 3) % 4) == 0 ? 1.0f : 0.0f) + 0.25f * tanhf(y);
+    }
 }
 
 // Recording, before the solve: each frame node's features and the block-Jacobi estimate u = (D^-1 rhs)_a (kept in
@@ -293,77 +287,158 @@ __global__ void k_mlp_store_dv(FemDev F, MlpDev M) {
 
 // ------------------------------------------------------------------------------------------ training
 // The loss L = sum_s sum_o w_so (y_so - t_so)^2 / (2 n) over a batch of n samples (idx: the samples, null: x, t, w in
-// order) and its gradient: a block of 32 samples does the forward, the backward, and its share of the gradient summed
-// over its samples in order (gpart: kParams a block; lpart: the block's loss). Deterministic.
-__global__ void __launch_bounds__(kLanes) k_mlp_grad(MlpDev M, const float* __restrict__ x, const float* __restrict__ t, const float* __restrict__ w,
-                                                     const int* __restrict__ idx, int n, float* __restrict__ gpart, float* __restrict__ lpart) {
-    __shared__ __align__(16) MlpSmem S;
-    MlpTc& T = S.tc;
-    const int s = threadIdx.x;
-    const int q = blockIdx.x * kLanes + s;
-    const bool on = q < n;
-    const size_t smp = on ? (size_t)(idx ? idx[q] : q) : 0;
-    for (int f = 0; f < kIn; f++) S.a0[f * kLd + s] = on ? x[kIn * smp + f] : 0.0f;
-    mlp_forward(M, S, T);
-    // d4 = w (y - t) / n into y's place; the sample's loss
-    float loss = 0.0f;
-    const float inv_n = 1.0f / (float)n;
-    for (int o = 0; o < kOut; o++) {
-        const float wo = on ? w[kOut * smp + o] : 0.0f;
-        const float e = on ? S.y[o * kLd + s] - t[kOut * smp + o] : 0.0f;
-        loss += 0.5f * wo * e * e;
-        S.y[o * kLd + s] = wo * e * inv_n;
+// order) and its gradient. A block strides over tiles of 32 samples: the forward, then layer by layer the weights'
+// gradient (a thread a 4 x 4 patch of each matrix, its sums kept in registers over all the block's tiles) and the data
+// gradient (a thread 2 samples x 4 inputs), in FP32 multiply-adds on rows in shared memory; at its end its share of the
+// gradient (gpart: kParams a block) and loss (lpart). Every sum in a fixed order: deterministic.
+// Reads of shared memory bound it (a multiply-add reads half a float of it; the arithmetic, 0.42 G multiply-adds at 20,660
+// samples, is 12 us). B200, 20,660 samples: 477 us with a warp a block, a lane a sample and a share of the gradient stored
+// a tile (29 MB), 72 us so; the sums over the blocks 48 and 10 us. Two blocks an SM: their tiles overlap each other's
+// barriers.
+struct MlpGradSmem {
+    MlpTile T;
+    float d[2][kTile * kPadF];  // the deltas of a layer's outputs and inputs
+    float W[kHid * kHid * 2 + kOut * kHid]; // W2, W3, W4 as FP32
+    double loss[kMlpThreads / 32];
+};
+// acc[o][i] += sum_s d[s][o0 + o] a[s][i0 + i]; db += sum_s d[s][ob]
+__device__ __forceinline__ void mlp_outer(float (&acc)[4][4], const float* d, int ldd, const float* a, int o0, int i0) {
+#pragma unroll 4
+    for (int s = 0; s < kTile; s++) {
+        const float4 dv = *reinterpret_cast<const float4*>(d + s * ldd + o0), av = *reinterpret_cast<const float4*>(a + s * kPadF + i0);
+        const float dd[4] = {dv.x, dv.y, dv.z, dv.w}, aa[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+        for (int o = 0; o < 4; o++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[o][i] = fmaf(dd[o], aa[i], acc[o][i]);
     }
-    // d3 = W4^T d4 (.) [a3 > 0] -> d0;  d2 = W3^T d3 (.) [a2 > 0] -> d1;  d1 = W2^T d2 (.) [a1 > 0] -> d0 (after W2's gradient)
-    auto back = [&](const __nv_bfloat16* W, int nin, int nout, const float* dout, const float* act, float* din) {
-        for (int i2 = 0; i2 < nin; i2++) {
-            float acc = 0.0f;
-            for (int o = 0; o < nout; o++) acc += __bfloat162float(W[(size_t)o * nin + i2]) * dout[o * kLd + s];
-            din[i2 * kLd + s] = act[i2 * kLd + s] > 0.0f ? acc : 0.0f;
+}
+// din[s][i] = [act > 0] sum_o W[o][i] dout[s][o]: samples s0, s0 + 1, inputs i0 .. i0 + 3
+template <int kN>
+__device__ __forceinline__ void mlp_back(const float* W, const float* dout, int ldd, const float* act, float* din, int s0, int i0) {
+    float r[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+#pragma unroll 4
+    for (int o = 0; o < kN; o += 4) {
+        const float4 d0 = *reinterpret_cast<const float4*>(dout + s0 * ldd + o), d1 = *reinterpret_cast<const float4*>(dout + (s0 + 1) * ldd + o);
+        const float dd[2][4] = {{d0.x, d0.y, d0.z, d0.w}, {d1.x, d1.y, d1.z, d1.w}};
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float4 w = *reinterpret_cast<const float4*>(W + (o + u) * kHid + i0);
+            const float ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) r[q][i] = fmaf(ww[i], dd[q][u], r[q][i]);
         }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const float4 a = *reinterpret_cast<const float4*>(act + (s0 + q) * kPadF + i0);
+        *reinterpret_cast<float4*>(din + (s0 + q) * kPadF + i0) =
+            make_float4(a.x > 0 ? r[q][0] : 0.0f, a.y > 0 ? r[q][1] : 0.0f, a.z > 0 ? r[q][2] : 0.0f, a.w > 0 ? r[q][3] : 0.0f);
+    }
+}
+
+__global__ void __launch_bounds__(kMlpThreads, 2) k_mlp_grad(MlpDev M, const float* __restrict__ x, const float* __restrict__ t,
+                                                             const float* __restrict__ w, const int* __restrict__ idx, int n, float* __restrict__ gpart,
+                                                             double* __restrict__ lpart) {
+    extern __shared__ __align__(16) unsigned char mlp_smem[];
+    MlpGradSmem& S = *reinterpret_cast<MlpGradSmem*>(mlp_smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    MlpFrag W;
+    mlp_load(M.wb, W);
+    float *W2 = S.W, *W3 = S.W + kHid * kHid, *W4 = S.W + 2 * kHid * kHid;
+    for (int e = tid; e < kHid * kHid; e += kMlpThreads) W2[e] = __bfloat162float(M.wb[kOffW2 + e]), W3[e] = __bfloat162float(M.wb[kOffW3 + e]);
+    for (int e = tid; e < kOut * kHid; e += kMlpThreads) W4[e] = __bfloat162float(M.wb[kOffW4 + e]);
+    const int og = tid >> 4, ig = tid & 15, o0 = 4 * og, i0 = 4 * ig, s0 = 2 * og; // (this thread's patches)
+    float g1[4][4], g2[4][4], g3[4][4], g4[4][4], b1 = 0, b2 = 0, b3 = 0, b4 = 0;
+#pragma unroll
+    for (int o = 0; o < 4; o++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) g1[o][i] = g2[o][i] = g3[o][i] = g4[o][i] = 0.0f;
+    auto bias = [&](float& b, const float* d, int ldd, int nout) {
+        if (tid < nout)
+            for (int s = 0; s < kTile; s++) b += d[s * ldd + tid];
     };
-    // the block's gradient of one layer: dW[o][i] = sum_s d[o][s] a[i][s], db[o] = sum_s d[o][s]
-    auto layer_grad = [&](float* g, int off_w, int off_b, int nin, int nout, const float* d, const float* a) {
-        __syncthreads();
-        for (int e = s; e < nout * nin; e += kLanes) {
-            const int o = e / nin, i2 = e % nin;
-            float acc = 0.0f;
-            for (int r = 0; r < kLanes; r++) acc += d[o * kLd + r] * a[i2 * kLd + r];
-            g[off_w + e] = acc;
+    double loss = 0.0;
+    const float inv_n = 1.0f / (float)n;
+    const int ntile = (n + kTile - 1) / kTile;
+    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+        const int q0 = tile * kTile;
+        auto sample = [&](int smp) { return (size_t)(idx ? idx[q0 + smp] : q0 + smp); };
+        mlp_forward(W, S.T, [&](int smp, int f) { return q0 + smp < n ? x[kIn * sample(smp) + f] : 0.0f; });
+        // d4 = w (y - t) / n into y's place, its padding zero; the samples' loss
+        for (int e = tid; e < kTile * 16; e += kMlpThreads) {
+            const int smp = e >> 4, o = e & 15;
+            float d = 0.0f;
+            if (o < kOut && q0 + smp < n) {
+                const size_t at = kOut * sample(smp) + o;
+                const float wo = w[at], er = S.T.y[e] - t[at];
+                loss += (double)(0.5f * wo * er * er);
+                d = wo * er * inv_n;
+            }
+            S.T.y[e] = d;
         }
-        for (int o = s; o < nout; o += kLanes) {
-            float acc = 0.0f;
-            for (int r = 0; r < kLanes; r++) acc += d[o * kLd + r];
-            g[off_b + o] = acc;
-        }
         __syncthreads();
-    };
+        if (og < 3) mlp_outer(g4, S.T.y, 16, S.T.a[3], o0, i0);
+        bias(b4, S.T.y, 16, kOut);
+        mlp_back<kOut>(W4, S.T.y, 16, S.T.a[3], S.d[0], s0, i0);
+        __syncthreads();
+        mlp_outer(g3, S.d[0], kPadF, S.T.a[2], o0, i0);
+        bias(b3, S.d[0], kPadF, kHid);
+        mlp_back<kHid>(W3, S.d[0], kPadF, S.T.a[2], S.d[1], s0, i0);
+        __syncthreads();
+        mlp_outer(g2, S.d[1], kPadF, S.T.a[1], o0, i0);
+        bias(b2, S.d[1], kPadF, kHid);
+        mlp_back<kHid>(W2, S.d[1], kPadF, S.T.a[1], S.d[0], s0, i0);
+        __syncthreads();
+        if (ig < kIn / 4) mlp_outer(g1, S.d[0], kPadF, S.T.a[0], o0, i0);
+        bias(b1, S.d[0], kPadF, kHid);
+        __syncthreads();
+    }
     float* g = gpart + (size_t)blockIdx.x * kParams;
-    layer_grad(g, kOffW4, kOffB4, kHid, kOut, S.y, S.a3);
-    back(M.wb + kOffW4, kHid, kOut, S.y, S.a3, S.d0);
-    layer_grad(g, kOffW3, kOffB3, kHid, kHid, S.d0, S.a2);
-    back(M.wb + kOffW3, kHid, kHid, S.d0, S.a2, S.d1);
-    layer_grad(g, kOffW2, kOffB2, kHid, kHid, S.d1, S.a1);
-    back(M.wb + kOffW2, kHid, kHid, S.d1, S.a1, S.d0);
-    layer_grad(g, kOffW1, kOffB1, kIn, kHid, S.d0, S.a0);
-    // the block's loss, in lane order
-    S.d1[s] = loss;
+#pragma unroll
+    for (int o = 0; o < 4; o++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (ig < kIn / 4) g[kOffW1 + (o0 + o) * kIn + i0 + i] = g1[o][i];
+            g[kOffW2 + (o0 + o) * kHid + i0 + i] = g2[o][i], g[kOffW3 + (o0 + o) * kHid + i0 + i] = g3[o][i];
+            if (og < 3) g[kOffW4 + (o0 + o) * kHid + i0 + i] = g4[o][i];
+        }
+    if (tid < kHid) g[kOffB1 + tid] = b1, g[kOffB2 + tid] = b2, g[kOffB3 + tid] = b3;
+    if (tid < kOut) g[kOffB4 + tid] = b4;
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    if (lane == 0) S.loss[warp] = loss;
     __syncthreads();
-    if (s == 0) {
-        float l = 0.0f;
-        for (int r = 0; r < kLanes; r++) l += S.d1[r];
+    if (tid == 0) {
+        double l = 0;
+        for (int r = 0; r < kMlpThreads / 32; r++) l += S.loss[r];
         lpart[blockIdx.x] = l;
     }
 }
 
-// The blocks' gradients summed in block order (into gsum), and, with lr > 0, one Adam step (t: its count from 1) of
-// the FP32 parameters and their BF16 copy
-__global__ void k_mlp_adam(MlpDev M, const float* __restrict__ gpart, int nblocks, float* __restrict__ gsum, float lr, float b1, float b2, float eps,
-                           int t) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kParams) return;
+// The blocks' gradients summed in a fixed order (into gsum; 8 groups of a block's threads each every 8th block's, then the
+// groups in order), and, with lr > 0, one Adam step (t: its count from 1) of the FP32 parameters and their BF16 copy. The
+// first block's second warp adds the blocks' losses to *acc.
+__global__ void __launch_bounds__(256) k_mlp_adam(MlpDev M, const float* __restrict__ gpart, const double* __restrict__ lpart, int nblocks,
+                                                  float* __restrict__ gsum, double* acc, float lr, float b1, float b2, float eps, int t) {
+    __shared__ float part[8][32];
+    const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
     float g = 0.0f;
-    for (int b = 0; b < nblocks; b++) g += gpart[(size_t)b * kParams + p];
+    if (p < kParams)
+#pragma unroll 8
+        for (int b = grp; b < nblocks; b += 8) g += gpart[(size_t)b * kParams + p];
+    part[grp][lane] = g;
+    __syncthreads();
+    if (acc && blockIdx.x == 0 && grp == 1) {
+        double s = 0;
+        for (int b = lane; b < nblocks; b += 32) s += lpart[b];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) *acc += s;
+    }
+    if (grp != 0 || p >= kParams) return;
+    g = 0.0f;
+    for (int r = 0; r < 8; r++) g += part[r][lane];
     if (gsum) gsum[p] = g;
     if (!(lr > 0)) return;
     const float m = b1 * M.m[p] + (1.0f - b1) * g;
@@ -375,31 +450,22 @@ __global__ void k_mlp_adam(MlpDev M, const float* __restrict__ gpart, int nblock
     ((__nv_bfloat16*)M.wb)[p] = __float2bfloat16(wn);
 }
 
-// acc += the blocks' losses, in block order
-__global__ void k_loss_acc(const float* __restrict__ lpart, int nblocks, double* acc) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0;
-        for (int b = 0; b < nblocks; b++) s += lpart[b];
-        *acc += s;
-    }
-}
-
 __global__ void k_mlp_sync_bf16(MlpDev M) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p < kParams) ((__nv_bfloat16*)M.wb)[p] = __float2bfloat16(M.w[p]);
 }
 
-// The network's outputs for n samples (tests)
-__global__ void __launch_bounds__(kLanes) k_mlp_forward_batch(MlpDev M, const float* __restrict__ x, int n, float* __restrict__ y) {
-    __shared__ __align__(16) MlpSmem S;
-    MlpTc& T = S.tc;
-    const int s = threadIdx.x;
-    const int q = blockIdx.x * kLanes + s;
-    const bool on = q < n;
-    for (int f = 0; f < kIn; f++) S.a0[f * kLd + s] = on ? x[(size_t)kIn * q + f] : 0.0f;
-    mlp_forward(M, S, T);
-    if (on)
-        for (int o = 0; o < kOut; o++) y[(size_t)kOut * q + o] = S.y[o * kLd + s];
+// The network's outputs for n samples
+__global__ void __launch_bounds__(kMlpThreads) k_mlp_forward_batch(MlpDev M, const float* __restrict__ x, int n, float* __restrict__ y) {
+    __shared__ __align__(16) MlpTile S;
+    MlpFrag W;
+    mlp_load(M.wb, W);
+    for (int q0 = blockIdx.x * kTile; q0 < n; q0 += gridDim.x * kTile) {
+        mlp_forward(W, S, [&](int smp, int f) { return q0 + smp < n ? x[(size_t)kIn * (q0 + smp) + f] : 0.0f; });
+        for (int e = threadIdx.x; e < kTile * kOut; e += kMlpThreads)
+            if (q0 + e / kOut < n) y[(size_t)kOut * q0 + e] = S.y[(e / kOut) * 16 + e % kOut];
+        __syncthreads();
+    }
 }
 
 } // namespace blg

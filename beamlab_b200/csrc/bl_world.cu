@@ -29,6 +29,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -77,6 +78,12 @@ struct DevBuf {
         free_();
         n = count;
         return cudaMalloc((void**)&p, sizeof(T) * std::max<size_t>(count, 1));
+    }
+    cudaError_t room(size_t count) { // (at least count: grown as needed)
+        if (n >= count) return cudaSuccess;
+        const cudaError_t e = alloc(count);
+        if (e != cudaSuccess) p = nullptr, n = 0;
+        return e;
     }
 };
 
@@ -172,7 +179,10 @@ struct bl_gpu_ctx {
     std::vector<int> lvl_ns;                   // per level: the slices of kUnit rows its columns' factor is cut in
     cudaStream_t aux = nullptr;                // (captures the bodies of conditional graph nodes)
     // the learned warm start (bl_mlp.cuh): parameters, the step's features, recorded samples, training scratch
-    DevBuf<float> mlp_w, mlp_m, mlp_v, feat, prev_dv, smp_x, smp_t, smp_w, gpart, lpart, gsum;
+    DevBuf<float> mlp_w, mlp_m, mlp_v, feat, prev_dv, smp_x, smp_t, smp_w, gpart, gsum;
+    DevBuf<double> lpart, mlp_acc;
+    DevBuf<float> mlp_x, mlp_y, mlp_tw;        // the network's calls on host memory: samples, outputs (targets), weights
+    std::mutex mlp_mutex;                      // (these calls, one at a time)
     DevBuf<__nv_bfloat16> mlp_wb;
     DevBuf<int> adj_ptr, adj, scount, sidx;
     int rec_cap = 0;                           // the samples' capacity
@@ -1560,7 +1570,7 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
             const MlpDev MD = mlp_dev(c);
             if (learned || rec) k_mlp_features<<<(c->NF + 127) / 128, 128, 0, s>>>(F, MD, c->nd.p, c->nforce.p);
             if (rec) k_mlp_record_pre<<<(c->NF + 127) / 128, 128, 0, s>>>(F, MD);
-            if (learned) k_mlp_infer<<<(c->NF + kLanes - 1) / kLanes, kLanes, 0, s>>>(F, MD, c->guess.p, c->gscale.p);
+            if (learned) k_mlp_infer<<<(c->NF + kTile - 1) / kTile, kMlpThreads, 0, s>>>(F, MD, c->guess.p, c->gscale.p);
             auto cholesky = [c, &F](cudaStream_t cs) {
                 if (c->fem_mode == 2) {
                     // multifrontal: the factorization, then the backward solves, a cooperative launch each (their flags zeroed first)
@@ -1846,6 +1856,9 @@ int bl_gpu_destroy(bl_gpu_ctx* c) {
     free_device(c);
     free_statics(c);
     c->deverr.free_();
+    c->mlp_w.free_(), c->mlp_m.free_(), c->mlp_v.free_(), c->mlp_wb.free_(), c->smp_x.free_(), c->smp_t.free_(), c->smp_w.free_();
+    c->scount.free_(), c->sidx.free_(), c->gpart.free_(), c->lpart.free_(), c->gsum.free_();
+    c->mlp_x.free_(), c->mlp_y.free_(), c->mlp_tw.free_(), c->mlp_acc.free_();
     if (c->order_event) cudaEventDestroy(c->order_event);
     if (c->stream) cudaStreamDestroy(c->stream);
     if (c->aux) cudaStreamDestroy(c->aux);
@@ -2267,16 +2280,29 @@ int bl_gpu_mlp_samples(bl_gpu_ctx* c, int32_t* n) {
     return BL_GPU_OK;
 }
 
+// The network's calls on host memory, one at a time: their device buffers are the context's, and are given back at the end
+// of a call that needed more than kMlpKeep floats of one (64 MB: 466,000 samples). To allocate and release them on each
+// call took as long as its kernels.
+constexpr size_t kMlpKeep = (size_t)16 << 20;
+struct MlpCall {
+    bl_gpu_ctx* c;
+    std::lock_guard<std::mutex> lock;
+    explicit MlpCall(bl_gpu_ctx* c) : c(c), lock(c->mlp_mutex) {}
+    ~MlpCall() {
+        if (c->mlp_x.n > kMlpKeep) c->mlp_x.free_(), c->mlp_y.free_(), c->mlp_tw.free_();
+    }
+};
+
 // one pass of k_mlp_grad over n samples (x, t, w on the device; idx: the samples, or null) and, with lr > 0, Adam
 static int mlp_batch(bl_gpu_ctx* c, const float* x, const float* t, const float* w, const int* idx, int n, float lr, float* gsum, double* acc) {
-    const int nblk = (n + kLanes - 1) / kLanes;
-    if (c->gpart.n < (size_t)nblk * kParams) BL_CUDA(c, c->gpart.alloc((size_t)nblk * kParams));
-    if (c->lpart.n < (size_t)nblk) BL_CUDA(c, c->lpart.alloc(nblk));
+    const int nblk = std::min((n + kTile - 1) / kTile, 2 * 148); // (two blocks an SM)
+    BL_CUDA(c, c->gpart.room((size_t)nblk * kParams));
+    BL_CUDA(c, c->lpart.room(nblk));
     const MlpDev M = mlp_dev(c);
-    k_mlp_grad<<<nblk, kLanes, 0, c->stream>>>(M, x, t, w, idx, n, c->gpart.p, c->lpart.p);
+    BL_CUDA(c, cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpGradSmem)));
+    k_mlp_grad<<<nblk, kMlpThreads, sizeof(MlpGradSmem), c->stream>>>(M, x, t, w, idx, n, c->gpart.p, c->lpart.p);
     if (lr > 0) c->adam_t++;
-    k_mlp_adam<<<(kParams + 255) / 256, 256, 0, c->stream>>>(M, c->gpart.p, nblk, gsum, lr, 0.9f, 0.999f, 1e-8f, std::max(c->adam_t, 1));
-    if (acc) k_loss_acc<<<1, 32, 0, c->stream>>>(c->lpart.p, nblk, acc);
+    k_mlp_adam<<<(kParams + 31) / 32, 256, 0, c->stream>>>(M, c->gpart.p, c->lpart.p, nblk, gsum, acc, lr, 0.9f, 0.999f, 1e-8f, std::max(c->adam_t, 1));
     BL_CUDA(c, cudaGetLastError());
     return BL_GPU_OK;
 }
@@ -2321,41 +2347,37 @@ int bl_gpu_mlp_forward(bl_gpu_ctx* c, const float* x, int32_t n, float* y) {
     if (!c || n < 0 || (n > 0 && (!x || !y))) return BL_GPU_EINVAL;
     if (n == 0) return BL_GPU_OK;
     BL_CUDA(c, cudaSetDevice(c->cfg.device));
-    DevBuf<float> dx, dy;
-    BL_CUDA(c, dx.alloc((size_t)kIn * n));
-    BL_CUDA(c, dy.alloc((size_t)kOut * n));
-    BL_CUDA(c, cudaMemcpy(dx.p, x, sizeof(float) * kIn * n, cudaMemcpyHostToDevice));
-    k_mlp_forward_batch<<<(n + kLanes - 1) / kLanes, kLanes, 0, c->stream>>>(mlp_dev(c), dx.p, n, dy.p);
+    const MlpCall call(c);
+    BL_CUDA(c, c->mlp_x.room((size_t)kIn * n));
+    BL_CUDA(c, c->mlp_y.room((size_t)kOut * n));
+    BL_CUDA(c, cudaMemcpyAsync(c->mlp_x.p, x, sizeof(float) * kIn * n, cudaMemcpyHostToDevice, c->stream));
+    k_mlp_forward_batch<<<std::min((n + kTile - 1) / kTile, 4 * 148), kMlpThreads, 0, c->stream>>>(mlp_dev(c), c->mlp_x.p, n, c->mlp_y.p);
     BL_CUDA(c, cudaGetLastError());
+    BL_CUDA(c, cudaMemcpyAsync(y, c->mlp_y.p, sizeof(float) * kOut * n, cudaMemcpyDeviceToHost, c->stream));
     BL_CUDA(c, cudaStreamSynchronize(c->stream));
-    BL_CUDA(c, cudaMemcpy(y, dy.p, sizeof(float) * kOut * n, cudaMemcpyDeviceToHost));
-    dx.free_(), dy.free_();
     return BL_GPU_OK;
 }
 
 int bl_gpu_mlp_gradient(bl_gpu_ctx* c, const float* x, const float* t, const float* w, int32_t n, float* grad, float* loss) {
     if (!c || n < 1 || !x || !t || !w || !grad) return BL_GPU_EINVAL;
     BL_CUDA(c, cudaSetDevice(c->cfg.device));
-    DevBuf<float> dx, dt, dw;
-    DevBuf<double> acc;
-    BL_CUDA(c, dx.alloc((size_t)kIn * n));
-    BL_CUDA(c, dt.alloc((size_t)kOut * n));
-    BL_CUDA(c, dw.alloc((size_t)kOut * n));
-    BL_CUDA(c, acc.alloc(1));
-    BL_CUDA(c, cudaMemcpy(dx.p, x, sizeof(float) * kIn * n, cudaMemcpyHostToDevice));
-    BL_CUDA(c, cudaMemcpy(dt.p, t, sizeof(float) * kOut * n, cudaMemcpyHostToDevice));
-    BL_CUDA(c, cudaMemcpy(dw.p, w, sizeof(float) * kOut * n, cudaMemcpyHostToDevice));
-    BL_CUDA(c, cudaMemset(acc.p, 0, sizeof(double)));
-    int rc = mlp_batch(c, dx.p, dt.p, dw.p, nullptr, n, 0.0f, c->gsum.p, acc.p);
-    if (!rc) {
-        BL_CUDA(c, cudaStreamSynchronize(c->stream));
-        BL_CUDA(c, cudaMemcpy(grad, c->gsum.p, sizeof(float) * kParams, cudaMemcpyDeviceToHost));
-        double a = 0;
-        BL_CUDA(c, cudaMemcpy(&a, acc.p, sizeof(double), cudaMemcpyDeviceToHost));
-        if (loss) *loss = (float)(a / n);
-    }
-    dx.free_(), dt.free_(), dw.free_(), acc.free_();
-    return rc;
+    const MlpCall call(c);
+    BL_CUDA(c, c->mlp_x.room((size_t)kIn * n));
+    BL_CUDA(c, c->mlp_y.room((size_t)kOut * n));
+    BL_CUDA(c, c->mlp_tw.room((size_t)kOut * n));
+    BL_CUDA(c, c->mlp_acc.room(1));
+    BL_CUDA(c, cudaMemcpyAsync(c->mlp_x.p, x, sizeof(float) * kIn * n, cudaMemcpyHostToDevice, c->stream));
+    BL_CUDA(c, cudaMemcpyAsync(c->mlp_y.p, t, sizeof(float) * kOut * n, cudaMemcpyHostToDevice, c->stream));
+    BL_CUDA(c, cudaMemcpyAsync(c->mlp_tw.p, w, sizeof(float) * kOut * n, cudaMemcpyHostToDevice, c->stream));
+    BL_CUDA(c, cudaMemsetAsync(c->mlp_acc.p, 0, sizeof(double), c->stream));
+    const int rc = mlp_batch(c, c->mlp_x.p, c->mlp_y.p, c->mlp_tw.p, nullptr, n, 0.0f, c->gsum.p, c->mlp_acc.p);
+    if (rc) return rc;
+    double a = 0;
+    BL_CUDA(c, cudaMemcpyAsync(grad, c->gsum.p, sizeof(float) * kParams, cudaMemcpyDeviceToHost, c->stream));
+    BL_CUDA(c, cudaMemcpyAsync(&a, c->mlp_acc.p, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    BL_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (loss) *loss = (float)(a / n);
+    return BL_GPU_OK;
 }
 
 int bl_gpu_fem_stats(bl_gpu_ctx* c, bl_fem_stats* out) {
