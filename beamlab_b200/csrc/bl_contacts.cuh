@@ -295,7 +295,8 @@ __global__ void __launch_bounds__(1024) k_islands(Body* __restrict__ bodies, int
 // ------------------------------------------------------------------------------------------ wake requests (each substep)
 // simulate_island's substep start (world.cpp:3333-3337): a sleeping body a moving partner touched wakes; its beams step
 // again (SoftBody::wake, softbody.h:996).
-__global__ void k_wake(Body* __restrict__ bodies, uint32_t* __restrict__ bmeta) {
+__global__ void k_wake(Body* bodies, uint32_t* bmeta) {
+    pdl_wait();
     Body& B = bodies[blockIdx.x];
     if (!B.wake_request || B.island < 0) return;
     for (int j = threadIdx.x; j < B.nbeams; j += blockDim.x) bmeta[B.beam0 + j] &= ~kBeamAsleep;

@@ -349,7 +349,8 @@ __device__ __forceinline__ void beam_step(int j, uint32_t meta, float4 s0, float
 }
 
 // ------------------------------------------------------------------------------------------ shocks
-// SoftBody::compute_shock_forces (softbody.cpp:472-566), a thread a shock: its model's rates for the beam's length and
+// SoftBody::compute_shock_forces (softbody.cpp:472-566), a thread a shock, in the beams' kernels beside the beams (which
+// leave a shock's beam alone; a launch of its own cost a 512-node car 2.4 us a substep): its model's rates for the beam's length and
 // rate (type 1 bounded, 2 progressive with soft bump stops, 3 split damping), the break test, the beam's stress, and
 // the scalar its ends add after their beams' (k_force: ssc, in the order of the shocks)
 struct ShockDev {
@@ -357,18 +358,17 @@ struct ShockDev {
     const int* ptr;          // per node + 1: its shocks in sinc
     const int2* inc;         // (shock | bit 31 where the node is the beam's b end, the other end)
     float* ssc;              // per shock: its scalar (kNoPush: none this substep)
+    const int2* ab;          // the beams' ends
+    int n;
 };
-__global__ void k_shocks(ShockDev S, int nshocks, const int2* __restrict__ ab, const float4* bst, uint32_t* __restrict__ bmeta,
-                         float* __restrict__ stress, const int* __restrict__ bbody, const float4* nd, Body* __restrict__ bodies) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    pdl_wait();
-    if (q >= nshocks) return;
+__device__ void shock_step(int q, const ShockDev& S, const float4* bst, uint32_t* bmeta, float* __restrict__ stress, const int* __restrict__ bbody,
+                           const float4* nd, Body* __restrict__ bodies) {
     S.ssc[q] = kNoPush;
     const bl_shock s = S.sh[q];
     const int j = (int)s.beam;
     const uint32_t meta = bmeta[j];
     if ((meta & kBeamAsleep) || (((meta >> 8) & 0xffu) & BF_BROKEN)) return;
-    const int2 e = ab[j];
+    const int2 e = S.ab[j];
     const float4 pa = nd[2 * e.x], va = nd[2 * e.x + 1], pb = nd[2 * e.y], vb = nd[2 * e.y + 1];
     const v3 dis = V(pa.x - pb.x, pa.y - pb.y, pa.z - pb.z);
     const float len2 = dot(dis, dis);
@@ -527,12 +527,16 @@ struct WheelDev {
 // controller's torque (every substep: the first short step's), the brake's stop torque against the average speed and
 // the last reaction, the share a tyre node, the tread's speed (summed in the builder's order), the average speed and
 // the reaction of the inertia, and the drive's reaction on the arm; the nodes' terms are k_force's.
-__device__ void wheel_step(int w, int lane, const float4* nd, const int4* __restrict__ info, const Body* __restrict__ bodies,
-                           const WheelDev& wh, float dt) {
+// wait: called once, before the nodes and the bodies are read (what stays as it is during the predecessor is read before).
+template <class Wait>
+__device__ __forceinline__ void wheel_step(int w, int lane, const float4* nd, const int4* __restrict__ info, const Body* bodies, const WheelDev& wh, float dt,
+                                           Wait wait) {
     const int4 W = wh.wheel[w];
-    if (W.w == 0 || bodies[info[W.x].w].sleeping) return; // (an asleep body's forces are not made)
     const float4 ctl = wh.wctl[w], st = wh.wst[w];
     const int4 A = wh.warm[w];
+    const int own = W.w > 0 ? info[W.x].w : 0, first = lane < W.w ? wh.wlist[W.z + lane] : 0;
+    wait();
+    if (W.w == 0 || bodies[own].sleeping) return; // (an asleep body's forces are not made)
     float T = ctl.x;
     if (ctl.y > 0) {
         const float stop = -st.y * ctl.z * ctl.w / dt - st.w;
@@ -548,7 +552,7 @@ __device__ void wheel_step(int w, int lane, const float4* nd, const int4* __rest
         float term = 0.0f;
         bool has = false;
         if (j < W.w) {
-            const int ni = wh.wlist[W.z + j];
+            const int ni = c == 0 ? first : wh.wlist[W.z + j];
             const float4 hp = (j & 1) ? H1 : H0, hv = (j & 1) ? U1 : U0, P = nd[2 * ni], Vn = nd[2 * ni + 1];
             v3 rad = V(P.x - hp.x, P.y - hp.y, P.z - hp.z);
             const float rl2 = dot(rad, rad);
@@ -585,29 +589,35 @@ __device__ void wheel_step(int w, int lane, const float4* nd, const int4* __rest
     wh.wst[w] = make_float4(sp, avg, T, lrt);
 }
 // The beams by plain loads: two beams a thread (j and j + blockDim.x of the block's pair of tiles), both beams' loads
-// issued before either computes, the beams' own arrays before the wait for the predecessor (which writes the nodes). The
-// blocks past bblocks take the wheels, a warp a wheel. Thread t < nbodies of the grid also resets body t's bounds
+// issued before either computes, the beams' own arrays before the wait for the predecessor (which writes the nodes, or the
+// meta words: k_wake). The sblocks blocks past bblocks take the shocks, those after them the wheels, a warp a wheel. Thread t < nbodies of the grid also resets body t's bounds
 // accumulator for this substep's k_integrate. The kernel of all but the largest worlds (kPlainBeams): no copy into shared
 // memory to wait for first, and the wheels beside the beams instead of after a block's tiles.
 __global__ void __launch_bounds__(256) k_beams(const int2* __restrict__ ab, const float2* __restrict__ kd, float4* __restrict__ bst,
-                                               uint32_t* __restrict__ bmeta, const float4* __restrict__ bcold, float* __restrict__ stress,
+                                               uint32_t* bmeta, const float4* __restrict__ bcold, float* __restrict__ stress,
                                                const int* __restrict__ bbody, float* __restrict__ fsc, const float4* nd,
-                                               Body* __restrict__ bodies, int nbeams, int nbodies, int bblocks, const int4* __restrict__ info, WheelDev wh,
-                                               float dt) {
+                                               Body* __restrict__ bodies, int nbeams, int nbodies, int bblocks, int sblocks, const int4* __restrict__ info,
+                                               WheelDev wh, ShockDev sk, float dt) {
+    if ((int)blockIdx.x >= bblocks + sblocks) {
+        const int w = (int)((blockIdx.x - bblocks - sblocks) * blockDim.x + threadIdx.x) >> 5; // (the warp's: its lanes go together)
+        if (w < wh.nreal) wheel_step(w, threadIdx.x & 31, nd, info, bodies, wh, dt, [] { pdl_wait(); });
+        else pdl_wait();
+        return;
+    }
     if ((int)blockIdx.x >= bblocks) {
         pdl_wait();
-        const int w = (int)((blockIdx.x - bblocks) * blockDim.x + threadIdx.x) >> 5;
-        if (w < wh.nreal) wheel_step(w, threadIdx.x & 31, nd, info, bodies, wh, dt); // (w is the warp's: its lanes go together)
+        const int q = (blockIdx.x - bblocks) * blockDim.x + threadIdx.x;
+        if (q < sk.n) shock_step(q, sk, bst, bmeta, stress, bbody, nd, bodies);
         return;
     }
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int j0 = 2 * blockIdx.x * blockDim.x + threadIdx.x, j1 = j0 + blockDim.x;
     const bool h0 = j0 < nbeams, h1 = j1 < nbeams;
-    const uint32_t m0 = h0 ? bmeta[j0] : kBeamAsleep, m1 = h1 ? bmeta[j1] : kBeamAsleep;
     const int2 e0 = h0 ? ab[j0] : make_int2(0, 0), e1 = h1 ? ab[j1] : make_int2(0, 0);
     const float4 s0 = h0 ? bst[j0] : make_float4(0, 0, 0, 0), s1 = h1 ? bst[j1] : make_float4(0, 0, 0, 0);
     const float2 c0 = h0 ? kd[j0] : make_float2(0, 0), c1 = h1 ? kd[j1] : make_float2(0, 0);
     pdl_wait();
+    const uint32_t m0 = h0 ? bmeta[j0] : kBeamAsleep, m1 = h1 ? bmeta[j1] : kBeamAsleep;
     if (t < nbodies) {
         Body& B = bodies[t];
         B.acc_mn[0] = B.acc_mn[1] = B.acc_mn[2] = 1e30f;
@@ -650,7 +660,7 @@ __global__ void __launch_bounds__(kBeamThreads) k_beams_tma(const void* __restri
                                                             float4* __restrict__ bst, uint32_t* __restrict__ bmeta, const float4* __restrict__ bcold,
                                                             float* __restrict__ stress, const int* __restrict__ bbody, float* __restrict__ fsc,
                                                             const float4* nd, Body* __restrict__ bodies, int nbeams, int nbodies, int ntiles,
-                                                            uint32_t* __restrict__ deverr, const int4* __restrict__ info, WheelDev wh, float dt,
+                                                            uint32_t* __restrict__ deverr, const int4* __restrict__ info, WheelDev wh, ShockDev sk, float dt,
                                                             unsigned long long wait_ns) {
     using Stage = BeamStage<kEnds16>;
     using AbT = typename std::remove_reference<decltype(Stage::ab[0])>::type;
@@ -724,10 +734,11 @@ __global__ void __launch_bounds__(kBeamThreads) k_beams_tma(const void* __restri
         }
         issued = min(issued + 1, mine);
     }
-    // then the wheels (a warp a wheel: it reads the substep's starting state as the beams do, and only
-    // k_force reads what it writes)
+    // then the shocks and the wheels (a warp a wheel): they read the substep's starting state as the beams do, and only
+    // k_force reads what they write
+    for (int q = blockIdx.x * kBeamThreads + tid; q < sk.n; q += gridDim.x * kBeamThreads) shock_step(q, sk, bst, bmeta, stress, bbody, nd, bodies);
     for (int w = blockIdx.x * (kBeamThreads / 32) + (tid >> 5); w < wh.nreal; w += gridDim.x * (kBeamThreads / 32))
-        wheel_step(w, tid & 31, nd, info, bodies, wh, dt);
+        wheel_step(w, tid & 31, nd, info, bodies, wh, dt, [] {});
 }
 
 // The frame bodies' gather (NodeFem): their nodes' forces go to the frame's implicit step
@@ -1219,33 +1230,40 @@ __global__ void __launch_bounds__(256) k_integrate(float4* nd, const int4* __res
 // wheel, a lane a tyre node (in chunks of 32) - each node in contact gets tyre_contact on its force and its normal
 // force; the touching ones' needs and caps summed in ascending node order (every lane adds the same broadcast values
 // in the same order); each touching node sticks (its need) if the patch as a whole can hold, else slides; then
-// SoftBody::integrate_nodes for them, the warp's bounds, top speed and contacts into the body's accumulators.
+// SoftBody::integrate_nodes for them, the warp's bounds, top speed and contacts into the body's accumulators. A chain of
+// dependent loads bounds it; those that k_integrate leaves alone are made beside it, before the wait. B200, a frame of 33
+// substeps of a car of four wheels and four shocks: 580 us with the shocks in a launch of their own and every load
+// after the wait, 474 us so.
 __global__ void __launch_bounds__(256) k_tyres(float4* nd, const int4* __restrict__ info, Body* __restrict__ bodies, float dt,
                                                int nwheels, int first, const float4* fnode, WheelDev wh) {
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    // (the wheel's lists are fixed, the forces complete before k_integrate starts, and k_integrate leaves the nodes in
+    // contact to this kernel: read before the wait, for a wheel of up to 32 nodes)
+    const bool mine = w < nwheels;
+    const int4 W = mine ? wh.wheel[w] : make_int4(0, 0, 0, 0);
+    int i = lane < W.w ? wh.wnodes[W.z + lane] : -1;
+    const int body = lane < W.w ? info[i].w : 0;
+    float4 P = make_float4(0, 0, 0, 0), Vv = P, f4 = P;
+    if (i >= 0) P = nd[2 * i], Vv = nd[2 * i + 1], f4 = fnode[i];
     pdl_wait();
-    if (w >= nwheels) return; // (w is the warp's: its lanes leave together)
-    const int4 W = wh.wheel[w];
-    if (W.w == 0) return;
-    const int body = info[wh.wnodes[W.z]].w;
+    if (W.w == 0) return; // (w is the warp's: its lanes leave together)
     v3 need = V(0, 0, 0), mn = V(1e30f, 1e30f, 1e30f), mx = V(-1e30f, -1e30f, -1e30f);
     float cap = 0.0f, vv = 0.0f;
     int cnt = 0;
     // pass 1: the contacts and the patch's sums (one chunk's nodes kept in registers for pass 2)
-    int i = -1;
     TyreC t = {};
     v3 f = V(0, 0, 0);
-    float4 P = make_float4(0, 0, 0, 0), Vv = P;
     bool pend = false;
     for (int c = 0; c < W.w; c += 32) {
         pend = false;
         if (c + lane < W.w) {
-            i = wh.wnodes[W.z + c + lane];
-            const float4 tf = wh.tfric[i];
+            if (c > 0) {
+                i = wh.wnodes[W.z + c + lane];
+                P = nd[2 * i], Vv = nd[2 * i + 1], f4 = fnode[i];
+            }
+            const float4 tf = wh.tfric[i], cn = wh.tcon[i];
             pend = tf.w != 0.0f;
             if (pend) {
-                const float4 cn = wh.tcon[i], f4 = fnode[i];
-                P = nd[2 * i], Vv = nd[2 * i + 1];
                 const int surf = __float_as_int(tf.y);
                 const GroundModel& gm = c_ground[surf < kSurfCount ? surf : 0];
                 f = V(f4.x, f4.y, f4.z);
@@ -1261,6 +1279,8 @@ __global__ void __launch_bounds__(256) k_tyres(float4* nd, const int4* __restric
             cap = cap + __shfl_sync(0xffffffffu, t.cap, l);
         }
     }
+    // (no node of the wheel in contact: nothing of it is integrated here)
+    if (W.w <= 32 && !__any_sync(0xffffffffu, pend)) return;
     const bool stick = length(need) <= cap;
     // pass 2: the forces applied and the nodes integrated (a wheel of more than 32 nodes: its contacts again)
     for (int c = 0; c < W.w; c += 32) {
@@ -1271,8 +1291,8 @@ __global__ void __launch_bounds__(256) k_tyres(float4* nd, const int4* __restric
                 const float4 tf = wh.tfric[i];
                 pend = tf.w != 0.0f;
                 if (pend) {
-                    const float4 cn = wh.tcon[i], f4 = fnode[i];
-                P = nd[2 * i], Vv = nd[2 * i + 1];
+                    const float4 cn = wh.tcon[i];
+                    f4 = fnode[i], P = nd[2 * i], Vv = nd[2 * i + 1];
                     const int surf = __float_as_int(tf.y);
                     const GroundModel& gm = c_ground[surf < kSurfCount ? surf : 0];
                     f = V(f4.x, f4.y, f4.z);

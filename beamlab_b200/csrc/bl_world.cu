@@ -153,7 +153,7 @@ struct bl_gpu_ctx {
     DevBuf<int> dup, dpid, dpart;
     DevBuf<float4> dpmv, dpacc;
     int NW = 0;                                // the wheels of all bodies, and lone tyre nodes (k_tyres: a warp a wheel)
-    int NSH = 0;                               // the shocks of all bodies (k_shocks)
+    int NSH = 0;                               // the shocks of all bodies (the beams' kernels step them)
     DevBuf<bl_shock> dshock;
     DevBuf<int> sh_ptr;
     DevBuf<int2> sh_inc;
@@ -1355,7 +1355,7 @@ static int ensure_committed(bl_gpu_ctx* c) {
 static bool rebuild_at(const bl_gpu_ctx* c, int k) { return k % c->interval == 0; } // (s == 0 || s >= next_rebuild)
 
 static int64_t frame_launches(const bl_gpu_ctx* c, int n) {
-    int64_t per = 3 + (c->any_drag ? 1 : 0) + (c->NW > 0 ? 1 : 0) + (c->NSH > 0 ? 1 : 0);
+    int64_t per = 3 + (c->any_drag ? 1 : 0) + (c->NW > 0 ? 1 : 0);
     if (c->NF > 0) {
         if (c->fem_only) per -= 2; // (no beams, no other nodes)
         per += c->fem_launches + (c->cfg.fem_check_residual ? 2 : 0) + (c->fem_ground ? 1 : 0);
@@ -1488,7 +1488,7 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
     DragDev dg{c->dup.p, c->dpid.p, c->dpart.p, c->dpmv.p, c->dpacc.p};
     WheelDev wh{c->dwheel.p, c->dwnodes.p, c->dwlist.p, c->dwc_ptr.p, c->dwc.p, c->dtcon.p, c->dtfric.p, c->dwst.p, c->dwctl.p,
                 c->dwarm.p, c->dwcf.p, c->dwper.p, c->NWR, c->cfg.tyre_grip};
-    ShockDev sk{c->dshock.p, c->sh_ptr.p, c->sh_inc.p, c->ssc.p};
+    ShockDev sk{c->dshock.p, c->sh_ptr.p, c->sh_inc.p, c->ssc.p, c->ab.p, c->NSH};
     NodeFem nfm{c->fslot.p, c->fiperm.p, c->gdiag_ptr.p, c->gdiag.p, c->ton.p, c->tf.p, c->tt.p, c->ftorque.p, c->nforce.p, c->ext.p,
                 c->mon.p, c->mfa.p, c->mta.p, c->mtb.p};
     const FemDev& F = c->fd;
@@ -1500,7 +1500,7 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
     for (int k = 0; k < n; k++) {
         if (c->contacts_on) {
             // wake requests, then the pair search on its substeps (on the positions and velocities the substep starts from)
-            k_wake<<<c->B, 256, 0, s>>>(c->dbodies.p, c->bmeta.p);
+            go(k_wake, c->B, 256, 0, c->dbodies.p, c->bmeta.p);
             if (rebuild_at(c, k)) {
                 cudaMemsetAsync(c->pair_total.p, 0, sizeof(int), s);
                 cudaMemsetAsync(c->sc.p, 0, 8 * sizeof(int), s);
@@ -1517,19 +1517,18 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
         if (c->fem_only) {
             // (no beams; the bounds accumulators are reset by the assembly)
         } else if (bulk) {
-            // (the wheels' step in the same launch, after each block's tiles)
+            // (the shocks and the wheels' step in the same launch, after each block's tiles)
             if (c->ends16)
                 go(k_beams_tma<true>, c->beam_grid, kBeamThreads, beam_smem<true>(), c->ab16.p, c->tbase.p, c->kd.p, c->bst.p, c->bmeta.p, c->bcold.p,
-                   c->stress.p, c->bbody.p, c->fsc.p, c->nd.p, c->dbodies.p, c->M, c->B, c->beam_tiles, c->deverr.p, c->info.p, wh, dt, c->wait_ns);
+                   c->stress.p, c->bbody.p, c->fsc.p, c->nd.p, c->dbodies.p, c->M, c->B, c->beam_tiles, c->deverr.p, c->info.p, wh, sk, dt, c->wait_ns);
             else
                 go(k_beams_tma<false>, c->beam_grid, kBeamThreads, beam_smem<false>(), c->ab.p, nullptr, c->kd.p, c->bst.p, c->bmeta.p, c->bcold.p,
-                   c->stress.p, c->bbody.p, c->fsc.p, c->nd.p, c->dbodies.p, c->M, c->B, c->beam_tiles, c->deverr.p, c->info.p, wh, dt, c->wait_ns);
+                   c->stress.p, c->bbody.p, c->fsc.p, c->nd.p, c->dbodies.p, c->M, c->B, c->beam_tiles, c->deverr.p, c->info.p, wh, sk, dt, c->wait_ns);
         } else {
-            go(k_beams, gb + (c->NWR * 32 + bt - 1) / bt, bt, 0, c->ab.p, c->kd.p, c->bst.p, c->bmeta.p, c->bcold.p, c->stress.p, c->bbody.p, c->fsc.p, c->nd.p,
-               c->dbodies.p, c->M, c->B, gb, c->info.p, wh, dt);
+            const int gs = (c->NSH + bt - 1) / bt;
+            go(k_beams, gb + gs + (c->NWR * 32 + bt - 1) / bt, bt, 0, c->ab.p, c->kd.p, c->bst.p, c->bmeta.p, c->bcold.p, c->stress.p, c->bbody.p, c->fsc.p, c->nd.p,
+               c->dbodies.p, c->M, c->B, gb, gs, c->info.p, wh, sk, dt);
         }
-        if (c->NSH > 0)
-            go(k_shocks, (c->NSH + 127) / 128, 128, 0, sk, c->NSH, c->ab.p, c->bst.p, c->bmeta.p, c->stress.p, c->bbody.p, c->nd.p, c->dbodies.p);
         if (c->NT > 0 && c->any_plastic) k_tri_eval<true><<<(c->NT + 127) / 128, 128, 0, s>>>(F, c->nd.p);
         else if (c->NT > 0) k_tri_eval<false><<<(c->NT + 127) / 128, 128, 0, s>>>(F, c->nd.p);
         if (c->NM > 0 && c->any_plastic_members) k_member_eval<true><<<(c->NM + 3) / 4, 128, 0, s>>>(F, c->nd.p);
