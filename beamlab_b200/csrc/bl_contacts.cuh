@@ -55,9 +55,6 @@ struct Contacts {
     float4* hit_b;             // per pair: normal.xyz, w = 1 when the pair is in contact
     uint32_t* hbits;           // per 32 pairs: bit j set when pair 32 w + j is in contact
     int* hidx;                 // per island's pair range: its contacts' pair indices, in pair order
-    ContactRec* crec;          // the contacts' records of the islands that run whole (a substep's, taken in turn)
-    int* crec_n;               // records taken this substep (reset by k_detect)
-    int crec_cap;
     int whole_max;             // contacts an island runs whole at most (bl_gpu_config.contact_whole_max)
     int max_pairs;
     // rebuild scratch
@@ -314,7 +311,6 @@ namespace blg {
 // the pair is in contact, hit_b.w = 0 when not
 __global__ void __launch_bounds__(256) k_detect(const float4* __restrict__ nd, const int4* __restrict__ info, const Body* __restrict__ bodies, Contacts C) {
     const int total = min(*C.pair_total, C.max_pairs);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *C.crec_n = 0; // (k_collide takes its records after this kernel)
     // (a warp takes 32 consecutive pairs: its ballot is their word of hit bits)
     for (int i0 = blockIdx.x * blockDim.x; i0 < total; i0 += gridDim.x * blockDim.x) {
         const int i = i0 + (int)threadIdx.x;
@@ -382,25 +378,38 @@ __global__ void __launch_bounds__(256) k_detect(const float4* __restrict__ nd, c
 // in pair order, as the reference's loop (world.cpp:2999) - but only contacts that share a node depend on each other.
 // A CTA an island:
 //  1. its contacts (its pairs with a hit bit, in pair order) listed by a block scan; their nodes hashed into
-//     shared-memory force slots and the forces loaded there;
-//  2. each contact's record - its slots, the accumulation weights, relative velocity and normal, and every term of the
+//     shared-memory force slots;
+//  2. each contact's level, one above its nodes' earlier contacts' levels, so the contacts of one level touch distinct
+//     nodes; the contacts sorted by level. Up to kParMax contacts: each slot's contacts in a list, from it each
+//     contact's nearest earlier one at each of its nodes, then one warp goes through the contacts 32 at a time
+//     (contact_levels). More: one thread, in pair order;
+//  3. each contact's record - its slots, the accumulation weights, relative velocity and normal, and every term of the
 //     contact law that does not depend on the forces (the slip direction and speed, the Stribeck exponentials, the
-//     restitution and push terms, the soft ground's drag and buoyancy) - formed in parallel;
-//  3. each contact's level, one above its nodes' earlier contacts' levels (one thread, in pair order), so the contacts
-//     of one level touch distinct nodes; the levels run one after another, a level's contacts at once, each contact
-//     with only its force-dependent arithmetic (apply_contact) - every contact sees the forces the serial loop gives
-//     it. Up to Contacts::whole_max contacts the island runs whole (its records in global memory, its levels over all
-//     of it, formed while the records are); more, 512 at a time (records and levels in shared memory);
-//  4. the forces written back. An island with more distinct contact nodes than the slots hold runs the loop on global
-//     memory (collide_island_global). Results are the same bits every way.
+//     restitution and push terms, the soft ground's drag and buoyancy) - formed in level order into shared memory, half a
+//     buffer at a time, while
+//  4. one warp runs the levels one after another, a level's contacts at once, each contact with only its force-dependent
+//     arithmetic (apply_contact) - every contact sees the forces the serial loop gives it;
+//  5. the forces written back. Above Contacts::whole_max contacts an island runs kRecChunk at a time (records and levels
+//     of each chunk in turn); with more distinct contact nodes than the slots hold it runs the loop on global memory
+//     (collide_island_global). Results are the same bits every way.
+// Up to kSmall contacts each has a thread, its record is formed while one warp finds the levels, and no half buffers are
+// needed (nearly every island: 350 contacts at the peak of two vehicles' crash).
+// The chain of levels bounds it, an island's latency whatever the others do; next the fetching of its code (the first
+// pass through any part of it costs several times the later ones, most with every SM at it). B200, at an island's 350
+// contacts in 41 to 57 levels, in 1,000 cycles: the levels 33 by one thread (95 a contact), 20 so; the chain 68 to 89 with the
+// records read from global memory and the law's cases branched on, 34 so; the nodes' forces into the slots 16, 7 so.
+// A launch for 128 head-on pairs of vehicles 100 us, 63 so; for two crashing trusses (46 contacts) 10.1 and 6.5 us.
 __device__ void collide_island_global(const float4* __restrict__ nd, const int4* __restrict__ info, Body* __restrict__ bodies, Contacts C,
                                       float4* __restrict__ Fs, int root, int off, int cnt);
 
-constexpr int kCollideThreads = 256;
-constexpr int kSlotBits = 13, kSlots = 1 << kSlotBits; // force slots (distinct contact nodes an island)
-constexpr int kRecChunk = 512;                          // contact records formed at a time
-constexpr int kSlotPad = 8;                             // slot levels past the slots (kSlots: a level that stays 0)
-constexpr int kStage = 6144;                            // contacts of an island that runs whole (slots, levels staged)
+constexpr int kCollideThreads = 512;
+constexpr int kKeyBits = 13, kKeys = 1 << kKeyBits; // the hash of an island's contact nodes
+constexpr int kSlots = kKeys / 2;                   // force slots, one a distinct contact node (the hash at most half full)
+constexpr int kSlotPad = 8;                         // slot levels past the slots (kSlots: a level that stays 0)
+constexpr int kRecChunk = 448;                      // contact records formed at a time where an island does not run whole
+constexpr int kStage = 6144;                        // contacts of an island that runs whole
+constexpr int kParMax = 2048;                       // ... whose levels are found from lists
+constexpr int kSmall = 448;                         // ... a thread each, the records of all at once; the last warps stay free
 
 struct alignas(16) ContactRec {
     int sa, sb[3];        // force slots of the node and the triangle's corners
@@ -418,84 +427,103 @@ struct alignas(16) ContactRec {
                           // | soft (drag, buoyancy) << 6 | pen >= soft depth << 7
 };
 
-__device__ __forceinline__ int slot_hash(int key) { return (int)(((uint32_t)key * 2654435761u) >> (32 - kSlotBits)); }
-__device__ __forceinline__ int slot_find(const int* keys, int key) {
-    int h = slot_hash(key);
-    while (keys[h] != key) h = (h + 1) & (kSlots - 1);
+struct alignas(16) ContactRecPad { // (a stride whose rows fall in distinct banks)
+    ContactRec r;
+    int4 pad;
+};
+// the work area of k_collide (bytes): a small island's records, then its contacts' nearest earlier ones, levels, order and
+// level starts - the lists of the levels in the records' place; otherwise up to kStage contacts' slots and levels, or
+// up to kParMax contacts' slots, nearest earlier ones, list entries, levels and the list heads
+constexpr int kWorkPred = kSmall * (int)sizeof(ContactRecPad), kWorkLv = kWorkPred + 8 * kSmall, kWorkOrd = kWorkLv + 2 * kSmall + 16,
+              kWorkLe = kWorkOrd + 2 * kSmall, kCollideWork = kWorkLe + 4 * kSmall + 16;
+constexpr int kWorkParPred = 8 * kParMax, kWorkParNext = 16 * kParMax, kWorkLv16 = 8 * kStage, kWorkParHead = kWorkLv16 + 2 * kParMax + 16;
+static_assert(kCollideWork >= 10 * kStage && kCollideWork >= kWorkParHead + 4 * kSlots && kWorkParNext + 8 * kParMax <= kWorkLv16, "the work area's uses");
+
+__device__ __forceinline__ int key_hash(int key) { return (int)(((uint32_t)key * 2654435761u) >> (32 - kKeyBits)); }
+__device__ __forceinline__ int key_find(const int* keys, int key) {
+    int h = key_hash(key);
+    while (keys[h] != key) h = (h + 1) & (kKeys - 1);
     return h;
 }
 
 // One contact of the chain on the forces in the slots: only the force-dependent arithmetic, the reference's operations
 // in its order (contact_force<1, 3> / hull_push_out<3> and primitive_collision, world.cpp:59-120,
-// static_world.cpp:8-51, split at their force-independent parts, which the record holds)
-__device__ __forceinline__ void apply_contact(const ContactRec& R, float* fx, float* fy, float* fz, const GroundModel& gm) {
+// static_world.cpp:8-51, split at their force-independent parts, which the record holds). The kinds and the stick and
+// slip cases are chosen at the end, not branched on: a warp's lanes hold different ones, and the chain waits for each.
+__device__ __forceinline__ void apply_contact(const ContactRec& R, float4* F_, const GroundModel& gm) {
     const int kind = R.kind & 15;
     const bool ma = R.kind & 16, mb = R.kind & 32;
-    v3 FA = V(fx[R.sa], fy[R.sa], fz[R.sa]);
-    v3 FB[3];
-    for (int q = 0; q < 3; q++) FB[q] = V(fx[R.sb[q]], fy[R.sb[q]], fz[R.sb[q]]);
+    const float4 a4 = F_[R.sa], b40 = F_[R.sb[0]], b41 = F_[R.sb[1]], b42 = F_[R.sb[2]];
+    const v3 FA = V(a4.x, a4.y, a4.z), FB[3] = {V(b40.x, b40.y, b40.z), V(b41.x, b41.y, b41.z), V(b42.x, b42.y, b42.z)};
     v3 acc = V(0, 0, 0);
-    if (ma) acc = acc + FA * R.ca;
-    for (int q = 0; q < 3; q++)
-        if (mb) acc = acc - FB[q] * R.cb[q];
+    const v3 acca = acc + FA * R.ca;
+    if (ma) acc = acca;
+    v3 accb = acc;
+#pragma unroll
+    for (int q = 0; q < 3; q++) accb = accb - FB[q] * R.cb[q];
+    if (mb) acc = accb;
     const v3 nrm = V(R.nx, R.ny, R.nz);
-    if (kind == 3) {
-        const float fn = R.rsub - dot(acc, nrm) * R.m;
-        if (fn > 0) {
-            const v3 f = nrm * fn;
-            if (ma) FA = FA + f;
-            if (mb)
-                for (int q = 0; q < 3; q++) FB[q] = FB[q] - f * R.wb[q];
-        }
-    } else {
-        const v3 f_rel = acc * R.m;
-        const v3 F = kind == 1 ? f_rel : neg(f_rel);
+    // kind 3: along the normal
+    const float fn = R.rsub - dot(acc, nrm) * R.m;
+    // kinds 1 and 2: primitive_collision (static_world.cpp:8-51) with its force-independent terms from the record
+    v3 F = acc * R.m;
+    if (kind != 1) F = neg(F);
+    v3 out = V(0, 0, 0);
+    const float Vn = R.Vn, Fn = dot(F, nrm);
+    if (R.kind & 64) {
         const v3 vel = V(R.vx, R.vy, R.vz);
-        // primitive_collision (static_world.cpp:8-51) with its force-independent terms from the record
-        v3 out = V(0, 0, 0);
-        const float Vn = R.Vn, Fn = dot(F, nrm);
-        if (R.kind & 64) {
-            out = out + vel * R.dragf;
-            float Fb = R.fb0;
-            if (Vn >= 0 && Fn < 0 && Fb > -Fn) Fb = -Fn;
-            out = out + nrm * Fb;
-        }
-        if (R.kind & 128) {
-            float Rn = -Fn;
-            if (Vn < 0) Rn -= R.rsub;
-            if (Rn > 0) {
-                const v3 slipF = F - nrm * Fn;
-                const v3 slip = V(R.sx, R.sy, R.sz);
-                const float G = Rn * gm.strength * R.fric;
-                if (R.sv < gm.va && G > 0 && length(slipF) <= gm.ms * G)
-                    out = out + (nrm * Rn - slip * smin(gm.ms * G * R.e1, R.stop) - slipF);
-                else
-                    out = out + (nrm * Rn - slip * smin(R.gsum * G, smax(0.0f, R.stop + dot(slipF, slip))));
-            }
-        }
-        if (kind == 2) {
-            for (int q = 0; q < 3; q++) FB[q] = FB[q] + out * R.wb[q];
-        } else {
-            FA = FA + out * 1.0f;
-            if (mb)
-                for (int q = 0; q < 3; q++) FB[q] = FB[q] - out * R.wb[q];
-        }
+        out = out + vel * R.dragf;
+        float Fb = R.fb0;
+        if (Vn >= 0 && Fn < 0 && Fb > -Fn) Fb = -Fn;
+        out = out + nrm * Fb;
     }
-    fx[R.sa] = FA.x, fy[R.sa] = FA.y, fz[R.sa] = FA.z;
-    for (int q = 0; q < 3; q++) fx[R.sb[q]] = FB[q].x, fy[R.sb[q]] = FB[q].y, fz[R.sb[q]] = FB[q].z;
+    float Rn = -Fn;
+    if (Vn < 0) Rn -= R.rsub;
+    const v3 slipF = F - nrm * Fn, slip = V(R.sx, R.sy, R.sz), nR = nrm * Rn;
+    const float G = Rn * gm.strength * R.fric;
+    const bool on = (R.kind & 128) && Rn > 0;
+    const v3 slide = nR - slip * smin(R.gsum * G, smax(0.0f, R.stop + dot(slipF, slip)));
+    v3 hard = slide;
+    if (on && R.sv < gm.va && G > 0 && length(slipF) <= gm.ms * G) hard = nR - slip * smin(gm.ms * G * R.e1, R.stop) - slipF;
+    const v3 sum = out + hard;
+    if (on) out = sum;
+    if (kind == 3) out = nrm * fn;
+    const bool toA = kind == 3 ? fn > 0 && ma : kind == 1, toB = kind == 3 ? fn > 0 && mb : kind == 2 || mb;
+    if (kind == 2) out = neg(out); // (FB + out w as FB - (-out) w: the same bits)
+    if (toA) F_[R.sa] = make_float4(FA.x + out.x, FA.y + out.y, FA.z + out.z, 0.0f);
+    if (toB)
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const v3 f = FB[q] - out * R.wb[q];
+            F_[R.sb[q]] = make_float4(f.x, f.y, f.z, 0.0f);
+        }
 }
 
-// One contact's record (pair i of the island; kind 0 where the law gives it no force): its slots, the accumulation
-// weights and every force-independent term of the law, and the wake requests of its sleeping sides. True when it is a
-// contact (counted).
-__device__ __forceinline__ bool form_record(ContactRec& R, int i, const float4* __restrict__ nd, const int4* __restrict__ info, Body* __restrict__ bodies,
-                                            const Contacts& C, const int* keys, const GroundModel& gm, float dt) {
+// What a contact's record is formed from
+struct ContactIn {
+    int2 pr;
+    int4 tr;
+    float4 ha, hb, P[4], Vv[4]; // (the node's and its triangle's corners')
+    int4 ina;
+};
+__device__ __forceinline__ void load_contact(ContactIn& I, int i, const float4* nd, const int4* __restrict__ info, const Contacts& C) {
+    I.ha = C.hit_a[i], I.hb = C.hit_b[i];
+    I.pr = C.pairs[i];
+    I.tr = C.tri[I.pr.y];
+    I.ina = info[I.pr.x];
+    const int at[4] = {I.pr.x, I.tr.x, I.tr.y, I.tr.z};
+#pragma unroll
+    for (int q = 0; q < 4; q++) I.P[q] = nd[2 * at[q]], I.Vv[q] = nd[2 * at[q] + 1];
+}
+
+// One contact's record (kind 0 where the law gives it no force; sl: its slots): the accumulation weights and every
+// force-independent term of the law, and the wake requests of its sleeping sides. True when it is a contact (counted).
+__device__ __forceinline__ bool form_record(ContactRec& R, const ContactIn& I, const int* sl, Body* __restrict__ bodies, const Contacts& C,
+                                            const GroundModel& gm, float dt) {
     R.kind = 0;
-    const float4 hb4 = C.hit_b[i];
-    const float4 ha = C.hit_a[i];
-    const int2 pr = C.pairs[i];
-    const int4 tr = C.tri[pr.y];
-    Body& bn = bodies[info[pr.x].w];
+    const float4 hb4 = I.hb, ha = I.ha;
+    const int4 tr = I.tr;
+    Body& bn = bodies[I.ina.w];
     Body& bt = bodies[tr.w >> 8];
     // movable (world.cpp:2983-2993): a sleeping side is immovable and asks to wake when the other moves
     bool ma = true, mb = true;
@@ -507,21 +535,18 @@ __device__ __forceinline__ bool form_record(ContactRec& R, int i, const float4* 
         if (sqrtf(bn.acc_v2) > smax(C.wake_speed, bn.sleep_speed) * 1.0f) bt.wake_request = 1;
         mb = false;
     }
-    const int ia = pr.x, ib[3] = {tr.x, tr.y, tr.z};
     const float wb[3] = {ha.x, ha.y, ha.z};
     const v3 n = V(hb4.x, hb4.y, hb4.z);
     const float pen = ha.w;
-    const float4 pa = nd[2 * ia], va4 = nd[2 * ia + 1];
-    const v3 Av = V(va4.x, va4.y, va4.z);
-    const float Aim = pa.w;
+    const v3 Av = V(I.Vv[0].x, I.Vv[0].y, I.Vv[0].z);
+    const float Aim = I.P[0].w;
     v3 Bv[3];
     float Bim[3];
-    for (int q = 0; q < 3; q++) {
-        const float4 pq = nd[2 * ib[q]], vq = nd[2 * ib[q] + 1];
-        Bv[q] = V(vq.x, vq.y, vq.z), Bim[q] = pq.w;
-    }
-    R.sa = slot_find(keys, ia);
-    for (int q = 0; q < 3; q++) R.sb[q] = slot_find(keys, ib[q]), R.wb[q] = wb[q], R.cb[q] = wb[q] * Bim[q];
+#pragma unroll
+    for (int q = 0; q < 3; q++) Bv[q] = V(I.Vv[q + 1].x, I.Vv[q + 1].y, I.Vv[q + 1].z), Bim[q] = I.P[q + 1].w;
+    R.sa = sl[0];
+#pragma unroll
+    for (int q = 0; q < 3; q++) R.sb[q] = sl[q + 1], R.wb[q] = wb[q], R.cb[q] = wb[q] * Bim[q];
     const int mv = (ma ? 16 : 0) | (mb ? 32 : 0);
     if (!(tr.w & TF_TWO_SIDED) && pen > bn.crad) {
         // hull_push_out<3> (world.cpp:97-118): behind a hull's face
@@ -538,8 +563,7 @@ __device__ __forceinline__ bool form_record(ContactRec& R, int i, const float4* 
     } else {
         // contact_force<1, 3> (world.cpp:59-92), the node's weight 1; a tyre node grips with its own friction
         // (world.cpp:3013)
-        const int4 ina = info[ia];
-        const float fric = ((uint32_t)ina.x & NF_TYRE) ? __int_as_float(ina.y) : 0.8f * smin(bn.cfric, bt.cfric);
+        const float fric = ((uint32_t)I.ina.x & NF_TYRE) ? __int_as_float(I.ina.y) : 0.8f * smin(bn.cfric, bt.cfric);
         float W = 0;
         if (ma) W += 1.0f * 1.0f * Aim;
         if (mb)
@@ -575,15 +599,106 @@ __device__ __forceinline__ bool form_record(ContactRec& R, int i, const float4* 
     return true;
 }
 
+// One warp: each contact's level from its nearest earlier contacts (pred: at each node, n where there is none; lv[n] 0),
+// 32 contacts at a time - those before the 32 have their levels, those among them are passed round until none moves.
+// Returns the deepest level.
+__device__ __forceinline__ int contact_levels(int n, const ushort4* pred, unsigned short* lv) {
+    const int lane = threadIdx.x & 31;
+    int deepest = 0;
+    if (lane == 0) lv[n] = 0;
+    __syncwarp();
+#pragma unroll 1
+    for (int c = 0; c < n; c += 32) {
+        const int j = c + lane;
+        const ushort4 e4 = j < n ? pred[j] : make_ushort4((unsigned short)n, (unsigned short)n, (unsigned short)n, (unsigned short)n);
+        const int e[4] = {e4.x, e4.y, e4.z, e4.w};
+        int l = 0;
+        bool here[4], any = false;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            here[q] = e[q] >= c && e[q] < n;
+            any |= here[q];
+            if (!here[q]) l = max(l, (int)lv[e[q]]);
+        }
+        l++;
+        if (__any_sync(0xffffffffu, any)) {
+            int before;
+#pragma unroll 1
+            do {
+                before = l;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int v = __shfl_sync(0xffffffffu, before, e[q] - c) + 1;
+                    if (here[q]) l = max(l, v);
+                }
+            } while (__any_sync(0xffffffffu, l != before));
+        }
+        if (j < n) lv[j] = (unsigned short)l, deepest = max(deepest, l);
+        __syncwarp();
+    }
+    return __reduce_max_sync(0xffffffffu, deepest);
+}
+// One warp: the contacts by level in ord (a level's in any order: they share no node); le[L]: level L's start, 1 <= L <=
+// depth + 1
+__device__ __forceinline__ void sort_by_level(int n, int depth, const unsigned short* lv, int* le, unsigned short* ord) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int l = lane; l < depth + 3; l += 32) le[l] = 0;
+    __syncwarp();
+#pragma unroll 1
+    for (int j = lane; j < n; j += 32) atomicAdd(&le[lv[j]], 1);
+    __syncwarp();
+    int carry = 0;
+#pragma unroll 1
+    for (int c = 0; c < depth + 2; c += 32) {
+        const int l = c + lane;
+        int x = l < depth + 2 ? le[l] : 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (l < depth + 2) le[l] = carry + x;
+        carry += __shfl_sync(0xffffffffu, x, 31);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int j = lane; j < n; j += 32) ord[atomicSub(&le[lv[j]], 1) - 1] = (unsigned short)j;
+    __syncwarp();
+}
+// One warp: the contacts at places p .. end of the order, level after level (L: the first's), a lane a contact; the next
+// contacts' records (at(place)) loaded while these run
+template <class At>
+__device__ __forceinline__ void run_levels(int p, int end, int& L, const int* le, At at, float4* F, const GroundModel& gm) {
+    const int lane = threadIdx.x & 31;
+    int n = p < end ? min(32, min(le[L + 1], end) - p) : 0, n2;
+    auto next = [&]() { // the contacts after these
+        const int pn = p + n;
+        if (pn == le[L + 1]) L++;
+        n2 = pn < end ? min(32, min(le[L + 1], end) - pn) : 0;
+        p = pn;
+    };
+    ContactRec cur, nxt;
+    if (lane < n) cur = at(p + lane);
+#pragma unroll 1
+    while (n > 0) {
+        const bool on = lane < n && (cur.kind & 15);
+        next();
+        if (lane < n2) nxt = at(p + lane);
+        if (on) apply_contact(cur, F, gm);
+        __syncwarp();
+        cur = nxt, n = n2;
+    }
+}
+
 __global__ void __launch_bounds__(kCollideThreads, 1) k_collide(const float4* __restrict__ nd, const int4* __restrict__ info, Body* __restrict__ bodies,
                                                             int nbodies, Contacts C, float4* __restrict__ Fs) {
     extern __shared__ __align__(16) unsigned char csm[];
-    int* keys = reinterpret_cast<int*>(csm);
-    float* fx = reinterpret_cast<float*>(keys + kSlots);
-    float* fy = fx + kSlots;
-    float* fz = fy + kSlots;
-    ContactRec* rec = reinterpret_cast<ContactRec*>(fz + kSlots);
-    unsigned short* slot_lvl = reinterpret_cast<unsigned short*>(rec + kRecChunk); // per slot: its latest contact's level
+    int* keys = reinterpret_cast<int*>(csm);                                   // the hash: a node, or -1
+    unsigned short* cid = reinterpret_cast<unsigned short*>(keys + kKeys);     // ... its slot
+    float4* F = reinterpret_cast<float4*>(cid + kKeys);                        // per slot: the node's force
+    int* unode = reinterpret_cast<int*>(F + kSlots);                           // per slot: the node
+    unsigned short* slot_lvl = reinterpret_cast<unsigned short*>(unode + kSlots); // per slot: its latest contact's level
+    unsigned char* work = reinterpret_cast<unsigned char*>(slot_lvl + kSlots + kSlotPad);
     __shared__ int used, overflow, ncontacts, s_depth;
     const int root = blockIdx.x, tid = threadIdx.x;
     pdl_wait();
@@ -593,9 +708,8 @@ __global__ void __launch_bounds__(kCollideThreads, 1) k_collide(const float4* __
     const int off = C.isl_poff[root];
     const float dt = C.dt;
     const GroundModel& gm = c_ground[3]; // SURF_CONCRETE
-    for (int h = tid; h < kSlots; h += kCollideThreads) keys[h] = -1, slot_lvl[h] = 0;
-    if (tid < kSlotPad) slot_lvl[kSlots + tid] = 0;
-    if (tid == 0) used = 0, overflow = 0, ncontacts = 0;
+    for (int h = tid; h < kKeys / 4; h += kCollideThreads) reinterpret_cast<int4*>(keys)[h] = make_int4(-1, -1, -1, -1);
+    if (tid == 0) used = 0, overflow = 0, ncontacts = 0, s_depth = 0;
     __shared__ int s_scan[32];
     // 0. the island's contacts (its pairs with a hit), in pair order, into hidx[off ...): a run of pairs a thread
     int nh_all;
@@ -618,9 +732,44 @@ __global__ void __launch_bounds__(kCollideThreads, 1) k_collide(const float4* __
             for (uint32_t m = word(w); m; m &= m - 1) C.hidx[at++] = ((w0 + w) << 5) + __ffs(m) - 1;
     }
     __syncthreads();
-    // 1. the contacts' nodes into slots (four contacts a thread at a time: their loads overlap)
-    for (int j0 = tid; j0 < nh_all; j0 += 4 * kCollideThreads) {
+    if (nh_all == 0) return;
+    const bool whole = nh_all <= C.whole_max, small = whole && nh_all <= kSmall;
+    ushort4* sq = reinterpret_cast<ushort4*>(work); // (whole, not small) per contact: its slots
+    // 1. the contacts' nodes into slots
+    auto insert = [&](int node) { // (the node's place in the hash)
+        int h = key_hash(node);
+        for (int probe = 0;; probe++) {
+            if (probe >= kKeys / 2 || *(volatile int*)&overflow) {
+                overflow = 1;
+                break;
+            }
+            int prev = *(volatile int*)&keys[h];
+            if (prev == -1) {
+                prev = atomicCAS(&keys[h], -1, node);
+                if (prev == -1) {
+                    const int at = atomicAdd(&used, 1);
+                    if (at >= kSlots) overflow = 1; // (kept at most half full: short probes)
+                    else cid[h] = (unsigned short)at, unode[at] = node;
+                    break;
+                }
+            }
+            if (prev == node) break;
+            h = (h + 1) & (kKeys - 1);
+        }
+        return h;
+    };
+    ContactIn own; // (small) the thread's contact
+    const bool mine = small && tid < nh_all;
+    unsigned long long places = 0; // (its nodes' places, 16 bits each)
+    if (mine) {
+        load_contact(own, C.hidx[off + tid], nd, info, C);
+#pragma unroll 1
+        for (int q = 0; q < 4; q++)
+            places |= (unsigned long long)insert(q == 0 ? own.pr.x : q == 1 ? own.tr.x : q == 2 ? own.tr.y : own.tr.z) << (16 * q);
+    }
+    for (int j0 = tid; !small && j0 < nh_all; j0 += 4 * kCollideThreads) { // (four contacts a thread at a time: their loads overlap)
         int nodes4[4][4];
+#pragma unroll
         for (int u = 0; u < 4; u++) {
             const int j = j0 + u * kCollideThreads;
             nodes4[u][0] = -1;
@@ -629,25 +778,12 @@ __global__ void __launch_bounds__(kCollideThreads, 1) k_collide(const float4* __
             const int4 tr = C.tri[pr.y];
             nodes4[u][0] = pr.x, nodes4[u][1] = tr.x, nodes4[u][2] = tr.y, nodes4[u][3] = tr.z;
         }
+#pragma unroll
         for (int u = 0; u < 4; u++) {
             if (nodes4[u][0] < 0) continue;
-            for (int q = 0; q < 4; q++) {
-                const int node = nodes4[u][q];
-                int h = slot_hash(node);
-                for (int probe = 0;; probe++) {
-                    if (probe >= kSlots / 2 || overflow) {
-                        overflow = 1;
-                        break;
-                    }
-                    const int prev = atomicCAS(&keys[h], -1, node);
-                    if (prev == -1) {
-                        if (atomicAdd(&used, 1) >= kSlots / 2) overflow = 1; // (kept at most half full: short probes)
-                        break;
-                    }
-                    if (prev == node) break;
-                    h = (h + 1) & (kSlots - 1);
-                }
-            }
+            const ushort4 h4 = make_ushort4((unsigned short)insert(nodes4[u][0]), (unsigned short)insert(nodes4[u][1]),
+                                            (unsigned short)insert(nodes4[u][2]), (unsigned short)insert(nodes4[u][3]));
+            if (whole) sq[j0 + u * kCollideThreads] = h4;
         }
     }
     __syncthreads();
@@ -655,95 +791,135 @@ __global__ void __launch_bounds__(kCollideThreads, 1) k_collide(const float4* __
         if (tid == 0) collide_island_global(nd, info, bodies, C, Fs, root, off, cnt);
         return;
     }
-    for (int h = tid; h < kSlots; h += kCollideThreads)
-        if (keys[h] >= 0) {
-            const float4 f = Fs[keys[h]];
-            fx[h] = f.x, fy[h] = f.y, fz[h] = f.z;
-        }
-    // The island's contacts at once where they fit (kStage at most, and the substep's record buffer has room): their
-    // records in global memory, their slots and levels staged in the record chunk's shared memory - levels over the
-    // whole island, with no barrier between chunks. Otherwise kRecChunk at a time, below.
-    __shared__ int s_base;
-    if (tid == 0) {
-        int b = -1;
-        if (nh_all > 0 && nh_all <= C.whole_max) {
-            b = atomicAdd(C.crec_n, nh_all);
-            if (b + nh_all > C.crec_cap) b = -1;
-        }
-        s_base = b;
+    const int nused = used;
+    for (int u = tid; u < nused; u += kCollideThreads) {
+        const float4 f = Fs[unode[u]];
+        F[u] = make_float4(f.x, f.y, f.z, 0.0f);
     }
-    __syncthreads();
-    if (s_base >= 0) {
-        const int base = s_base;
-        ushort4* sq = reinterpret_cast<ushort4*>(rec);                          // per contact: its slots
-        unsigned short* lv16 = reinterpret_cast<unsigned short*>(sq + kStage); // per contact: its level
-        // 2. each contact's slots
+    const bool last = tid >= kCollideThreads - 32; // (the warp of the levels and the chain)
+    int L = 1;
+    auto slots_of = [&](const ContactIn& I, int* sl) {
+        sl[0] = cid[key_find(keys, I.pr.x)], sl[1] = cid[key_find(keys, I.tr.x)], sl[2] = cid[key_find(keys, I.tr.y)], sl[3] = cid[key_find(keys, I.tr.z)];
+    };
+    // contact j's nearest earlier contacts, from its nodes' lists (the four side by side)
+    auto nearest = [&](int j, ushort4 h, const int* head, const unsigned short* next) {
+        int e[4] = {head[h.x], head[h.y], head[h.z], head[h.w]}, best[4] = {-1, -1, -1, -1};
+        while ((e[0] & e[1] & e[2] & e[3]) != 0xffff)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (e[q] == 0xffff) continue;
+                const int o = e[q] >> 2;
+                if (o < j && o > best[q]) best[q] = o;
+                e[q] = next[e[q]];
+            }
+        auto at = [&](int q) { return (unsigned short)(best[q] < 0 ? nh_all : best[q]); };
+        return make_ushort4(at(0), at(1), at(2), at(3));
+    };
+    auto list = [&](int j, ushort4 h, int* head, unsigned short* next) {
+        next[4 * j] = (unsigned short)atomicExch(&head[h.x], 4 * j), next[4 * j + 1] = (unsigned short)atomicExch(&head[h.y], 4 * j + 1);
+        next[4 * j + 2] = (unsigned short)atomicExch(&head[h.z], 4 * j + 2), next[4 * j + 3] = (unsigned short)atomicExch(&head[h.w], 4 * j + 3);
+    };
+    if (small) {
+        int* head = reinterpret_cast<int*>(work);                                                      // per slot: its last-listed entry
+        unsigned short* next = reinterpret_cast<unsigned short*>(work + 16 * kSmall);                  // per entry: the one listed before
+        ushort4* pred = reinterpret_cast<ushort4*>(work + kWorkPred);
+        unsigned short *lv = reinterpret_cast<unsigned short*>(work + kWorkLv), *ord = reinterpret_cast<unsigned short*>(work + kWorkOrd);
+        int* le = reinterpret_cast<int*>(work + kWorkLe);
+        ContactRecPad* rec = reinterpret_cast<ContactRecPad*>(work);
+        for (int u = tid; u < nused; u += kCollideThreads) head[u] = 0xffff;
+        const ushort4 h = mine ? make_ushort4(cid[places & 0xffff], cid[(places >> 16) & 0xffff], cid[(places >> 32) & 0xffff], cid[places >> 48])
+                               : make_ushort4(0, 0, 0, 0);
+        __syncthreads();
+        if (mine) list(tid, h, head, next);
+        __syncthreads();
+        if (mine) pred[tid] = nearest(tid, h, head, next);
+        __syncthreads();
+        // 2. the levels and the order by the last warp, 3. the records by the others
+        if (last) {
+            const int depth = contact_levels(nh_all, pred, lv);
+            sort_by_level(nh_all, depth, lv, le, ord);
+        } else if (mine) {
+            ContactRec R;
+            const int sl[4] = {h.x, h.y, h.z, h.w};
+            if (form_record(R, own, sl, bodies, C, gm, dt)) atomicAdd(&ncontacts, 1);
+            rec[tid].r = R;
+        }
+        __syncthreads();
+        // 4. the chain
+        if (last) run_levels(0, nh_all, L, le, [&](int p) { return rec[ord[p]].r; }, F, gm);
+    } else if (whole) {
+        unsigned short* lv16 = reinterpret_cast<unsigned short*>(work + kWorkLv16); // per contact: its level
         for (int j = tid; j < nh_all; j += kCollideThreads) {
-            const int2 pr = C.pairs[C.hidx[off + j]];
-            const int4 tr = C.tri[pr.y];
-            sq[j] = make_ushort4((unsigned short)slot_find(keys, pr.x), (unsigned short)slot_find(keys, tr.x), (unsigned short)slot_find(keys, tr.y),
-                                 (unsigned short)slot_find(keys, tr.z));
+            const ushort4 h = sq[j];
+            sq[j] = make_ushort4(cid[h.x], cid[h.y], cid[h.z], cid[h.w]);
         }
-        __syncthreads();
-        // 3. the levels (one thread, in pair order; a pair the law gives no force keeps its place, which only orders
-        // more) while the other warps form the records
-        if (tid == 0) {
-            int depth = 0;
-            ushort4 h = sq[0];
-            for (int j = 0; j < nh_all; j++) {
-                const ushort4 hn = sq[min(j + 1, nh_all - 1)]; // (loaded before this contact's levels are stored)
-                const int l = max(max((int)slot_lvl[h.x], (int)slot_lvl[h.y]), max((int)slot_lvl[h.z], (int)slot_lvl[h.w])) + 1;
-                slot_lvl[h.x] = slot_lvl[h.y] = slot_lvl[h.z] = slot_lvl[h.w] = (unsigned short)l;
-                lv16[j] = (unsigned short)l;
-                depth = max(depth, l);
-                h = hn;
+        // 2. the levels (a pair the law gives no force keeps its place, which only orders more)
+        unsigned short* ord = reinterpret_cast<unsigned short*>(work); // (over the slots, done with)
+        const int ord_bytes = (2 * nh_all + 15) & ~15;
+        int* le = reinterpret_cast<int*>(work + ord_bytes);
+        if (nh_all <= kParMax) {
+            int* head = reinterpret_cast<int*>(work + kWorkParHead);
+            unsigned short* next = reinterpret_cast<unsigned short*>(work + kWorkParNext);
+            ushort4* pred = reinterpret_cast<ushort4*>(work + kWorkParPred);
+            for (int u = tid; u < nused; u += kCollideThreads) head[u] = 0xffff;
+            __syncthreads();
+            for (int j = tid; j < nh_all; j += kCollideThreads) list(j, sq[j], head, next);
+            __syncthreads();
+            for (int j = tid; j < nh_all; j += kCollideThreads) pred[j] = nearest(j, sq[j], head, next);
+            __syncthreads();
+            if (last) {
+                const int depth = contact_levels(nh_all, pred, lv16);
+                if ((tid & 31) == 0) s_depth = depth;
             }
-            s_depth = depth;
-        } else if (tid >= 32) {
-            for (int j = tid - 32; j < nh_all; j += kCollideThreads - 32) {
-                ContactRec R;
-                if (form_record(R, C.hidx[off + j], nd, info, bodies, C, keys, gm, dt)) atomicAdd(&ncontacts, 1);
-                C.crec[base + j] = R;
-            }
-        }
-        __syncthreads();
-        // by level: counts, ends (a running sum), places (a level's contacts in any order: they share no node)
-        const int depth = s_depth;
-        unsigned short* ord = reinterpret_cast<unsigned short*>(rec); // (over the slots, done with)
-        int* le = reinterpret_cast<int*>(ord + kStage);
-        for (int l = tid; l < depth + 3; l += kCollideThreads) le[l] = 0;
-        __syncthreads();
-        for (int j = tid; j < nh_all; j += kCollideThreads) atomicAdd(&le[lv16[j]], 1);
-        __syncthreads();
-        block_scan_incl_inplace(le, depth + 1, s_scan);
-        __syncthreads();
-        if (tid == 0) le[depth + 1] = le[depth];
-        __syncthreads();
-        for (int j = tid; j < nh_all; j += kCollideThreads) ord[atomicSub(&le[lv16[j]], 1) - 1] = (unsigned short)j; // (le[L]: level L's start)
-        __syncthreads();
-        // 4. the chain: one warp, level after level, a lane a contact; the next level's records loaded while one runs
-        if (tid < 32) {
-            const ContactRec* __restrict__ cr = C.crec + base;
-            int s0 = le[1], e0 = le[2];
-            bool has = s0 + tid < e0;
-            ContactRec cur;
-            if (has) cur = cr[ord[s0 + tid]];
-            for (int L = 1; L <= depth; L++) {
-                const int s1 = le[L + 1], e1 = L < depth ? le[L + 2] : s1;
-                const bool hasn = s1 + tid < e1;
-                ContactRec nxt;
-                if (hasn) nxt = cr[ord[s1 + tid]];
-                if (has && (cur.kind & 15)) apply_contact(cur, fx, fy, fz, gm);
-                for (int k = s0 + tid + 32; k < e0; k += 32) {
-                    const ContactRec R = cr[ord[k]];
-                    if (R.kind & 15) apply_contact(R, fx, fy, fz, gm);
+        } else {
+            for (int u = tid; u < nused; u += kCollideThreads) slot_lvl[u] = 0;
+            __syncthreads();
+            if (tid == kCollideThreads - 32) {
+                int depth = 0;
+                ushort4 h = sq[0];
+                for (int j = 0; j < nh_all; j++) {
+                    const ushort4 hn = sq[min(j + 1, nh_all - 1)]; // (loaded before this contact's levels are stored)
+                    const int l = max(max((int)slot_lvl[h.x], (int)slot_lvl[h.y]), max((int)slot_lvl[h.z], (int)slot_lvl[h.w])) + 1;
+                    slot_lvl[h.x] = slot_lvl[h.y] = slot_lvl[h.z] = slot_lvl[h.w] = (unsigned short)l;
+                    lv16[j] = (unsigned short)l;
+                    depth = max(depth, l);
+                    h = hn;
                 }
-                __syncwarp();
-                cur = nxt, has = hasn, s0 = s1, e0 = e1;
+                s_depth = depth;
             }
+        }
+        __syncthreads();
+        const int le_bytes = (4 * (s_depth + 3) + 15) & ~15; // (with the order below the lists and levels: 6 bytes a contact and 44)
+        if (last) sort_by_level(nh_all, s_depth, lv16, le, ord);
+        __syncthreads();
+        // 3, 4. the records of half a buffer formed by the other warps while the last runs the half before
+        ContactRecPad* buf = reinterpret_cast<ContactRecPad*>(work + ord_bytes + le_bytes);
+        const int half = (int)((kCollideWork - ord_bytes - le_bytes) / sizeof(ContactRecPad)) / 2;
+        auto form = [&](int p0, int step) {
+            ContactRecPad* dst = buf + ((p0 / half) & 1) * half;
+            const int n = min(half, nh_all - p0);
+            for (int r = tid; r < n; r += step) {
+                ContactIn I;
+                ContactRec R;
+                int sl[4];
+                load_contact(I, C.hidx[off + ord[p0 + r]], nd, info, C);
+                slots_of(I, sl);
+                if (form_record(R, I, sl, bodies, C, gm, dt)) atomicAdd(&ncontacts, 1);
+                dst[r].r = R;
+            }
+        };
+        form(0, kCollideThreads);
+        __syncthreads();
+        for (int p0 = 0; p0 < nh_all; p0 += half) {
+            const ContactRecPad* src = buf + ((p0 / half) & 1) * half;
+            if (last) run_levels(p0, min(nh_all, p0 + half), L, le, [&](int p) { return src[p - p0].r; }, F, gm);
+            else if (p0 + half < nh_all) form(p0 + half, kCollideThreads - 32);
+            __syncthreads();
         }
     } else {
         // the island's contacts in pair order, kRecChunk at a time
+        ContactRec* rec = reinterpret_cast<ContactRec*>(work);
+        for (int h = tid; h < kSlots + kSlotPad; h += kCollideThreads) slot_lvl[h] = 0;
         __shared__ int order[kRecChunk], lend[kRecChunk + 3], lv[kRecChunk];
         __shared__ int4 sl[kRecChunk + 1]; // per record: its slots (kSlots x 4: not a contact)
         for (int c0 = 0; c0 < nh_all; c0 += kRecChunk) {
@@ -754,7 +930,11 @@ __global__ void __launch_bounds__(kCollideThreads, 1) k_collide(const float4* __
                 const int i = C.hidx[off + c0 + r];
                 ContactRec& R = rec[r];
                 sl[r] = make_int4(kSlots, kSlots, kSlots, kSlots); // (none: the slot whose level stays 0)
-                if (form_record(R, i, nd, info, bodies, C, keys, gm, dt)) {
+                ContactIn I;
+                int s4[4];
+                load_contact(I, i, nd, info, C);
+                slots_of(I, s4);
+                if (form_record(R, I, s4, bodies, C, gm, dt)) {
                     sl[r] = make_int4(R.sa, R.sb[0], R.sb[1], R.sb[2]);
                     atomicAdd(&ncontacts, 1);
                 }
@@ -785,7 +965,7 @@ __global__ void __launch_bounds__(kCollideThreads, 1) k_collide(const float4* __
             if (depth < 0) {
                 if (tid == 0)
                     for (int r = 0; r < nh; r++)
-                        if (lv[r]) apply_contact(rec[r], fx, fy, fz, gm);
+                        if (lv[r]) apply_contact(rec[r], F, gm);
             } else if (depth > 0) {
                 // by level: counts, ends (a running sum), places (each level's contacts in any order: they share no node)
                 for (int r = tid; r < nh; r += kCollideThreads)
@@ -805,8 +985,8 @@ __global__ void __launch_bounds__(kCollideThreads, 1) k_collide(const float4* __
                     for (int L = 1; L <= depth; L++) {
                         const int s1 = lend[L + 1], e1 = L < depth ? lend[L + 2] : s1;
                         const int rn = s1 + tid < e1 ? order[s1 + tid] : -1;
-                        if (rr >= 0) apply_contact(rec[rr], fx, fy, fz, gm);
-                        for (int k = s0 + tid + 32; k < e0; k += 32) apply_contact(rec[order[k]], fx, fy, fz, gm);
+                        if (rr >= 0) apply_contact(rec[rr], F, gm);
+                        for (int k = s0 + tid + 32; k < e0; k += 32) apply_contact(rec[order[k]], F, gm);
                         __syncwarp();
                         s0 = s1, e0 = e1, rr = rn;
                     }
@@ -820,16 +1000,16 @@ __global__ void __launch_bounds__(kCollideThreads, 1) k_collide(const float4* __
         }
     }
     __syncthreads();
-    // 4. the forces back
-    for (int h = tid; h < kSlots; h += kCollideThreads)
-        if (keys[h] >= 0) Fs[keys[h]] = make_float4(fx[h], fy[h], fz[h], 0.0f);
+    // 5. the forces back
+    for (int u = tid; u < nused; u += kCollideThreads) Fs[unode[u]] = F[u];
     if (tid == 0) {
         C.isl_contacts[root] += ncontacts;
         if (ncontacts) atomicAdd(&C.counters[1], ncontacts);
     }
 }
-constexpr size_t kCollideSmem = sizeof(int) * kSlots + 3 * sizeof(float) * kSlots + sizeof(ContactRec) * kRecChunk +
-                                sizeof(unsigned short) * (kSlots + kSlotPad);
+constexpr size_t kCollideSmem = sizeof(int) * kKeys + sizeof(unsigned short) * kKeys + sizeof(float4) * kSlots + sizeof(int) * kSlots +
+                                sizeof(unsigned short) * (kSlots + kSlotPad) + kCollideWork;
+static_assert(sizeof(ContactRec) * kRecChunk <= kCollideWork && sizeof(ContactRec) == 128, "the work area's uses");
 
 // The serial loop on global memory (the path of an island with more distinct contact nodes than the slots hold)
 __device__ void collide_island_global(const float4* __restrict__ nd, const int4* __restrict__ info, Body* __restrict__ bodies, Contacts C,

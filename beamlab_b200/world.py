@@ -77,7 +77,7 @@ class WorldSettings:
     fem_dense_front: int = 3
     tyre_grip: float = 1.0                    # WorldSettings::tyre_grip: a factor on the tyres' friction
     bulk_wait_s: float = 1.0                  # the beams kernel's bound on a wait for its bulk copies (0: runs out)
-    contact_whole_max: int = 6144             # an island's contacts run whole up to this many, else 512 at a time
+    contact_whole_max: int = 6144             # an island's contacts run whole up to this many, else 448 at a time
     # launch shapes (None: the tuned ones of beamlab_b200/tuned.json when present, else the library's defaults);
     # results do not depend on them
     force_block: int | None = None
