@@ -66,7 +66,6 @@ struct Contacts {
     int* bk_items;             // hashed nodes by bucket
     int* run_end;
     int* g_start;              // fast grids: each fast body's cells' starts (a pool of cell_cap)
-    int* g_fill;
     int* g_items;              // fast grids' nodes, each listed once, in the lowest cell of its travel
     float4* g_rec;             // ... in the same order: position, reach of its travel (|v| x travel)
     int* g_hi;                 // ... the highest cell of its travel (x | y << 8 | z << 16)

@@ -238,7 +238,7 @@ struct bl_gpu_ctx {
     DevBuf<int4> dtri, pt_cell;
     DevBuf<float> tri_rest2, ibox;
     DevBuf<int> parent, isl_live, isl_cnt, isl_nodes, isl_idx, isl_noff, isl_poff, isl_pcnt, isl_contacts, pair_total;
-    DevBuf<int> pt_node, pt_body, bk_start, bk_fill, bk_items, run_end, g_start, g_fill, g_items, counters;
+    DevBuf<int> pt_node, pt_body, bk_start, bk_fill, bk_items, run_end, g_start, g_items, counters;
     DevBuf<int2> pairs;
     DevBuf<float4> hit_a, hit_b;
     // the pair search's records, island states, queries and counters (bl_pair_search.cuh)
@@ -311,7 +311,7 @@ static void free_contacts(bl_gpu_ctx* c) {
     c->dtri.free_(), c->pt_cell.free_(), c->tri_rest2.free_(), c->ibox.free_(), c->parent.free_(), c->isl_live.free_();
     c->isl_cnt.free_(), c->isl_nodes.free_(), c->isl_idx.free_(), c->isl_noff.free_(), c->isl_poff.free_(), c->isl_pcnt.free_();
     c->isl_contacts.free_(), c->pair_total.free_(), c->pt_node.free_(), c->pt_body.free_(), c->bk_start.free_(), c->bk_fill.free_();
-    c->bk_items.free_(), c->run_end.free_(), c->g_start.free_(), c->g_fill.free_(), c->g_items.free_(), c->counters.free_();
+    c->bk_items.free_(), c->run_end.free_(), c->g_start.free_(), c->g_items.free_(), c->counters.free_();
     c->pairs.free_(), c->hit_a.free_(), c->hit_b.free_();
     c->g_rec.free_(), c->sb_pos.free_(), c->sb_cell.free_(), c->q_group.free_(), c->g_hi.free_(), c->q_count.free_(), c->sc.free_();
     c->q_chunk.free_(), c->ptmp.free_(), c->q_tmp.free_(), c->isl.free_(), c->hbits.free_(), c->hidx.free_();
@@ -999,7 +999,6 @@ static int commit_contacts(bl_gpu_ctx* c, std::vector<Body>& recs) {
     // (fast grids: the starts of every fast body's cells from one pool, the fill counters one grid per island)
     const int cell_cap = std::min(B, 512) * (kGridCells + 1);
     BL_CUDA(c, c->g_start.alloc((size_t)cell_cap));
-    BL_CUDA(c, c->g_fill.alloc((size_t)c->max_isl * (kGridCells + 1)));
     BL_CUDA(c, c->g_items.alloc(N));
     BL_CUDA(c, c->g_rec.alloc(N));
     BL_CUDA(c, c->g_hi.alloc(N));
@@ -1030,7 +1029,7 @@ static int commit_contacts(bl_gpu_ctx* c, std::vector<Body>& recs) {
     C.isl_noff = c->isl_noff.p, C.isl_poff = c->isl_poff.p, C.isl_pcnt = c->isl_pcnt.p, C.isl_contacts = c->isl_contacts.p;
     C.pair_total = c->pair_total.p, C.pairs = c->pairs.p, C.hit_a = c->hit_a.p, C.hit_b = c->hit_b.p, C.max_pairs = c->cfg.max_pairs;
     C.pt_node = c->pt_node.p, C.pt_body = c->pt_body.p, C.pt_cell = c->pt_cell.p, C.bk_start = c->bk_start.p, C.bk_fill = c->bk_fill.p;
-    C.bk_items = c->bk_items.p, C.run_end = c->run_end.p, C.g_start = c->g_start.p, C.g_fill = c->g_fill.p, C.g_items = c->g_items.p;
+    C.bk_items = c->bk_items.p, C.run_end = c->run_end.p, C.g_start = c->g_start.p, C.g_items = c->g_items.p;
     C.g_rec = c->g_rec.p, C.g_hi = c->g_hi.p, C.sb_cell = c->sb_cell.p, C.sb_pos = c->sb_pos.p, C.isl = c->isl.p;
     C.q_group = c->q_group.p, C.q_chunk = c->q_chunk.p, C.q_count = c->q_count.p, C.sc = c->sc.p;
     C.ptmp = c->ptmp.p, C.q_tmp = c->q_tmp.p, C.ptmp_cap = c->cfg.max_pairs;
@@ -1363,7 +1362,7 @@ static int64_t frame_launches(const bl_gpu_ctx* c, int n) {
     int64_t total = per * n + 3 + (c->NF > 0 ? 1 : 0); // (k_fem_begin a frame)
     if (c->contacts_on) {
         total += 1 + 3 * (int64_t)n; // k_islands; k_wake, k_detect, k_collide a substep
-        for (int k = 0; k < n; k++) total += rebuild_at(c, k) ? 4 : 0; // (k_rebuild, k_pair_count, k_pair_place, k_pair_write)
+        for (int k = 0; k < n; k++) total += rebuild_at(c, k) ? 5 : 0; // (k_rebuild, k_grids, k_pair_count, k_pair_place, k_pair_write)
     }
     return total;
 }
@@ -1499,6 +1498,7 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
                 cudaMemsetAsync(c->pair_total.p, 0, sizeof(int), s);
                 cudaMemsetAsync(c->sc.p, 0, 8 * sizeof(int), s);
                 k_rebuild<<<c->B, 1024, sizeof(RebuildShared), s>>>(c->dbodies.p, c->B, c->nd.p, c->info.p, CT, k == 0 ? 1 : 0, c->deverr.p);
+                k_grids<<<c->B, 1024, 0, s>>>(c->dbodies.p, c->nd.p, c->info.p, CT);
                 k_pair_count<<<kQueryGrid, kQueryChunk, 0, s>>>(c->dbodies.p, c->nd.p, CT);
                 k_pair_place<<<c->B, 1024, 0, s>>>(c->dbodies.p, c->B, CT, c->deverr.p);
                 k_pair_write<<<kQueryGrid, kQueryChunk, 0, s>>>(c->dbodies.p, c->nd.p, CT);
