@@ -33,12 +33,9 @@ __device__ __forceinline__ float dot3(f3 a, f3 b) { return a.x * b.x + a.y * b.y
 __device__ __forceinline__ float smin_(float a, float b) { return (b < a) ? b : a; }
 __device__ __forceinline__ float smax_(float a, float b) { return (a < b) ? b : a; }
 
-// SoftBody::compute_beam_forces (softbody.cpp:412-470) on bl_beam records, one beam a thread; the beam's force goes
-// to the scratch (w = 1: it pushes this substep), its state is updated in place.
-__global__ void k_noalloc_beams(const bl_node* __restrict__ nodes, bl_beam* __restrict__ beams, int n_beams, int deform, int brk, int ductile,
-                                float4* __restrict__ fv) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n_beams) return;
+// SoftBody::compute_beam_forces (softbody.cpp:412-470) on bl_beam record j; the beam's force goes to the scratch (w = 1: it
+// pushes this substep), its state is updated in place.
+__device__ __forceinline__ void noalloc_beam(int j, const bl_node* nodes, bl_beam* beams, int deform, int brk, int ductile, float4* fv) {
     bl_beam b = beams[j];
     float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (!(b.flags & (BL_BF_BROKEN | BL_BF_SHOCK))) {
@@ -101,20 +98,39 @@ __global__ void k_noalloc_beams(const bl_node* __restrict__ nodes, bl_beam* __re
 }
 
 // clear_forces' gravity, the node's beams in beam order (softbody.cpp:376, 466-467), SoftBody::integrate_nodes
-// (softbody.cpp:769-795)
-__global__ void k_noalloc_nodes(bl_node* __restrict__ nodes, int n_nodes, const int* __restrict__ inc_ptr, const int* __restrict__ inc,
-                                const float4* __restrict__ fv, float gx, float gy, float gz, float dt) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_nodes) return;
+// (softbody.cpp:769-795). wait: called once, between what is read of the node itself and the forces. kAtOnce forces are
+// loaded together, then added in order.
+constexpr int kAtOnce = 8;
+template <class Wait>
+__device__ __forceinline__ void noalloc_node(int i, bl_node* nodes, const int* __restrict__ inc_ptr, const int* __restrict__ inc, const float4* fv, float gx,
+                                             float gy, float gz, float dt, Wait wait) {
     bl_node x = nodes[i];
     const float m = x.mass;
     float fx = gx * m, fy = gy * m, fz = gz * m;
-    for (int q = inc_ptr[i]; q < inc_ptr[i + 1]; q++) {
-        const int e = inc[q];
-        const float4 b = fv[e & 0x7fffffff];
-        if (b.w != 0.0f) {
-            if (e < 0) fx = fx - b.x, fy = fy - b.y, fz = fz - b.z;
-            else fx = fx + b.x, fy = fy + b.y, fz = fz + b.z;
+    const int q1 = inc_ptr[i + 1];
+    int q = inc_ptr[i], e[kAtOnce];
+    auto load = [&]() {
+#pragma unroll
+        for (int u = 0; u < kAtOnce; u++) e[u] = q + u < q1 ? inc[q + u] : 0;
+    };
+    load();
+    wait();
+    while (q < q1) {
+        const int n = q1 - q;
+        float4 b[kAtOnce];
+        bool minus[kAtOnce];
+#pragma unroll
+        for (int u = 0; u < kAtOnce; u++) {
+            minus[u] = e[u] < 0;
+            b[u] = u < n ? __ldcg(fv + (e[u] & 0x7fffffff)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        q += kAtOnce;
+        load();
+#pragma unroll
+        for (int u = 0; u < kAtOnce; u++) {
+            if (b[u].w == 0.0f) continue;
+            if (minus[u]) fx = fx - b[u].x, fy = fy - b[u].y, fz = fz - b[u].z;
+            else fx = fx + b[u].x, fy = fy + b[u].y, fz = fz + b[u].z;
         }
     }
     if (x.inv_mass > 0) {
@@ -131,6 +147,22 @@ __global__ void k_noalloc_nodes(bl_node* __restrict__ nodes, int n_nodes, const 
         x.p[0] = x.p[0] + vx * dt, x.p[1] = x.p[1] + vy * dt, x.p[2] = x.p[2] + vz * dt;
         nodes[i] = x;
     }
+}
+
+// The beams, then the nodes as a programmatic dependent launch (both kernels read the nodes: a node's own record and first
+// incidences are read before the wait for the forces). Latency bounds both: blocks of 64 spread a small body over the
+// SMs. B200, 400 nodes and 3,121 beams: 12.3 us a substep with one force at a time, blocks of 256 and the second launch
+// behind the whole first, 11.1 us so (12.3 as one launch of a cluster of 8 blocks with its barrier between).
+constexpr int kBlock = 64;
+__global__ void k_noalloc_beams(const bl_node* nodes, bl_beam* beams, int n_beams, int deform, int brk, int ductile, float4* fv) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); // (k_noalloc_nodes may start: it waits before it reads fv)
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < n_beams) noalloc_beam(j, nodes, beams, deform, brk, ductile, fv);
+}
+__global__ void k_noalloc_nodes(bl_node* nodes, int n_nodes, const int* __restrict__ inc_ptr, const int* __restrict__ inc, const float4* fv, float gx,
+                                float gy, float gz, float dt) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_nodes) noalloc_node(i, nodes, inc_ptr, inc, fv, gx, gy, gz, dt, [] { asm volatile("griddepcontrol.wait;" ::: "memory"); });
 }
 
 // The scratch's address per CUDA context, for the calls made while their stream is being captured (a capture forbids
@@ -192,15 +224,22 @@ extern "C" int bl_gpu_substep_noalloc(bl_node* nodes, int32_t n_nodes, bl_beam* 
     float4* fv = nullptr;
     if (scratch_address(s, &fv) != BL_GPU_OK) return BL_GPU_ECUDA;
     if (n_nodes == 0) return BL_GPU_OK;
-    // each launch's own status (cudaLaunchKernel returns it), not an earlier error left pending by other code
+    // each launch's own status (the launch returns it), not an earlier error left pending by other code
+    float gx = gravity[0], gy = gravity[1], gz = gravity[2];
     if (n_beams > 0) {
         const bl_node* cn = nodes;
         void* args[] = {(void*)&cn, (void*)&beams, (void*)&n_beams, (void*)&allow_deform, (void*)&allow_break, (void*)&ductile, (void*)&fv};
-        if (cudaLaunchKernel((const void*)k_noalloc_beams, dim3((n_beams + 255) / 256), dim3(256), args, 0, s) != cudaSuccess) return BL_GPU_ECUDA;
+        if (cudaLaunchKernel((const void*)k_noalloc_beams, dim3((n_beams + kBlock - 1) / kBlock), dim3(kBlock), args, 0, s) != cudaSuccess) return BL_GPU_ECUDA;
     }
     const float4* cfv = fv;
-    float gx = gravity[0], gy = gravity[1], gz = gravity[2];
     void* args[] = {(void*)&nodes, (void*)&n_nodes, (void*)&inc_ptr, (void*)&inc, (void*)&cfv, (void*)&gx, (void*)&gy, (void*)&gz, (void*)&dt};
-    if (cudaLaunchKernel((const void*)k_noalloc_nodes, dim3((n_nodes + 255) / 256), dim3(256), args, 0, s) != cudaSuccess) return BL_GPU_ECUDA;
+    // (only after this call's own first kernel may it start early: what ran before on the stream may write the nodes)
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3((n_nodes + kBlock - 1) / kBlock), lc.blockDim = dim3(kBlock), lc.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at, lc.numAttrs = n_beams > 0 ? 1 : 0;
+    if (cudaLaunchKernelExC(&lc, (const void*)k_noalloc_nodes, args) != cudaSuccess) return BL_GPU_ECUDA;
     return BL_GPU_OK;
 }
