@@ -2,7 +2,7 @@
 //
 //   k_frame_begin     one thread per body: static candidates over the box grown by its travel, terrain height bound
 //   n x { k_beams     one thread per beam: spring-damper, plastic yield, break -> the beam's force scalar (fsc)
-//         k_force     one thread per node: gravity + its beams' forces in beam order (each made again from the scalar
+//         k_force     one thread (small worlds: a warp) per node: gravity + its beams' forces in beam order (each made again from the scalar
 //                     and the two positions) -> the node's force
 //         (contacts between bodies add to the force: bl_contacts.cuh)
 //         k_integrate } one thread per node: static contact, integration, bounds / top speed / contacts per body

@@ -165,7 +165,7 @@ struct bl_gpu_ctx {
     DevBuf<float4> dwst, dwctl, dwcf;
     DevBuf<int4> dwarm;
     DevBuf<float> dwper;
-    int NWR = 0;                               // of those, the builders' wheels (k_wheels)
+    int NWR = 0;                               // of those, the builders' wheels (wheel_step)
     DevBuf<float4> dtcon, dtfric;
     std::vector<int> lvl_grp_ptr, lvl_col_ptr; // per level: its update groups / columns
     int64_t fem_launches = 0;                  // kernels of one substep's frame step (with the Cholesky)
@@ -180,8 +180,7 @@ struct bl_gpu_ctx {
     cudaStream_t aux = nullptr;                // (captures the bodies of conditional graph nodes)
     // the learned warm start (bl_mlp.cuh): parameters, the step's features, recorded samples, training scratch
     DevBuf<float> mlp_w, mlp_m, mlp_v, feat, prev_dv, smp_x, smp_t, smp_w, gpart, gsum;
-    DevBuf<double> lpart, mlp_acc;
-    DevBuf<float> mlp_x, mlp_y, mlp_tw;        // the network's calls on host memory: samples, outputs (targets), weights
+    DevBuf<float> mlp_io;                      // the network's calls on host memory: the loss, samples, outputs (targets), weights
     std::mutex mlp_mutex;                      // (these calls, one at a time)
     DevBuf<__nv_bfloat16> mlp_wb;
     DevBuf<int> adj_ptr, adj, scount, sidx;
@@ -1850,8 +1849,7 @@ int bl_gpu_destroy(bl_gpu_ctx* c) {
     free_statics(c);
     c->deverr.free_();
     c->mlp_w.free_(), c->mlp_m.free_(), c->mlp_v.free_(), c->mlp_wb.free_(), c->smp_x.free_(), c->smp_t.free_(), c->smp_w.free_();
-    c->scount.free_(), c->sidx.free_(), c->gpart.free_(), c->lpart.free_(), c->gsum.free_();
-    c->mlp_x.free_(), c->mlp_y.free_(), c->mlp_tw.free_(), c->mlp_acc.free_();
+    c->scount.free_(), c->sidx.free_(), c->gpart.free_(), c->gsum.free_(), c->mlp_io.free_();
     if (c->order_event) cudaEventDestroy(c->order_event);
     if (c->stream) cudaStreamDestroy(c->stream);
     if (c->aux) cudaStreamDestroy(c->aux);
@@ -2273,29 +2271,31 @@ int bl_gpu_mlp_samples(bl_gpu_ctx* c, int32_t* n) {
     return BL_GPU_OK;
 }
 
-// The network's calls on host memory, one at a time: their device buffers are the context's, and are given back at the end
-// of a call that needed more than kMlpKeep floats of one (64 MB: 466,000 samples). To allocate and release them on each
-// call took as long as its kernels.
-constexpr size_t kMlpKeep = (size_t)16 << 20;
+// The network's calls on host memory, one at a time: their device buffer is the context's, and is given back at the end
+// of a call that needed more than kMlpKeep floats (128 MB: 559,000 samples). To allocate and release buffers on each call
+// took as long as its kernels.
+constexpr size_t kMlpKeep = (size_t)32 << 20, kMlpHead = 64; // (kMlpHead: the loss's floats before the samples)
 struct MlpCall {
     bl_gpu_ctx* c;
     std::lock_guard<std::mutex> lock;
     explicit MlpCall(bl_gpu_ctx* c) : c(c), lock(c->mlp_mutex) {}
     ~MlpCall() {
-        if (c->mlp_x.n > kMlpKeep) c->mlp_x.free_(), c->mlp_y.free_(), c->mlp_tw.free_();
+        if (c->mlp_io.n > kMlpKeep) c->mlp_io.free_();
     }
 };
 
 // one pass of k_mlp_grad over n samples (x, t, w on the device; idx: the samples, or null) and, with lr > 0, Adam
 static int mlp_batch(bl_gpu_ctx* c, const float* x, const float* t, const float* w, const int* idx, int n, float lr, float* gsum, double* acc) {
     const int nblk = std::min((n + kTile - 1) / kTile, 2 * 148); // (two blocks an SM)
-    BL_CUDA(c, c->gpart.room((size_t)nblk * kParams));
-    BL_CUDA(c, c->lpart.room(nblk));
+    const size_t nl = (size_t)(nblk + 31) / 32 * 32; // (the blocks' losses, then their gradients)
+    BL_CUDA(c, c->gpart.room(2 * nl + (size_t)nblk * kParams));
+    double* lpart = reinterpret_cast<double*>(c->gpart.p);
+    float* gpart = c->gpart.p + 2 * nl;
     const MlpDev M = mlp_dev(c);
     BL_CUDA(c, cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpGradSmem)));
-    k_mlp_grad<<<nblk, kMlpThreads, sizeof(MlpGradSmem), c->stream>>>(M, x, t, w, idx, n, c->gpart.p, c->lpart.p);
+    k_mlp_grad<<<nblk, kMlpThreads, sizeof(MlpGradSmem), c->stream>>>(M, x, t, w, idx, n, gpart, lpart);
     if (lr > 0) c->adam_t++;
-    k_mlp_adam<<<(kParams + 31) / 32, 256, 0, c->stream>>>(M, c->gpart.p, c->lpart.p, nblk, gsum, acc, lr, 0.9f, 0.999f, 1e-8f, std::max(c->adam_t, 1));
+    k_mlp_adam<<<(kParams + 31) / 32, 256, 0, c->stream>>>(M, gpart, lpart, nblk, gsum, acc, lr, 0.9f, 0.999f, 1e-8f, std::max(c->adam_t, 1));
     BL_CUDA(c, cudaGetLastError());
     return BL_GPU_OK;
 }
@@ -2341,12 +2341,12 @@ int bl_gpu_mlp_forward(bl_gpu_ctx* c, const float* x, int32_t n, float* y) {
     if (n == 0) return BL_GPU_OK;
     BL_CUDA(c, cudaSetDevice(c->cfg.device));
     const MlpCall call(c);
-    BL_CUDA(c, c->mlp_x.room((size_t)kIn * n));
-    BL_CUDA(c, c->mlp_y.room((size_t)kOut * n));
-    BL_CUDA(c, cudaMemcpyAsync(c->mlp_x.p, x, sizeof(float) * kIn * n, cudaMemcpyHostToDevice, c->stream));
-    k_mlp_forward_batch<<<std::min((n + kTile - 1) / kTile, 4 * 148), kMlpThreads, 0, c->stream>>>(mlp_dev(c), c->mlp_x.p, n, c->mlp_y.p);
+    BL_CUDA(c, c->mlp_io.room(kMlpHead + (size_t)(kIn + kOut) * n));
+    float *dx = c->mlp_io.p + kMlpHead, *dy = dx + (size_t)kIn * n;
+    BL_CUDA(c, cudaMemcpyAsync(dx, x, sizeof(float) * kIn * n, cudaMemcpyHostToDevice, c->stream));
+    k_mlp_forward_batch<<<std::min((n + kTile - 1) / kTile, 4 * 148), kMlpThreads, 0, c->stream>>>(mlp_dev(c), dx, n, dy);
     BL_CUDA(c, cudaGetLastError());
-    BL_CUDA(c, cudaMemcpyAsync(y, c->mlp_y.p, sizeof(float) * kOut * n, cudaMemcpyDeviceToHost, c->stream));
+    BL_CUDA(c, cudaMemcpyAsync(y, dy, sizeof(float) * kOut * n, cudaMemcpyDeviceToHost, c->stream));
     BL_CUDA(c, cudaStreamSynchronize(c->stream));
     return BL_GPU_OK;
 }
@@ -2355,19 +2355,18 @@ int bl_gpu_mlp_gradient(bl_gpu_ctx* c, const float* x, const float* t, const flo
     if (!c || n < 1 || !x || !t || !w || !grad) return BL_GPU_EINVAL;
     BL_CUDA(c, cudaSetDevice(c->cfg.device));
     const MlpCall call(c);
-    BL_CUDA(c, c->mlp_x.room((size_t)kIn * n));
-    BL_CUDA(c, c->mlp_y.room((size_t)kOut * n));
-    BL_CUDA(c, c->mlp_tw.room((size_t)kOut * n));
-    BL_CUDA(c, c->mlp_acc.room(1));
-    BL_CUDA(c, cudaMemcpyAsync(c->mlp_x.p, x, sizeof(float) * kIn * n, cudaMemcpyHostToDevice, c->stream));
-    BL_CUDA(c, cudaMemcpyAsync(c->mlp_y.p, t, sizeof(float) * kOut * n, cudaMemcpyHostToDevice, c->stream));
-    BL_CUDA(c, cudaMemcpyAsync(c->mlp_tw.p, w, sizeof(float) * kOut * n, cudaMemcpyHostToDevice, c->stream));
-    BL_CUDA(c, cudaMemsetAsync(c->mlp_acc.p, 0, sizeof(double), c->stream));
-    const int rc = mlp_batch(c, c->mlp_x.p, c->mlp_y.p, c->mlp_tw.p, nullptr, n, 0.0f, c->gsum.p, c->mlp_acc.p);
+    BL_CUDA(c, c->mlp_io.room(kMlpHead + (size_t)(kIn + 2 * kOut) * n));
+    double* acc = reinterpret_cast<double*>(c->mlp_io.p);
+    float *dx = c->mlp_io.p + kMlpHead, *dt = dx + (size_t)kIn * n, *dw = dt + (size_t)kOut * n;
+    BL_CUDA(c, cudaMemcpyAsync(dx, x, sizeof(float) * kIn * n, cudaMemcpyHostToDevice, c->stream));
+    BL_CUDA(c, cudaMemcpyAsync(dt, t, sizeof(float) * kOut * n, cudaMemcpyHostToDevice, c->stream));
+    BL_CUDA(c, cudaMemcpyAsync(dw, w, sizeof(float) * kOut * n, cudaMemcpyHostToDevice, c->stream));
+    BL_CUDA(c, cudaMemsetAsync(acc, 0, sizeof(double), c->stream));
+    const int rc = mlp_batch(c, dx, dt, dw, nullptr, n, 0.0f, c->gsum.p, acc);
     if (rc) return rc;
     double a = 0;
     BL_CUDA(c, cudaMemcpyAsync(grad, c->gsum.p, sizeof(float) * kParams, cudaMemcpyDeviceToHost, c->stream));
-    BL_CUDA(c, cudaMemcpyAsync(&a, c->mlp_acc.p, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    BL_CUDA(c, cudaMemcpyAsync(&a, acc, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     BL_CUDA(c, cudaStreamSynchronize(c->stream));
     if (loss) *loss = (float)(a / n);
     return BL_GPU_OK;

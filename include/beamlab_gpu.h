@@ -85,14 +85,14 @@ typedef struct {
                                   none - measured on the plates, the scale as trained costs iterations */
     int32_t graphs;            /* 1 (default): a frame of n substeps is captured once as a CUDA graph and replayed; 0: its
                                   kernels are launched one by one every call (the plain path, one launch per kernel) */
-    int32_t beam_kernel;       /* 0 (default): the beams' kernel streams the beam arrays through shared memory by bulk
-                                  (TMA) copies and the nodes' kernel reads 4-byte incidences where the rig allows; 1:
+    int32_t beam_kernel;       /* 0 (default): the beams' kernel streams the beam arrays of worlds above 4 M beams
+                                  through shared memory by bulk (TMA) copies and the nodes' kernel reads 4-byte incidences where the rig allows; 1:
                                   plain loads and 8-byte incidences. Results are the same. */
     int32_t fem_dense_front;   /* how the FEM step factors its system:
                                   3 (default): 2;
                                   2: multifrontal - the columns in a nested-dissection order, grouped into dense fronts
-                                  (supernodes of the elimination tree, small ones amalgamated) of 48 x 48 tiles, the whole
-                                  factorization and both solves one launch; with the reference's order, pattern and fill
+                                  (supernodes of the elimination tree, small ones amalgamated) of 48 x 48 tiles, the factorization
+                                  one launch, the backward solves another; with the reference's order, pattern and fill
                                   1: block column by block column, with the top chain of the elimination tree
                                   (levels of one column each) as one dense front; 0: block column by block column in the
                                   reference's order of sums throughout. 2 and 1 differ from 0 in the order of the
@@ -429,7 +429,7 @@ typedef struct {
     int64_t levels;            /* elimination-tree levels */
     int64_t repasses;          /* unload re-passes: the steps' systems assembled and factored again where the step
                                   unloaded a flowing hinge, bar or twist of a yielding member */
-    int64_t fronts;            /* fem_dense_front == 2: the multifrontal factorization's dense fronts (0 otherwise); */
+    int64_t fronts;            /* fem_dense_front 2 or 3: the multifrontal factorization's dense fronts (else 0); */
     double factor_flops;       /* the flops of one factorization as this path runs it (multiplies and adds counted
                                   apart; the multifrontal's dense fronts include their explicit zeros) */
 } bl_fem_stats;

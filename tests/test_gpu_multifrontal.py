@@ -38,3 +38,14 @@ def test_one_launch_agrees_with_block_columns(name):
         pos.append(np.concatenate([np.ascontiguousarray(h.nodes()["p"]) for h in w.bodies()]).astype(np.float64))
         w.close()
     assert np.abs(pos[0] - pos[1]).max() < 1e-9
+
+
+def test_wide_level_and_many_children():
+    """A shell body of 10,000 nodes: its lowest level's fronts go a block each (more than 3,000 tiles' tasks otherwise), and the
+    separators above gather many children: every solution's residual is at rounding level."""
+    w = world_from_rig(rigs.shell_body(10000), fem_dense_front=2, fem_check_residual=True)
+    w.step_substeps(6)
+    st = w.fem_stats()
+    assert st["max_residual"] < 1e-11 and st["fronts"] > 0 and w.stats()["device_errors"] == 0
+    assert all(h.state()["fem_failures"] == 0 for h in w.bodies())
+    w.close()
