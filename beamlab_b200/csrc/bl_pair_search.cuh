@@ -358,6 +358,7 @@ __global__ void __launch_bounds__(1024) k_rebuild(Body* __restrict__ bodies, int
         S.b[k].extra = 0.0f, S.b[k].bulk = 0.0f;
         S.b[k].g_dim[0] = S.b[k].g_dim[1] = S.b[k].g_dim[2] = 0;
     }
+    __syncthreads(); // (every body's speed, for the margins)
     const float dt = C.dt;
     const int interval = C.interval;
     if (tid == 0) {
