@@ -319,7 +319,7 @@ __device__ __forceinline__ bool mf_assemble(const FemDev& F, const MfDev& M, con
             const int rp = rx < re ? pos[rx] : -1, cq = cx < ce ? pos[cx] : -1;
             if (k == 0) K.base[q] = cf.tile0, K.nt[q] = cf.nt, K.P[q] = cf.P, K.bt[q] = cf.bt, K.br[q] = cf.br;
             K.row[q][k] = -1, K.col[q][k] = -1;
-            __syncwarp(__activemask());
+            __syncwarp(0xffu << (tid & 24)); // (the child's eight threads: q < nq holds for all of them or none)
             if (rp >= 0) K.row[q][rp & 7] = rx;
             if (cq >= 0) K.col[q][cq & 7] = cx;
             if (k == 0) ok = mf_wait(M.fdone + c, cf.need, M.ctr + 1);
