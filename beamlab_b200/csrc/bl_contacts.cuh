@@ -307,8 +307,13 @@ namespace blg {
 
 // ------------------------------------------------------------------------------------------ narrow phase (each substep)
 // World::pair_detect for node-triangle pairs (world.cpp:2819-2858): hit_a = (bary, pen), hit_b = (normal, 1) when
-// the pair is in contact, hit_b.w = 0 when not
-__global__ void __launch_bounds__(256) k_detect(const float4* __restrict__ nd, const int4* __restrict__ info, const Body* __restrict__ bodies, Contacts C) {
+// the pair is in contact, hit_b.w = 0 when not. All of it before the wait (bl_device.cuh): the nodes and the bodies' sleep
+// from L2.
+__global__ void __launch_bounds__(256) k_detect(const float4* nd, const int4* __restrict__ info, const Body* bodies, Contacts C) {
+    auto at = [nd](int i) {
+        const float4 p = __ldcg(nd + i);
+        return V(p.x, p.y, p.z);
+    };
     const int total = min(*C.pair_total, C.max_pairs);
     // (a warp takes 32 consecutive pairs: its ballot is their word of hit bits)
     for (int i0 = blockIdx.x * blockDim.x; i0 < total; i0 += gridDim.x * blockDim.x) {
@@ -321,11 +326,11 @@ __global__ void __launch_bounds__(256) k_detect(const float4* __restrict__ nd, c
             const Body& bt = bodies[tr.w >> 8];
             float4 ha = make_float4(0, 0, 0, 0), hb = make_float4(0, 0, 0, 0);
             do {
-                if (bn.sleeping && bt.sleeping) break;
+                if (__ldcg(&bn.sleeping) && __ldcg(&bt.sleeping)) break;
                 if (tr.w & TF_TORN) break; // (torn since the pairs were found)
                 const bool two_sided = (tr.w & TF_TWO_SIDED) != 0;
-                const v3 np = nd_p(nd, pr.x);
-                const v3 a = nd_p(nd, tr.x), b = nd_p(nd, tr.y), cc = nd_p(nd, tr.z);
+                const v3 np = at(2 * pr.x);
+                const v3 a = at(2 * tr.x), b = at(2 * tr.y), cc = at(2 * tr.z);
                 v3 bary;
                 const float r = bt.faces_only && !two_sided ? bt.face_skin : bn.crad;
                 if (!two_sided) {
@@ -355,8 +360,8 @@ __global__ void __launch_bounds__(256) k_detect(const float4* __restrict__ nd, c
                     nrm = divs(d, dist);
                 } else {
                     nrm = normalize(cross(b - a, cc - a));
-                    const v3 vt = nd_v(nd, tr.x) * bary.x + nd_v(nd, tr.y) * bary.y + nd_v(nd, tr.z) * bary.z;
-                    if (dot(nd_v(nd, pr.x) - vt, nrm) > 0) nrm = neg(nrm);
+                    const v3 vt = at(2 * tr.x + 1) * bary.x + at(2 * tr.y + 1) * bary.y + at(2 * tr.z + 1) * bary.z;
+                    if (dot(at(2 * pr.x + 1) - vt, nrm) > 0) nrm = neg(nrm);
                 }
                 ha = make_float4(bary.x, bary.y, bary.z, r - dist), hb = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
                 hit = true;
@@ -398,7 +403,7 @@ __global__ void __launch_bounds__(256) k_detect(const float4* __restrict__ nd, c
 // contacts in 41 to 57 levels, in 1,000 cycles: the levels 33 by one thread (95 a contact), 20 so; the chain 68 to 89 with the
 // records read from global memory and the law's cases branched on, 34 so; the nodes' forces into the slots 16, 7 so.
 // A launch for 128 head-on pairs of vehicles 100 us, 63 so; for two crashing trusses (46 contacts) 10.1 and 6.5 us.
-__device__ void collide_island_global(const float4* __restrict__ nd, const int4* __restrict__ info, Body* __restrict__ bodies, Contacts C,
+__device__ void collide_island_global(const float4* nd, const int4* __restrict__ info, Body* __restrict__ bodies, Contacts C,
                                       float4* __restrict__ Fs, int root, int off, int cnt);
 
 constexpr int kCollideThreads = 512;
@@ -689,7 +694,7 @@ __device__ __forceinline__ void run_levels(int p, int end, int& L, const int* le
     }
 }
 
-__global__ void __launch_bounds__(kCollideThreads, 1) k_collide(const float4* __restrict__ nd, const int4* __restrict__ info, Body* __restrict__ bodies,
+__global__ void __launch_bounds__(kCollideThreads, 1) k_collide(const float4* nd, const int4* __restrict__ info, Body* __restrict__ bodies,
                                                             int nbodies, Contacts C, float4* __restrict__ Fs) {
     extern __shared__ __align__(16) unsigned char csm[];
     int* keys = reinterpret_cast<int*>(csm);                                   // the hash: a node, or -1
@@ -1011,7 +1016,7 @@ constexpr size_t kCollideSmem = sizeof(int) * kKeys + sizeof(unsigned short) * k
 static_assert(sizeof(ContactRec) * kRecChunk <= kCollideWork && sizeof(ContactRec) == 128, "the work area's uses");
 
 // The serial loop on global memory (the path of an island with more distinct contact nodes than the slots hold)
-__device__ void collide_island_global(const float4* __restrict__ nd, const int4* __restrict__ info, Body* __restrict__ bodies, Contacts C,
+__device__ void collide_island_global(const float4* nd, const int4* __restrict__ info, Body* __restrict__ bodies, Contacts C,
                                       float4* __restrict__ Fs, int root, int off, int cnt) {
     const float dt = C.dt;
     const GroundModel& gm = c_ground[3]; // SURF_CONCRETE

@@ -30,8 +30,9 @@ enum : uint32_t { DEVERR_CANDIDATES = 1, DEVERR_NONFINITE = 2, DEVERR_TIMEOUT = 
 // Programmatic dependent launches: a kernel launched so starts while the one before it (its predecessor) still runs, does
 // what does not depend on the predecessor's writes, and waits here until the predecessor is done. Every such kernel waits
 // (in every block, before it ends) before it lets its own successor start, so when a kernel runs, everything before its
-// predecessor is complete. Launched otherwise both are no-ops. What the predecessor writes is never read through a const
-// __restrict__ pointer: such loads may be moved above the wait.
+// predecessor is complete. Launched otherwise both are no-ops. What any kernel of the chain writes is never read through a
+// const __restrict__ pointer (such loads may be moved above the wait, or go through the non-coherent path), and what one
+// before the predecessor wrote and is read before the wait is read from L2 (__ldcg): the wait is what makes writes seen.
 __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

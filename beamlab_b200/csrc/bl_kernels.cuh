@@ -532,7 +532,7 @@ template <class Wait>
 __device__ __forceinline__ void wheel_step(int w, int lane, const float4* nd, const int4* __restrict__ info, const Body* bodies, const WheelDev& wh, float dt,
                                            Wait wait) {
     const int4 W = wh.wheel[w];
-    const float4 ctl = wh.wctl[w], st = wh.wst[w];
+    const float4 ctl = wh.wctl[w], st = __ldcg(wh.wst + w);
     const int4 A = wh.warm[w];
     const int own = W.w > 0 ? info[W.x].w : 0, first = lane < W.w ? wh.wlist[W.z + lane] : 0;
     wait();
@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(256) k_beams(const int2* __restrict__ ab, cons
     const int j0 = 2 * blockIdx.x * blockDim.x + threadIdx.x, j1 = j0 + blockDim.x;
     const bool h0 = j0 < nbeams, h1 = j1 < nbeams;
     const int2 e0 = h0 ? ab[j0] : make_int2(0, 0), e1 = h1 ? ab[j1] : make_int2(0, 0);
-    const float4 s0 = h0 ? bst[j0] : make_float4(0, 0, 0, 0), s1 = h1 ? bst[j1] : make_float4(0, 0, 0, 0);
+    const float4 s0 = h0 ? __ldcg(bst + j0) : make_float4(0, 0, 0, 0), s1 = h1 ? __ldcg(bst + j1) : make_float4(0, 0, 0, 0);
     const float2 c0 = h0 ? kd[j0] : make_float2(0, 0), c1 = h1 ? kd[j1] : make_float2(0, 0);
     pdl_wait();
     const uint32_t m0 = h0 ? bmeta[j0] : kBeamAsleep, m1 = h1 ? bmeta[j1] : kBeamAsleep;
@@ -916,9 +916,10 @@ __global__ void k_drag_parts(Body* __restrict__ bodies, int nbodies, const float
 // kWide: a warp a node, a lane an incidence - the gathers of a node's beams all at once, their forces then added in their
 // order by broadcasts (the same sums) - for worlds whose nodes all fit on the GPU that way: a node of 26 beams waits for
 // one gather instead of seven (B200, a frame of 33 substeps of the 400-node truss car: 333 us a thread a node, 265 so).
-// The gathers of the nodes come before the wait for the beams' kernel, whose scalars are all that is new.
+// The gathers of the nodes come before the wait for the beams' kernel, whose scalars are all that is new (from L2, bl_device.cuh;
+// after the wait: 3.5 % of a frame of 400 to 500 nodes).
 template <bool kPacked, bool kWide>
-__global__ void __launch_bounds__(256, kWide ? 4 : 6) k_force(const float4* __restrict__ nd, const int4* __restrict__ info, const int* __restrict__ ell_ptr,
+__global__ void __launch_bounds__(256, kWide ? 4 : 6) k_force(const float4* nd, const int4* __restrict__ info, const int* __restrict__ ell_ptr,
                                                const void* __restrict__ ell_, const int* __restrict__ ell_base, const float* fsc,
                                                Body* __restrict__ bodies, float gx, float gy, float gz, int nnodes, int first, NodeFem nf,
                                                float4* __restrict__ fnode, DragDev dg, WheelDev wh, ShockDev sk) {
@@ -930,7 +931,8 @@ __global__ void __launch_bounds__(256, kWide ? 4 : 6) k_force(const float4* __re
     if (i < nnodes) {
         // (the node's own loads and its warp's incidence range issued before its body's state arrives)
         const int4 inf = info[i];
-        const float4 P = nd[2 * i], Vv = nd[2 * i + 1];
+        float4 P, Vv;
+        if (kWide) P = __ldcg(nd + 2 * i), Vv = __ldcg(nd + 2 * i + 1);
         const int w = i >> 5, lane = i & 31;
         const int q0 = ell_ptr[w], width = (ell_ptr[w + 1] - q0) >> 5;
         const int base = kPacked ? ell_base[w] : 0;
@@ -953,9 +955,10 @@ __global__ void __launch_bounds__(256, kWide ? 4 : 6) k_force(const float4* __re
         float4 Po1 = make_float4(0, 0, 0, 0);
         if (kWide) {
             if ((int)(g & 31) < width) entry(g & 31, beam1, other1, pad1, bend1);
-            if (!pad1) Po1 = nd[2 * other1];
+            if (!pad1) Po1 = __ldcg(nd + 2 * other1);
         }
         pdl_wait();
+        if (!kWide) P = nd[2 * i], Vv = nd[2 * i + 1]; // (after the wait: by L1, for the neighbours' gathers)
         if (!B.sleeping) {
             const float m = Vv.w;
             v3 f;
@@ -1164,10 +1167,10 @@ __global__ void __launch_bounds__(256) k_integrate(float4* nd, const int4* __res
     if (i < nnodes) {
         // (the node's own loads issued before its body's state arrives)
         inf = info[i];
-        P = nd[2 * i], Vv = nd[2 * i + 1];
+        P = __ldcg(nd + 2 * i), Vv = __ldcg(nd + 2 * i + 1);
         body = inf.w;
         const Body& B = bodies[body];
-        live = !B.sleeping && !B.is_fem;
+        live = !__ldcg(&B.sleeping) && !B.is_fem;
         if (live && ((uint32_t)inf.x & NF_GROUND) && !(P.w <= 0) && !(P.y < st.kill_y))
             hit = static_query(st, B, V(P.x, P.y, P.z), __int_as_float(inf.z), c);
     }
@@ -1244,7 +1247,7 @@ __global__ void __launch_bounds__(256) k_tyres(float4* nd, const int4* __restric
     int i = lane < W.w ? wh.wnodes[W.z + lane] : -1;
     const int body = lane < W.w ? info[i].w : 0;
     float4 P = make_float4(0, 0, 0, 0), Vv = P, f4 = P;
-    if (i >= 0) P = nd[2 * i], Vv = nd[2 * i + 1], f4 = fnode[i];
+    if (i >= 0) P = __ldcg(nd + 2 * i), Vv = __ldcg(nd + 2 * i + 1), f4 = __ldcg(fnode + i);
     pdl_wait();
     if (W.w == 0) return; // (w is the warp's: its lanes leave together)
     v3 need = V(0, 0, 0), mn = V(1e30f, 1e30f, 1e30f), mx = V(-1e30f, -1e30f, -1e30f);
