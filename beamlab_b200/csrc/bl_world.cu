@@ -1218,7 +1218,7 @@ static int commit_bodies(bl_gpu_ctx* c) {
         }
     }
     c->beam_grid = 0, c->ends16 = false;
-    if (c->cfg.beam_kernel == 0 && M > 0) {
+    if (c->cfg.beam_kernel != 1 && M > 0) {
         // each tile's beams' ends as 16-bit offsets from its lowest node, where every tile spans fewer than 65,536 nodes
         std::vector<int> tbase(c->beam_tiles, 0);
         std::vector<uint32_t> ab16(Mpad, 0u);
@@ -1277,7 +1277,7 @@ static int commit_bodies(bl_gpu_ctx* c) {
         // the 4-byte form where every warp's beams lie within 32,767 of its first and every neighbour within 32,767
         // nodes (k_force<true>): half the bytes of the incidence stream
         std::vector<int> base(nw, 0);
-        bool packed = c->cfg.beam_kernel == 0;
+        bool packed = c->cfg.beam_kernel != 1;
         for (int w = 0; w < nw && packed; w++) {
             int lo = INT32_MAX;
             for (int q = eptr[w]; q < eptr[w + 1]; q++) {
@@ -1465,8 +1465,8 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
     const float dt = c->cfg.dt;
     const float frame_time = (float)n * dt;
     const int tb = 256, gbody = (c->B + tb - 1) / tb;
-    // (bulk_wait_s 0 keeps the copies whose waits it makes run out)
-    const bool bulk = c->beam_grid > 0 && (c->M > kPlainBeams || c->wait_ns == 0), wide = c->N <= kWideNodes;
+    // (beam_kernel 2 asks for the bulk copies at any size, and so does bulk_wait_s 0, which makes their waits run out)
+    const bool bulk = c->beam_grid > 0 && (c->M > kPlainBeams || c->cfg.beam_kernel == 2 || c->wait_ns == 0), wide = c->N <= kWideNodes;
     const int bt = 64, gb = std::max(1, std::max((c->M + 2 * bt - 1) / (2 * bt), (c->B + bt - 1) / bt));
     // the substep's kernels as programmatic dependent launches (not between timing events)
     auto go = [&](auto kernel, int grid, int block, size_t smem, auto... args) { launch_after(s, ev == nullptr && !bulk, kernel, grid, block, smem, args...); };
@@ -1798,7 +1798,7 @@ int bl_gpu_create(const bl_gpu_config* cfg, bl_gpu_ctx** out) {
     bl_gpu_default_config(&c0);
     if (cfg) c0 = *cfg;
     if (!(c0.dt > 0) || c0.deterministic != 1 || c0.max_pairs < 1 || c0.fem_solver < 0 || c0.fem_solver > 3 || c0.pcg_max_iters < 0 ||
-        !(c0.pcg_tol > 0) || c0.beam_kernel < 0 || c0.beam_kernel > 1 || c0.fem_dense_front < 0 || c0.fem_dense_front > 3 ||
+        !(c0.pcg_tol > 0) || c0.beam_kernel < 0 || c0.beam_kernel > 2 || c0.fem_dense_front < 0 || c0.fem_dense_front > 3 ||
         !(c0.force_block == 0 || c0.force_block == 64 || c0.force_block == 128 || c0.force_block == 256) ||
         !(c0.integrate_block == 0 || c0.integrate_block == 64 || c0.integrate_block == 128 || c0.integrate_block == 256) ||
         c0.beams_per_sm < 0 || c0.beams_per_sm > 16 || !(c0.tyre_grip >= 0) || !(c0.bulk_wait_s >= 0 && c0.bulk_wait_s <= 10) ||

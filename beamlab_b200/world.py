@@ -71,7 +71,8 @@ class WorldSettings:
     pcg_learned_scale: bool = False
     # True: each frame captured once as a CUDA graph and replayed; False: its kernels launched one by one (plain path)
     graphs: bool = True
-    # the beams' kernel: 0 streams the beam arrays by bulk (TMA) copies, 1 plain loads (the same results)
+    # the beams' kernel: 0 bulk (TMA) copies of the beam arrays above 4 M beams, else plain loads; 1 plain loads and 8-byte
+    # incidences; 2 bulk copies at any size (the same results)
     beam_kernel: int = 0
     # the FEM factorization: 3 the fastest (2), 2 multifrontal (dense fronts of tiles, one launch), 1 block columns with the top chain as one dense front, 0 block columns in the reference's order
     fem_dense_front: int = 3

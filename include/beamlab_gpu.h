@@ -85,9 +85,10 @@ typedef struct {
                                   none - measured on the plates, the scale as trained costs iterations */
     int32_t graphs;            /* 1 (default): a frame of n substeps is captured once as a CUDA graph and replayed; 0: its
                                   kernels are launched one by one every call (the plain path, one launch per kernel) */
-    int32_t beam_kernel;       /* 0 (default): the beams' kernel streams the beam arrays of worlds above 4 M beams
-                                  through shared memory by bulk (TMA) copies and the nodes' kernel reads 4-byte incidences where the rig allows; 1:
-                                  plain loads and 8-byte incidences. Results are the same. */
+    int32_t beam_kernel;       /* 0 (default): the beams' kernel streams the beam arrays of worlds above 4 M beams through
+                                  shared memory by bulk (TMA) copies, those of smaller worlds come by plain loads, and the
+                                  nodes' kernel reads 4-byte incidences where the rig allows; 1: plain loads and 8-byte
+                                  incidences; 2: as 0, the bulk copies at any size. Results are the same. */
     int32_t fem_dense_front;   /* how the FEM step factors its system:
                                   3 (default): 2;
                                   2: multifrontal - the columns in a nested-dissection order, grouped into dense fronts
@@ -105,7 +106,8 @@ typedef struct {
     float bulk_wait_s;         /* (no counterpart in the reference) the beams kernel's bound on a wait for its own bulk
                                   copies, in seconds (default 1, at most 10): one that runs out raises
                                   BL_GPU_DEVERR_TIMEOUT, lets the copies in flight land and ends the block's work for that
-                                  substep; 0 makes every such wait report as run out (for tests of that path) */
+                                  substep; 0 makes every such wait report as run out, and takes the bulk copies at any
+                                  size unless beam_kernel is 1 (for tests of that path) */
     int32_t contact_whole_max; /* (no counterpart in the reference) an island's contacts run whole - their order found
                                   over the island - up to this many (default and most: 6144); more run 448 at a time. The
                                   same results either way; 0 runs every island 448 at a time (for tests of that path) */
