@@ -1531,8 +1531,8 @@ static int enqueue_frame(bl_gpu_ctx* c, int n, cudaStream_t s, cudaEvent_t* ev =
             go(kernel, grid, block, 0, c->nd.p, c->info.p, c->ell_ptr.p, ell, base, c->fsc.p, c->dbodies.p, c->cfg.gravity[0], c->cfg.gravity[1],
                c->cfg.gravity[2], c->N, k == 0 ? 1 : 0, nfm, c->nodef.p, dg, wh, sk);
         };
-        if (wide && c->packed_inc) force(k_force<true, true>, c->inc4.p, c->ell_base.p, (c->N + 7) / 8, 256);
-        else if (wide) force(k_force<false, true>, c->inc2.p, nullptr, (c->N + 7) / 8, 256);
+        if (wide && c->packed_inc) force(k_force<true, true>, c->inc4.p, c->ell_base.p, std::max((c->N + 7) / 8, 1), 256);
+        else if (wide) force(k_force<false, true>, c->inc2.p, nullptr, std::max((c->N + 7) / 8, 1), 256);
         else if (c->packed_inc) force(k_force<true, false>, c->inc4.p, c->ell_base.p, std::max(gfn, 1), fb);
         else force(k_force<false, false>, c->inc2.p, nullptr, std::max(gfn, 1), fb);
         mark();
