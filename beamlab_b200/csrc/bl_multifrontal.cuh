@@ -160,20 +160,10 @@ __device__ __forceinline__ void mf_ab8(double (&acc)[2], const double* A, const 
 // where this lane's pair of an 8 x 8 accumulator lies in a block
 __device__ __forceinline__ int mf_pair8(int lane) { return ((lane & 3) >> 1) * 32 + (lane >> 2) * 4 + 2 * (lane & 1); }
 
-// 1 / sqrt(s) for a normal s > 0 without a branch (the panel's other work is scheduled into its latency): the
-// instruction's 20-bit approximation y, then one step of Householder's third-order iteration,
-// y (1 + e / 2 + 3 e^2 / 8) with e = 1 - s y^2 (e below 2^-18 leaves 5 e^3 / 16, under a tenth of an ulp)
-__device__ __forceinline__ double mf_rsqrt(double s) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
-    const double e = fma(-(s * y), y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
 // The inverse of an 8 x 8 block's Cholesky factor, by one warp: every lane factors the block in its own registers, so
 // that a column's chain is the inverse square root, a multiply and a multiply-add with no exchange of lanes; lane i < 8
 // carries row i of an identity along, which comes out as column i of the inverse. (Lanes a row each and the columns
-// broadcast by shuffles: 190 cycles a column against 85.) False at a pivot that is not positive.
+// broadcast by shuffles: 190 cycles a column against 85.) False at a pivot that is not positive or not finite.
 __device__ __forceinline__ bool mf_inv8(const double* B, double* inv, int lane) {
     double d[8][8], a[8];
 #pragma unroll
@@ -188,10 +178,8 @@ __device__ __forceinline__ bool mf_inv8(const double* B, double* inv, int lane) 
     bool ok = true;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-        const bool good = d[j][j] >= 2.2250738585072014e-308;
-        ok = ok && good;
-        double id = mf_rsqrt(d[j][j]);
-        id = good ? id : 1.0; // (after the root, as a select: the test is off the chain)
+        const double id = bl_pivot_rsqrt(d[j][j], ok);
+        if (j == 7) ok = ok && id == id; // (an infinite pivot: no number from it on, so the next pivot says so, or this)
 #pragma unroll
         for (int l = j + 1; l < 8; l++) d[l][j] *= id;
         a[j] *= id;
