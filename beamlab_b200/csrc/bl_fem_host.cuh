@@ -16,6 +16,8 @@
 #include <functional>
 #include <vector>
 
+#include "bl_mf_plan.cuh"
+
 namespace blg {
 
 struct FemSection { // ShellSection (frame_fem.h:114-150): the elastic step's fields
@@ -581,10 +583,12 @@ struct FemDissection {
 };
 
 // the factor's pattern of an order: a column's rows are its node's later neighbours and its children's rows but itself
-// (its children: the columns whose first row it is), ascending
-static void fem_symbolic(const std::vector<int>& order, const std::vector<int>& iperm, const std::vector<int>& ptr, const std::vector<int>& nbr,
-                         std::vector<int>& col_ptr, std::vector<int>& row) {
+// (its children: the columns whose first row it is), ascending. False, and unfinished, once the columns' block updates
+// take more than max_flops.
+static bool fem_symbolic(const std::vector<int>& order, const std::vector<int>& iperm, const std::vector<int>& ptr, const std::vector<int>& nbr,
+                         std::vector<int>& col_ptr, std::vector<int>& row, double max_flops = 1e300) {
     const int n = (int)order.size();
+    double flops = 0;
     std::vector<int> mark(n, -1), first_child(n, -1), next_child(n, -1);
     col_ptr.assign(1, 0);
     row.clear();
@@ -600,7 +604,56 @@ static void fem_symbolic(const std::vector<int>& order, const std::vector<int>& 
         std::sort(row.begin() + r0, row.end());
         col_ptr.push_back((int)row.size());
         if (row.size() > r0) next_child[k] = first_child[row[r0]], first_child[row[r0]] = k;
+        const double d = (double)(row.size() - r0);
+        flops += 216.0 * d * (d + 1);
+        if (flops > max_flops) return false;
     }
+    return true;
+}
+
+// The multifrontal path's order and its pattern: nested dissection, except where the planes cut badly - rest positions that do
+// not follow the connectivity, a sheet rolled up - and the minimum-degree order, which looks at the connectivity alone, gives
+// the cheaper plan. That order is made only when dissection takes more than kSurfaceFlops n^1.5 (summed over the components):
+// plates and shell bodies take 2,000 to 5,500 n^1.5, the 64 x 64 plate rolled up in 2 turns 6,200, in 8 turns 23,000, with its
+// nodes' positions shuffled 1.7 M. A plan's time: its flops at kPlanRate, its longest chain of panels at kPanelTime each
+// (there and back, bl_multifrontal.cuh). B200, a frame of 33 substeps of that plate: flat 20.5 ms by dissection; rolled up in
+// 2, 4 and 8 turns 32.7, 40.8 and 43.7 by dissection, 28.1 by minimum degree each.
+constexpr double kSurfaceFlops = 6000.0, kPlanRate = 1e13, kPanelTime = 15e-6;
+static double fem_plan_time(const std::vector<int>& col_ptr, const std::vector<int>& row, const std::vector<int>& comp) {
+    std::vector<std::vector<int>> cols;
+    std::vector<int> top, fcomp;
+    const int n = (int)col_ptr.size() - 1;
+    mf_plan_columns(n, col_ptr, row, comp, cols, top, fcomp);
+    const MfPlan P = mf_finish(n, col_ptr, row, cols, top, fcomp);
+    return P.flops / kPlanRate + P.chain * kPanelTime;
+}
+static void fem_nested_order(const FemComponents& C, const std::vector<int>& ptr, const std::vector<int>& nbr, const std::vector<double>& x,
+                             std::vector<int>& order, std::vector<int>& col_ptr, std::vector<int>& row) {
+    const int n = (int)ptr.size() - 1;
+    std::vector<int> iperm(n), comp;
+    auto place = [&](const std::vector<int>& o) {
+        for (int k = 0; k < n; k++) iperm[o[k]] = k;
+    };
+    FemDissection D{ptr, nbr, x, std::vector<uint8_t>(n, 0)};
+    double surface = 0;
+    for (int c = 0; c < C.count; c++) {
+        D.run(C.nodes[c], order);
+        comp.resize(order.size(), c);
+        surface += kSurfaceFlops * std::pow((double)C.nodes[c].size(), 1.5);
+    }
+    place(order);
+    if (fem_symbolic(order, iperm, ptr, nbr, col_ptr, row, surface)) return;
+    QuotientGraph G(n);
+    std::vector<int> order2, reach, col_ptr2(1, 0), row2;
+    for (int c = 0; c < C.count; c++) fem_min_degree(C.nodes[c], ptr, nbr, G, order2, reach, col_ptr2);
+    place(order2);
+    row2.resize(reach.size());
+    for (size_t q = 0; q < reach.size(); q++) row2[q] = iperm[reach[q]];
+    for (int k = 0; k < n; k++) std::sort(row2.begin() + col_ptr2[k], row2.begin() + col_ptr2[k + 1]);
+    const double time2 = fem_plan_time(col_ptr2, row2, comp);
+    place(order); // (past time2's worth of flops it cannot be the cheaper)
+    if (fem_symbolic(order, iperm, ptr, nbr, col_ptr, row, time2 * kPlanRate) && fem_plan_time(col_ptr, row, comp) <= time2) return;
+    order.swap(order2), col_ptr.swap(col_ptr2), row.swap(row2);
 }
 
 // The update list of the column-by-column factorization: each source column k: the rows of column c = row[i]
@@ -624,7 +677,7 @@ static void fem_update_list(FemModel& M) {
 }
 
 // FemModel's ordering, pattern, block maps and gather lists; the update list too where want_updates; nested: the
-// multifrontal path's order instead of the reference's
+// multifrontal path's order (fem_nested_order) instead of the reference's
 static void fem_analyse(FemModel& M, bool want_updates = true, bool nested = false) {
     const int n = (int)M.node.size();
     const size_t T = M.tn.size(), E = M.mn.size();
@@ -636,20 +689,16 @@ static void fem_analyse(FemModel& M, bool want_updates = true, bool nested = fal
     std::vector<int> order, reach, reach_ptr(1, 0);
     order.reserve(n);
     QuotientGraph G(nested ? 0 : n);
-    FemDissection D{gptr, gnbr, M.xd, std::vector<uint8_t>(nested ? n : 0, 0)};
     for (int c = 0; c < C.count; c++) {
-        M.comp_first[c] = (int)order.size();
-        if (nested) D.run(C.nodes[c], order);
-        else fem_min_degree(C.nodes[c], gptr, gnbr, G, order, reach, reach_ptr);
+        M.comp_first[c + 1] = M.comp_first[c] + (int)C.nodes[c].size();
+        if (!nested) fem_min_degree(C.nodes[c], gptr, gnbr, G, order, reach, reach_ptr);
     }
-    M.comp_first[C.count] = n;
+    if (nested) fem_nested_order(C, gptr, gnbr, M.xd, order, M.col_ptr, M.row);
     M.perm = order;
     M.iperm.assign(n, 0);
     for (int k = 0; k < n; k++) M.iperm[order[k]] = k;
     // the pattern: column k's rows are the elimination positions of its node's neighbours at elimination, ascending
-    if (nested) {
-        fem_symbolic(M.perm, M.iperm, gptr, gnbr, M.col_ptr, M.row);
-    } else {
+    if (!nested) {
         M.col_ptr.assign(reach_ptr.begin(), reach_ptr.end());
         M.row.resize(reach.size());
         for (size_t q = 0; q < reach.size(); q++) M.row[q] = M.iperm[reach[q]];

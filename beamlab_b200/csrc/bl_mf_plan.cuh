@@ -40,6 +40,7 @@ struct MfPlan {
     std::vector<int> level_ptr;     // fronts of level L: [level_ptr[L], level_ptr[L + 1])
     std::vector<int> comp;          // the component each front belongs to (global)
     double flops = 0;               // per factorization (multiply and add counted apart)
+    int chain = 0;                  // the most pivot tiles of 8 nodes (panels) from a leaf to its root
     double entries = 0;             // dense lower-triangle entries over all fronts (DOF^2 / 2)
 };
 
@@ -175,6 +176,11 @@ static MfPlan mf_finish(int NF, const std::vector<int>& col_ptr, const std::vect
         const double p = 6.0 * P.npiv.back(), r = 6.0 * P.nrow.back();
         P.flops += p * p * p / 3 + p * p * r + p * r * r;
         P.entries += (p + r) * (p + r + 1) / 2;
+    }
+    std::vector<int> chain(nfr, 0);
+    for (int f = 0; f < nfr; f++) { // (children first)
+        P.chain = std::max(P.chain, chain[f] += (P.npiv[f] + 7) / 8);
+        if (P.parent[f] >= 0) chain[P.parent[f]] = std::max(chain[P.parent[f]], chain[f]);
     }
     // each front's rows in its parent's node list (both ascending: one merge walk)
     P.cmap.assign(P.idx.size(), -1);
