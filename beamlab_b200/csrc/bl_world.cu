@@ -181,7 +181,7 @@ struct bl_gpu_ctx {
     // the learned warm start (bl_mlp.cuh): parameters, the step's features, recorded samples, training scratch
     DevBuf<float> mlp_w, mlp_m, mlp_v, feat, prev_dv, smp_x, smp_t, smp_w, gpart, gsum;
     DevBuf<float> mlp_io;                      // the network's calls on host memory: the loss, samples, outputs (targets), weights
-    std::mutex mlp_mutex;                      // (these calls, one at a time)
+    std::mutex mlp_mutex;                      // (the calls that share mlp_io, gpart and gsum, one at a time)
     DevBuf<__nv_bfloat16> mlp_wb;
     DevBuf<int> adj_ptr, adj, scount, sidx;
     int rec_cap = 0;                           // the samples' capacity
@@ -2271,9 +2271,9 @@ int bl_gpu_mlp_samples(bl_gpu_ctx* c, int32_t* n) {
     return BL_GPU_OK;
 }
 
-// The network's calls on host memory, one at a time: their device buffer is the context's, and is given back at the end
-// of a call that needed more than kMlpKeep floats (128 MB: 559,000 samples). To allocate and release buffers on each call
-// took as long as its kernels.
+// The network's training, forward and gradient calls, one at a time whichever threads make them: their device buffers are the
+// context's. The samples' buffer of a call that needed more than kMlpKeep floats (128 MB: 559,000 samples) is given back at its
+// end. To allocate and release buffers on each call took as long as its kernels.
 constexpr size_t kMlpKeep = (size_t)32 << 20, kMlpHead = 64; // (kMlpHead: the loss's floats before the samples)
 struct MlpCall {
     bl_gpu_ctx* c;
@@ -2303,6 +2303,7 @@ static int mlp_batch(bl_gpu_ctx* c, const float* x, const float* t, const float*
 int bl_gpu_mlp_train(bl_gpu_ctx* c, int32_t epochs, int32_t batch, float lr, uint64_t seed, float* loss) {
     if (!c || epochs < 0 || batch < 1 || !(lr > 0)) return BL_GPU_EINVAL;
     BL_CUDA(c, cudaSetDevice(c->cfg.device));
+    const MlpCall call(c);
     BL_CUDA(c, cudaDeviceSynchronize());
     int n = 0;
     int rc = bl_gpu_mlp_samples(c, &n);
