@@ -38,7 +38,10 @@ namespace blg {
 constexpr int kMfChunk = kMfT * 16;    // doubles a chunk (16 columns)
 constexpr int kMfThreads = 128;
 constexpr int kMfStages = 4;           // the ring: chunks of both operands in flight
-constexpr unsigned long long kMfWaitNs = 4000000000ull;
+#ifndef BL_MF_WAIT_NS // (a test builds the library with 0: every wait that is not over at once runs out)
+#define BL_MF_WAIT_NS 4000000000ull
+#endif
+constexpr unsigned long long kMfWaitNs = BL_MF_WAIT_NS;
 constexpr size_t kMfSmem = sizeof(double) * (2 * kMfStages * kMfChunk + kMfTile);
 
 struct MfDev {
@@ -80,7 +83,7 @@ __device__ __forceinline__ bool mf_wait(const int* p, int target, int* abort_fla
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
             if (t0 == 0) t0 = t;
-            else if (t - t0 > kMfWaitNs) {
+            if (t - t0 >= kMfWaitNs) {
                 atomicExch(abort_flag, 1);
                 return false;
             }
