@@ -210,8 +210,10 @@ constexpr int kMfT = 48;               // tile side (8 frame nodes)
 constexpr int kMfTile = kMfT * kMfT;   // doubles a tile
 // In a level of many tasks (over kMfWide: several rounds of all resident CTAs) a front of one pivot tile and up to
 // kMfFuseRows row tiles is one task: no flags, its tiles still in the cache. In a narrower level its tiles are tasks of
-// their own, side by side. (B200: the 21 x 21 plate 231 us whole-front tasks off, 254 on; the 50k-node shell body 6.84
-// and 6.49 ms.)
+// their own, side by side. (B200, ms a substep with the line at 0, 1,000, 3,000, 10,000 and no whole fronts: the 41 x 41 plate
+// 0.51, 0.41 and so on; 64 x 64 0.69, 0.65, 0.62, 0.62, 0.62; 91 x 91 1.03, 1.03, 1.05, 1.05, 1.05; shell bodies of 5,000 nodes
+// 1.02, 1.02, 0.97, 0.97, 0.97; 10,000 1.53, 1.52, 1.55, 1.58, 1.58; 20,000 2.64, 2.64, 2.64, 2.78, 2.79; 50,000 6.66, 6.65,
+// 6.65, 6.65, 7.03.)
 constexpr int kMfFuseRows = 3, kMfWide = 3000;
 
 struct MfFrontDev {

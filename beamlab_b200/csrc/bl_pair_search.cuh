@@ -26,7 +26,9 @@ constexpr int kQueryChunk = 256;       // queries of one chunk (a CTA of k_pair_
 constexpr int kQueryGrid = 148 * 8;    // CTAs of k_pair_count / k_pair_write (they stride over the chunks)
 constexpr int kLocPairs = 64;          // a query's pairs the count pass keeps (more: the write pass runs it again)
 constexpr int kChunkPairs = 2048;      // ... of a chunk's by rows
-constexpr int kFewChunks = 148;        // chunks up to which fast queries go by rows (an SM each)
+// Chunks up to which fast queries go by rows (an SM each). B200, a search with 51, 83, 132, 177, 240, 473 and 1,049 chunks:
+// a query a thread 282, 284, 320, 329, 324, 382 and 481 us, by rows 253, 256, 317, 324, 357, 586 and 741.
+constexpr int kFewChunks = 148;
 
 struct IslBody {
     int id;               // global body index
