@@ -99,9 +99,11 @@ typedef struct {
                                   reference's order of sums throughout. 2 and 1 differ from 0 in the order of the
                                   floating-point sums only. */
     /* launch shapes (results do not depend on them; beamlab_b200/autotune.py measures them for a device and workload): */
-    int32_t force_block;       /* the nodes' force kernel's block size: 64, 128 or 256; 0 (default): 256 */
+    int32_t force_block;       /* the nodes' force kernel's block size: 64, 128 or 256; 0 (default): 256. Worlds of up to
+                                  6,000 nodes take a warp a node, always in blocks of 256 */
     int32_t integrate_block;   /* the integration kernel's block size: 64, 128 or 256; 0 (default): 256 */
-    int32_t beams_per_sm;      /* the beams' persistent kernel's blocks an SM (at most what fits); 0 (default): what fits */
+    int32_t beams_per_sm;      /* the beams' persistent kernel's blocks an SM (at most what fits); 0 (default): what fits.
+                                  Worlds whose beams come by plain loads (beam_kernel) have no such kernel */
     float tyre_grip;           /* WorldSettings::tyre_grip (1): a factor on the tyres' friction (tyre_contact) */
     float bulk_wait_s;         /* (no counterpart in the reference) the beams kernel's bound on a wait for its own bulk
                                   copies, in seconds (default 1, at most 10): one that runs out raises
@@ -469,7 +471,8 @@ int bl_gpu_mlp_gradient(bl_gpu_ctx* ctx, const float* x, const float* t, const f
 int bl_gpu_download_pairs(bl_gpu_ctx* ctx, int32_t* pairs, int32_t capacity, int32_t* n_pairs);
 
 /* One frame of n substeps, like bl_gpu_step_substeps, with a timing event between its kernels; waits for it and
- * returns the GPU time of each kind of kernel (summed over the frame's substeps). */
+ * returns the GPU time of each kind of kernel (summed over the frame's substeps). Its kernels run one after another, an
+ * event between the kinds; where a stepped frame's overlap (beam arrays by plain loads) its times add up to more. */
 typedef struct {
     int32_t substeps;
     float frame_ms;            /* the whole frame */
