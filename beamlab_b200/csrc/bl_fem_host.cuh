@@ -505,9 +505,9 @@ static void fem_min_degree(const std::vector<int>& comp, const std::vector<int>&
 // of the axes (near the middle, between two layers of nodes) into two sides and the separator that keeps them apart -
 // the nodes of one side next to the other - where the separator is smallest for its balance; both sides come before
 // it, each ordered the same way. The factor's fronts are then the separators, in a tree of halving sets: its longest
-// chain of dependent panels is about half the minimum-degree order's (the 64 x 64 plate 31 panels of 48 columns against
-// 55, the 50k-node shell body 136 against 204) and large bodies need fewer operations (63 against 83 GFLOP there).
-constexpr int kDissectLeaf = 16; // sets of this many nodes are ordered as they come (two tiles of a front)
+// chain of dependent panels is shorter than the minimum-degree order's (the 64 x 64 plate 31 panels of 48 columns against
+// 43, the 50k-node shell body 136 against 155) and large bodies need fewer operations (63 against 79 GFLOP there).
+constexpr int kDissectLeaf = 16; // sets of up to this many nodes keep the order they come in (two tiles of a front)
 struct FemDissection {
     const std::vector<int>&ptr, &nbr;
     const std::vector<double>& x;    // 3 per frame node

@@ -915,7 +915,7 @@ __global__ void k_drag_parts(Body* __restrict__ bodies, int nbodies, const float
 // close enough (bl_world.cu checks every warp)
 // kWide: a warp a node, a lane an incidence - the gathers of a node's beams all at once, their forces then added in their
 // order by broadcasts (the same sums) - for worlds whose nodes all fit on the GPU that way: a node of 26 beams waits for
-// one gather instead of seven (B200, a frame of 33 substeps of the 400-node truss car: 333 us a thread a node, 265 so).
+// one gather instead of seven (B200, a frame of 33 substeps of the 400-node truss car: 345 us a thread a node, 269 so).
 // The gathers of the nodes come before the wait for the beams' kernel, whose scalars are all that is new (from L2, bl_device.cuh;
 // after the wait: 3.5 % of a frame of 400 to 500 nodes).
 template <bool kPacked, bool kWide>

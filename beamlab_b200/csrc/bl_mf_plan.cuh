@@ -9,9 +9,10 @@
 //  * Relaxed amalgamation: a group merges into its parent group while the merged group stays small or adds few
 //    explicit zeros (the thresholds below, in frame nodes: 6 degrees of freedom each).
 //  * Each front holds its pivots (its columns) and its rows (the structure above them), both in elimination order, as
-//    one dense lower triangle in degrees of freedom, column-major. Its factorization eliminates the pivots and leaves
-//    the Schur complement of its rows in place, which its parent adds into its own front (extend-add).
-//  * Fronts run level by level of the front tree (leaves first), every front of a level at once.
+//    a lower triangle of 48 x 48 tiles, the pivots in tiles of their own. Its factorization eliminates the pivots and
+//    leaves the Schur complement of its rows in place, which its parent adds into its own front (extend-add).
+//  * The tiles are tasks in one list - fronts by level of the front tree, leaves first, a level's tiles column by column -
+//    in which every task's inputs come before it (mf_layout).
 // The solution equals the column-by-column one up to the order of the floating-point sums.
 #pragma once
 

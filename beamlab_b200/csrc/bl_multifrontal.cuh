@@ -15,15 +15,16 @@
 //                    cores' accumulators, L tiles stream through a ring of asynchronous copies as they become ready);
 //                    then for a pivot column j: the diagonal tile is factored and its inverse kept, a tile below it is
 //                    multiplied by that inverse; a tile past the pivots is the Schur complement its parent takes.
-//   front (f)        a front of one pivot tile and at most two row tiles (most leaves): all its tiles by one CTA, no flags
+//   front (f)        a front of one pivot tile and up to three row tiles, b's among them, in a wide level (most leaves of large
+//                    bodies): all its tiles by one CTA, no flags
 //   backward (f, s)  from the root down: x_s = L_ss^-T (y_s - sum_(i > s) L_is^T x_i), the rows' x from the ancestors
 // No atomics on values and every sum in a fixed order: the same bits every run. rhs gets the solution in column order.
 // A pivot that is not positive marks the front's component failed (the reference's chol6 failing, frame_fem.cpp:
 // 2900-2909: that component's step falls back to its explicit forces) and goes on as 1.
 //
-// What bounds it: small frames by the chain of dependent panels (a panel ~11 us: the diagonal tile's inverse factor 4.0, a
-// product with it 2.5, the update of the next diagonal tile 2.5, their flags 1 each; backward 2.7), large ones by the
-// fp64 rate. 48: a multiple of a node's 6 degrees of freedom and of the instruction's 8, three CTAs an SM with both
+// What bounds it: small frames by the chain of dependent panels (a panel ~12 us: the diagonal tile's inverse factor 4.0, a
+// product with it 2.5, the update of the next diagonal tile 2.5, the rest flags and loads through L2; 3.9 on the way back), large
+// ones by the tiles' operands from L2 and a barrier a chunk, at 0.27 of the fp64 rate. 48: a multiple of a node's 6 degrees of freedom and of the instruction's 8, three CTAs an SM with both
 // operands' ring. Measured on B200 (factorization and solves alone; before: minimum-degree fronts, a launch a panel and
 // a launch an update, 32 x 32 tiles on the plain fp64 units): the 21 x 21 plate 0.21 ms, the 64 x 64 plate 0.56 (3.9),
 // the 10k-node shell body 1.43 (7.8), the 50k-node one 6.3 (38.0): 63.3 GFLOP at 10.1 TFLOP/s of the 35.5 a cuBLAS

@@ -545,12 +545,8 @@ static int pull_state(bl_gpu_ctx* c) {
     return BL_GPU_OK;
 }
 
-// The FEM frames of all bodies on the device, back to back, and the factorization's schedule: the columns by
-// elimination-tree level (a column's level is one more than its deepest child's), each level's target blocks (a
-// column's diagonal block then its off-diagonal ones) with each target's updates in the order of their source columns,
-// each row's blocks in the order of their columns for the forward substitution.
 // The multifrontal plan over every frame's columns (global pattern col_ptr / row, components col_comp): the fronts,
-// their tiles' maps and the pool on the device, and k_mf_solve's task list (bl_multifrontal.cuh)
+// their tiles' maps and the pool on the device, and k_mf_factor's and k_mf_back's task list (bl_multifrontal.cuh)
 static int commit_multifrontal(bl_gpu_ctx* c, const std::vector<int>& col_ptr, const std::vector<int>& row, const std::vector<int>& col_comp,
                                const std::vector<int>& goff_ptr, int ncomp) {
     const int NF = (int)col_ptr.size() - 1;
@@ -588,6 +584,10 @@ static int commit_multifrontal(bl_gpu_ctx* c, const std::vector<int>& col_ptr, c
     return BL_GPU_OK;
 }
 
+// The FEM frames of all bodies on the device, back to back, and the factorization's schedule: the columns by
+// elimination-tree level (a column's level is one more than its deepest child's), each level's target blocks (a
+// column's diagonal block then its off-diagonal ones) with each target's updates in the order of their source columns,
+// each row's blocks in the order of their columns for the forward substitution.
 static int commit_fem(bl_gpu_ctx* c) {
     int NF = 0, NT = 0, NB = 0, NC = 0, NS = 0, nfem_nodes = 0;
     for (const HostBody& hb : c->bodies)
@@ -1436,11 +1436,11 @@ static void launch_pcg(bl_gpu_ctx* c, cudaStream_t s, cudaGraphConditionalHandle
 }
 
 // Beams by plain loads up to this many, by bulk copies above; forces a warp a node up to this many nodes. Measured on B200, a
-// frame of 33 substeps in us, each rule alone against its alternative: the 400-node truss car 261 (bulk copies 368 with
-// programmatic launches, 458 without; a thread a node 333), one vehicle of 5,072 nodes 816 (976; 884), two of
-// 8,536 nodes 885 a thread a node, 935 a warp; 16 vehicles with 0.55 M beams 1150 by plain loads, 1207 by bulk copies, 64 with
-// 2.2 M 2498 and 2528, 256 with 8.9 M even. Programmatic launches beside the bulk copies' persistent blocks, which hold
-// the shared memory the running kernel's blocks need: 6 to 8 % slower from 32 vehicles on, so those go without.
+// frame of 33 substeps in us, each rule alone against its alternative: the 400-node truss car 269 (bulk copies 413; a thread
+// a node 345), trusses of 5,096 nodes 329 (448; 344), of 6,400 nodes 356 a thread a node, 371 a warp, of 8,670 376 and 409; 16
+// vehicles with 0.55 M beams 1,067 by plain loads, 1,163 by bulk copies, 64 with 2.2 M 2,418 and 2,555, 256 with 8.9 M 6,450 and
+// 6,120. Programmatic launches beside the bulk copies' persistent blocks, which hold the shared memory the running kernel's
+// blocks need: 6 to 8 % slower from 32 vehicles on, so those go without.
 constexpr int kPlainBeams = 4000000, kWideNodes = 6000;
 
 // kernel<<<grid, block, smem, s>>>(args...); early: it may start while the kernel before it on the stream still runs

@@ -74,7 +74,8 @@ class WorldSettings:
     # the beams' kernel: 0 bulk (TMA) copies of the beam arrays above 4 M beams, else plain loads; 1 plain loads and 8-byte
     # incidences; 2 bulk copies at any size (the same results)
     beam_kernel: int = 0
-    # the FEM factorization: 3 the fastest (2), 2 multifrontal (dense fronts of tiles, one launch), 1 block columns with the top chain as one dense front, 0 block columns in the reference's order
+    # the FEM factorization: 3 the fastest (2), 2 multifrontal (dense fronts of tiles; a launch for the factorization, one for
+    # the way back), 1 block columns with the top chain as one dense front, 0 block columns in the reference's order
     fem_dense_front: int = 3
     tyre_grip: float = 1.0                    # WorldSettings::tyre_grip: a factor on the tyres' friction
     bulk_wait_s: float = 1.0                  # the beams kernel's bound on a wait for its bulk copies (0: runs out)

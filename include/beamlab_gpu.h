@@ -91,9 +91,10 @@ typedef struct {
                                   incidences; 2: as 0, the bulk copies at any size. Results are the same. */
     int32_t fem_dense_front;   /* how the FEM step factors its system:
                                   3 (default): 2;
-                                  2: multifrontal - the columns in a nested-dissection order, grouped into dense fronts
-                                  (supernodes of the elimination tree, small ones amalgamated) of 48 x 48 tiles, the factorization
-                                  one launch, the backward solves another; with the reference's order, pattern and fill
+                                  2: multifrontal - the columns in a nested-dissection order (a minimum-degree one where that
+                                  is cheaper), grouped into dense fronts (supernodes of the elimination tree, small ones
+                                  amalgamated) of 48 x 48 tiles, the factorization one launch, the backward solves another;
+                                  with the reference's order, pattern and fill -
                                   1: block column by block column, with the top chain of the elimination tree
                                   (levels of one column each) as one dense front; 0: block column by block column in the
                                   reference's order of sums throughout. 2 and 1 differ from 0 in the order of the
@@ -205,10 +206,9 @@ typedef struct {
 
 /* A body's FEM frame (FemFrame, frame_fem.h:330-815): its add_element calls (the members) and its add_tri calls (the
  * triangles) - the frame nodes are numbered as those calls meet them, the members' first unless tris_first; no mounts
- * or springs. The
- * library does what the reference's FemFrame::finalize and analyse do (rest frames and shapes, inertias, the
- * minimum-degree ordering and the factor's pattern) and steps it implicitly every substep (FemFrame::solve,
- * frame_fem.cpp:2512-3027). */
+ * or springs. The library does what the reference's FemFrame::finalize and analyse do (rest frames and shapes, inertias,
+ * an elimination order and the factor's pattern: fem_dense_front) and steps it implicitly every substep
+ * (FemFrame::solve, frame_fem.cpp:2512-3027). */
 typedef struct {
     int32_t n_sections;
     const bl_shell_section* sections;
@@ -489,8 +489,8 @@ typedef struct {
 int bl_gpu_profile_frame(bl_gpu_ctx* ctx, int32_t n, void* stream, bl_frame_profile* out);
 
 /* The symbolic phase of a FEM frame, on the host, no GPU needed: what bl_gpu_add_body computes for the frame of `fem`
- * over the body's nodes - FemFrame::analyse's exact minimum-degree order and factor pattern (frame_fem.cpp:544-860)
- * and FemFrame::finalize's rest shapes and inertias (frame_fem.cpp:224-260, 3075-3086). sizes[0..3] receive the frame
+ * over the body's nodes - FemFrame::analyse's exact minimum-degree order and factor pattern (frame_fem.cpp:544-860; those
+ * of fem_dense_front 0 and 1) and FemFrame::finalize's rest shapes and inertias (frame_fem.cpp:224-260, 3075-3086). sizes[0..3] receive the frame
  * nodes, off-diagonal blocks, block updates and components; any array may be NULL (call once with NULLs for sizes):
  * perm (frame nodes), col_ptr (frame nodes + 1), row (blocks), upd (3 per update: pi, pj, target as the reference
  * stores them), rest (6 per triangle: its corners in its plane), inertia (frame nodes). */
