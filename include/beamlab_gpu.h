@@ -333,8 +333,10 @@ enum {
     BL_GPU_DEVERR_PAIRS = 1 << 2,      /* the contact pair list (or the search's queries) overflowed bl_gpu_config.max_pairs */
     BL_GPU_DEVERR_ISLAND = 1 << 3,     /* an island with contact pairs held more than BL_GPU_MAX_ISLAND_BODIES bodies */
     BL_GPU_DEVERR_CONTACT_UNSUPPORTED = 1 << 5, /* a body with a FEM frame met another body's triangles (not stepped) */
-    BL_GPU_DEVERR_TIMEOUT = 1 << 6     /* a kernel's bounded wait on its own bulk copies ran out (bulk_wait_s): the
-                                          substep's beams were not all stepped */
+    BL_GPU_DEVERR_TIMEOUT = 1 << 6     /* a kernel's bounded wait ran out: on the beams' bulk copies (bulk_wait_s), the
+                                          substep's beams were not all stepped; between the blocks of the FEM factorization
+                                          (fem_dense_front 2 and 3; 4 s), the frames took their elements' forces that substep,
+                                          as at a factorization that fails */
 };
 #define BL_GPU_MAX_ISLAND_BODIES 256
 #define BL_GPU_MAX_CANDIDATES 64
